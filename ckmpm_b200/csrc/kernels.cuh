@@ -215,7 +215,7 @@ __device__ __forceinline__ float4 node_velocity(const SceneDev& sc, const long l
     v.x = __ll2float_rn(__ldcg(blk + 128 + cell)) * unit * inv;
     v.y = __ll2float_rn(__ldcg(blk + 256 + cell)) * unit * inv;
     v.z = __ll2float_rn(__ldcg(blk + 384 + cell)) * unit * inv;
-    v.y += sc.gravity * dt;
+    v.y = fmaf(sc.gravity, dt, v.y);
     if (sc.boundary == 0) {
       const bool out = (bx < 2 || bx + 2 >= sc.dims[0]) || (by < 2 || by + 2 >= sc.dims[1]) ||
                        (bz < 2 || bz + 2 >= sc.dims[2]);
@@ -308,49 +308,49 @@ __device__ __forceinline__ void load_velocity_tile(const SceneDev& sc, const lon
   }
 }
 
-// Per-axis stencil of one grid at scaled position xs (= x / dx): base cell,
-// offset o in [0,1) and weight w0 (include/mpm_algorithm.cuh:60-67,
-// include/mpm_kernel.cuh:91-114).  g = -1 or +1.
+// Cell of grid -dx/4 that holds coordinate x (the binning's cell).
+__device__ __forceinline__ int cell_of(float x, float inv_dx) { return static_cast<int>(fmaf(x, inv_dx, 0.25f)); }
+
+// Both grids' stencils along one axis at position x: base cells b, offsets o in [0, 1) and first-node weights w0 = 1 - o + sin(2 pi o) / (2 pi)
+// (include/mpm_algorithm.cuh:60-67, include/mpm_kernel.cuh:91-114); index 0 is
+// grid -dx/4, 1 is grid +dx/4.  The grids are half a cell apart, so the second
+// stencil follows from the first: o1 = o0 -+ 1/2 and sin(2 pi o1) = -sin(2 pi o0).
+// The sine is taken of the centred offset c = o0 - 1/2 (sin(2 pi o0) =
+// -sin(2 pi c)), which keeps the argument within [-pi, pi], where __sinf's error
+// is bounded (2^-21.4).
 struct AxisStencil {
-  int base;
-  float o, w0;
+  int b[2];
+  float o[2], w0[2];
+  float c, s;  // o0 - 1/2; sin(2 pi o0) / (2 pi)
 };
 
-template <int G>
-__device__ __forceinline__ AxisStencil axis_stencil(float xs) {
-  AxisStencil s;
-  s.base = static_cast<int>(xs - 0.25f * G);
-  const float local = xs - static_cast<float>(s.base);
-  s.o = local - 0.25f * G;
-  s.w0 = ck_w0(s.o);
-  return s;
+__device__ __forceinline__ AxisStencil axis_stencil(float x, float inv_dx) {
+  AxisStencil st;
+  st.b[0] = cell_of(x, inv_dx);
+  st.o[0] = fmaf(x, inv_dx, 0.25f - static_cast<float>(st.b[0]));
+  st.c = st.o[0] - 0.5f;
+  st.s = __fmul_rn(-0.15915494309189535f, __sinf(6.283185307179586f * st.c));
+  const bool upper = st.c >= 0.f;
+  st.b[1] = upper ? st.b[0] : st.b[0] - 1;
+  st.o[1] = upper ? st.c : st.c + 1.0f;
+  st.w0[0] = 1.0f - st.o[0] + st.s;
+  st.w0[1] = 1.0f - st.o[1] - st.s;
+  return st;
 }
 
-
-// First and second weighted moments of one grid along one axis (world units):
-// m1 = sum_d w_d (d - o) dx, m2 = sum_d w_d (d - o)^2 dx^2.  With a tensor
-// product kernel whose 1-D weights sum to one, D = sum_nodes w r r^T has
-// D_aa = m2_a and D_ab = m1_a m1_b for each grid.
-__device__ __forceinline__ void axis_moments(const AxisStencil& s, float dx, float& m1, float& m2) {
-  const float w1 = 1.0f - s.w0;
-  m1 = (w1 - s.o) * dx;
-  const float a = s.o, b = 1.0f - s.o;
-  m2 = (s.w0 * a * a + w1 * b * b) * dx * dx;
-}
-
-// D (symmetric, 6 entries: 00, 11, 22, 01, 02, 12) summed over both grids.
-__device__ __forceinline__ void d_matrix(const AxisStencil (&st)[2][3], float dx, float* D6) {
-  float m1[2][3], m2[2][3];
+// D / dx^2 with D = sum_nodes w r r^T over both grids (symmetric, 6 entries: 00,
+// 11, 22, 01, 02, 12).  With a tensor product kernel whose 1-D weights sum to
+// one, each grid adds its second moments to the diagonal and the products of
+// its first moments elsewhere.  The first moments are -s and +s, and the sum of
+// the two second moments o (1 - o) -+ s (1 - 2 o) is 1/4 + |c| - 2 c^2 - |s|.
+__device__ __forceinline__ void d_matrix(const AxisStencil (&st)[3], float* D6) {
 #pragma unroll
-  for (int g = 0; g < 2; ++g)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) axis_moments(st[g][a], dx, m1[g][a], m2[g][a]);
-  D6[0] = m2[0][0] + m2[1][0];
-  D6[1] = m2[0][1] + m2[1][1];
-  D6[2] = m2[0][2] + m2[1][2];
-  D6[3] = m1[0][0] * m1[0][1] + m1[1][0] * m1[1][1];
-  D6[4] = m1[0][0] * m1[0][2] + m1[1][0] * m1[1][2];
-  D6[5] = m1[0][1] * m1[0][2] + m1[1][1] * m1[1][2];
+  for (int a = 0; a < 3; ++a)
+    D6[a] = fmaf(-2.0f * st[a].c, st[a].c, 0.25f + fabsf(st[a].c)) - fabsf(st[a].s);
+  const float t = 2.0f * st[0].s;
+  D6[3] = t * st[1].s;
+  D6[4] = t * st[2].s;
+  D6[5] = 2.0f * st[1].s * st[2].s;
 }
 
 __device__ __forceinline__ void sym_to_full(const float* s6, float* f) {
@@ -363,19 +363,18 @@ __device__ __forceinline__ void sym_to_full(const float* s6, float* f) {
 }
 
 // G2P on both grids (include/mpm_algorithm.cuh:1555-1638): returns the
-// halved interpolated velocity and C = B D^-1, where B = sum v_i (w r_i)^T
+// halved interpolated velocity, C dx = (B / dx) (D / dx^2)^-1, where B = sum v_i (w r_i)^T
 // and D = sum w r_i r_i^T with r_i = x_i - x_p, both over the 16 nodes, and
-// D itself (6 entries) in D6.
-// B is accumulated through the separable sums S = sum w v and
-// T_a = sum over nodes with d_a = 1 of w v:  B[r][a] = dx (T_a[r] - o_a S[r]).
-__device__ __forceinline__ void g2p(const float4* __restrict__ vtile, const float (&xs)[3], int4 key, float dx,
-                                    float* v, float* C, bool& inside, float* D6) {
-  AxisStencil st[2][3];
+// D / dx^2 itself (6 entries) in D6.
+// B is accumulated through the separable sums S = sum w v and T_a = sum over
+// nodes with d_a = 1 of w v:  B[r][a] / dx = T_a[r] - o_a S[r], reduced one axis
+// at a time (z, y, x): 66 multiply-adds per grid, where one weight per node
+// takes about 100.
+__device__ __forceinline__ void g2p(const float4* __restrict__ vtile, const float (&x)[3], float inv_dx, int4 key,
+                                    float* v, float* Cdx, bool& inside, float* D6) {
+  AxisStencil st[3];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    st[0][a] = axis_stencil<-1>(xs[a]);
-    st[1][a] = axis_stencil<1>(xs[a]);
-  }
+  for (int a = 0; a < 3; ++a) st[a] = axis_stencil(x[a], inv_dx);
   float B[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) B[k] = 0.f;
@@ -387,46 +386,47 @@ __device__ __forceinline__ void g2p(const float4* __restrict__ vtile, const floa
     const int lo = g == 0 ? 2 : 1;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      l[a] = st[g][a].base - kb[a];
+      l[a] = st[a].b[g] - kb[a];
       if (l[a] < lo || l[a] > 5) {
         inside = false;
         l[a] = min(max(l[a], lo), 5);
       }
     }
-    const float wx[2] = {st[g][0].w0, 1.f - st[g][0].w0};
-    const float wy[2] = {st[g][1].w0, 1.f - st[g][1].w0};
-    const float wz[2] = {st[g][2].w0, 1.f - st[g][2].w0};
-    float S[3] = {0.f, 0.f, 0.f}, T[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) T[r][0] = T[r][1] = T[r][2] = 0.f;
+    const float wx0 = st[0].w0[g], wx1 = 1.f - wx0;
+    const float wy0 = st[1].w0[g], wy1 = 1.f - wy0;
+    const float wz0 = st[2].w0[g], wz1 = 1.f - wz0;
     const int sx = g == 0 ? 25 : 36, sy = g == 0 ? 5 : 6;
     const float4* base = vtile + vtile_index(g, l[0], l[1], l[2]);
+    float Sy[2][3], Ty[2][3], Tz[2][3];
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const int dxn = (n >> 2) & 1, dyn = (n >> 1) & 1, dzn = n & 1;
-      const float w = wx[dxn] * wy[dyn] * wz[dzn];
-      const float4 vi = base[dxn * sx + dyn * sy + dzn];
-      const float wv[3] = {w * vi.x, w * vi.y, w * vi.z};
+    for (int i = 0; i < 2; ++i) {
+      const float4 a0 = base[i * sx], a1 = base[i * sx + 1], b0 = base[i * sx + sy], b1 = base[i * sx + sy + 1];
+      const float va[2][3] = {{a0.x, a0.y, a0.z}, {a1.x, a1.y, a1.z}};
+      const float vb[2][3] = {{b0.x, b0.y, b0.z}, {b1.x, b1.y, b1.z}};
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        S[r] += wv[r];
-        if (dxn) T[r][0] += wv[r];
-        if (dyn) T[r][1] += wv[r];
-        if (dzn) T[r][2] += wv[r];
+        const float ta = wz1 * va[1][r], tb = wz1 * vb[1][r];
+        const float sa = fmaf(wz0, va[0][r], ta), sb = fmaf(wz0, vb[0][r], tb);
+        Ty[i][r] = wy1 * sb;
+        Sy[i][r] = fmaf(wy0, sa, Ty[i][r]);
+        Tz[i][r] = fmaf(wy0, ta, wy1 * tb);
       }
     }
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-      vs[r] += S[r];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) B[r * 3 + a] += dx * (T[r][a] - st[g][a].o * S[r]);
+      const float Tx = wx1 * Sy[1][r];
+      const float S = fmaf(wx0, Sy[0][r], Tx);
+      vs[r] += S;
+      B[r * 3] += fmaf(-st[0].o[g], S, Tx);
+      B[r * 3 + 1] += fmaf(-st[1].o[g], S, fmaf(wx0, Ty[0][r], wx1 * Ty[1][r]));
+      B[r * 3 + 2] += fmaf(-st[2].o[g], S, fmaf(wx0, Tz[0][r], wx1 * Tz[1][r]));
     }
   }
   float Di6[6], Di[9];
-  d_matrix(st, dx, D6);
+  d_matrix(st, D6);
   inv_sym3(D6[0], D6[1], D6[2], D6[3], D6[4], D6[5], Di6);
   sym_to_full(Di6, Di);
-  matmul3(B, Di, C);
+  matmul3(B, Di, Cdx);
 #pragma unroll
   for (int r = 0; r < 3; ++r) v[r] = 0.5f * vs[r];
 }
@@ -470,18 +470,19 @@ __device__ __forceinline__ unsigned long long tile_sum(const unsigned* tile, int
 // Per unit particle mass: node mass w, node momentum w (v + Ah (d - o)) with
 // Ah = A dx / m (A the reference's affine contribution).  Integer atomics make
 // the tile sum independent of the order in which particles arrive.
-__device__ __forceinline__ void p2g_scatter(unsigned* __restrict__ ptile, const AxisStencil (&st)[2][3],
-                                            const int (&lbase)[2][3], const float* v, const float* Ah) {
+__device__ __forceinline__ void p2g_scatter(unsigned* __restrict__ ptile, const AxisStencil (&st)[3], int4 key,
+                                            const float* v, const float* Ah) {
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
     float Q[3];
 #pragma unroll
     for (int r = 0; r < 3; ++r)
-      Q[r] = v[r] - (Ah[r * 3] * st[g][0].o + Ah[r * 3 + 1] * st[g][1].o + Ah[r * 3 + 2] * st[g][2].o);
-    const float wx[2] = {st[g][0].w0 * kFixScale, (1.f - st[g][0].w0) * kFixScale};
-    const float wy[2] = {st[g][1].w0, 1.f - st[g][1].w0};
-    const float wz[2] = {st[g][2].w0, 1.f - st[g][2].w0};
-    unsigned* base = ptile + ((g * 8 + lbase[g][0]) * kTileRow + lbase[g][1] * 8 + lbase[g][2]);
+      Q[r] = v[r] - dot3(Ah[r * 3], st[0].o[g], Ah[r * 3 + 1], st[1].o[g], Ah[r * 3 + 2], st[2].o[g]);
+    const float wx[2] = {st[0].w0[g] * kFixScale, (1.f - st[0].w0[g]) * kFixScale};
+    const float wy[2] = {st[1].w0[g], 1.f - st[1].w0[g]};
+    const float wz[2] = {st[2].w0[g], 1.f - st[2].w0[g]};
+    unsigned* base = ptile + ((g * 8 + st[0].b[g] - 4 * key.x) * kTileRow + (st[1].b[g] - 4 * key.y) * 8 + st[2].b[g] -
+                              4 * key.z);
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       const int dxn = (n >> 2) & 1, dyn = (n >> 1) & 1, dzn = n & 1;
@@ -616,7 +617,11 @@ __device__ __forceinline__ void incoming_groups(const SceneDev& sc, const BlockL
   if (lane == 26) s_off[27] = incl;
 }
 
+// The group that holds incoming particle q.  Almost every particle stays in its
+// block (direction 13), so that group is tried before the binary search.
 __device__ __forceinline__ int find_group(const uint32_t* s_off, uint32_t q) {
+  const uint32_t stay = s_off[13];
+  if (q - stay < s_off[14] - stay) return 13;
   int lo = 0, hi = 27;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -691,7 +696,8 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
   long long* __restrict__ gout = gd.grid[parity ^ 1];
   const int32_t* __restrict__ stin = gd.stamp[parity];
   const uint32_t nb = *cur.nblocks;
-  const float dx = sc.dx, inv_dx = sc.inv_dx;
+  const float inv_dx = sc.inv_dx;
+  const float dtdx = dt * inv_dx;
   const uint32_t maxp = min(md.max_per_block, static_cast<uint32_t>(kMaxParticlesPerBlock));
 
   for (int i = threadIdx.x; i < 2 * kTilePlane / 4; i += NT)
@@ -758,16 +764,15 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         for (int k = 0; k < 9; ++k) F[k] = sin.F[k][iin];
       }
       if (material_has_aux(kind)) aux = sin.aux[iin];
-      float xs[3] = {x[0] * inv_dx, x[1] * inv_dx, x[2] * inv_dx};
       bool inside = true;
-      float v[3], C[9], Dold[6];
-      g2p(vtile, xs, key, dx, v, C, inside, Dold);
+      float v[3], Cdx[9], Dold[6];  // C dx and D / dx^2
+      g2p(vtile, x, inv_dx, key, v, Cdx, inside, Dold);
       float adv[3] = {v[0], v[1], v[2]};
       if (RIGID && rigid_attribute(kind, F, aux) == 0.f) {
         // Rigid: moves with the scene's rigid velocity and carries no velocity,
         // no affine field and no G2P D (include/mpm_algorithm.cuh:1609-1618).
 #pragma unroll
-        for (int k = 0; k < 9; ++k) C[k] = 0.f;
+        for (int k = 0; k < 9; ++k) Cdx[k] = 0.f;
 #pragma unroll
         for (int k = 0; k < 6; ++k) Dold[k] = 0.f;
 #pragma unroll
@@ -777,15 +782,18 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         }
       }
 #pragma unroll
-      for (int a = 0; a < 3; ++a) x[a] += dt * adv[a];
+      for (int a = 0; a < 3; ++a) x[a] = fmaf(dt, adv[a], x[a]);
 
       float tau[9];
       if (kind == kFluid) {
+        float C[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) C[k] = __fmul_rn(Cdx[k], inv_dx);
         stress_fluid(mp0, mp1, mp2, C, dt, aux, tau);
       } else {
         float dW[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) dW[k] = C[k] * dt + ((k & 3) ? 0.f : 1.f);
+        for (int k = 0; k < 9; ++k) dW[k] = (k & 3) ? Cdx[k] * dtdx : fmaf(Cdx[k], dtdx, 1.f);
         matmul3(dW, F, F);
         if (kind == kFixedCorotated) {
           stress_fixed_corotated(mp0, mp1, F, tau);
@@ -799,9 +807,12 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
           for (int k = 0; k < kMaterialParams; ++k) prm[k] = KIND == kMixed ? md.smat[key.w].p[k] : md.mat.p[k];
           stress_nacc(prm, F, aux, tau);
         } else {  // kLinear
-          float Q[9];
+          float Q[9], C[9];
 #pragma unroll
-          for (int k = 0; k < 9; ++k) Q[k] = sin.Q[k][iin];
+          for (int k = 0; k < 9; ++k) {
+            Q[k] = sin.Q[k][iin];
+            C[k] = __fmul_rn(Cdx[k], inv_dx);
+          }
           stress_linear(C, dt, F, Q, tau);
 #pragma unroll
           for (int k = 0; k < 9; ++k) sout.Q[k][o_slot(start, q)] = Q[k];
@@ -820,14 +831,12 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       if (md.track_ids) sout.id[o] = sin.id[iin];
 
       // Rebin record: direction code of (old block - new block), 27 = lost.
-#pragma unroll
-      for (int a = 0; a < 3; ++a) xs[a] = x[a] * inv_dx;
       int cn[3], sh3[3];
       bool win = true, ok = true;
       const int kk[3] = {key.x, key.y, key.z};
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        cn[a] = static_cast<int>(xs[a] + 0.25f);
+        cn[a] = cell_of(x[a], inv_dx);
         const int nbk = trunc_div4(cn[a] - 2);
         sh3[a] = kk[a] - nbk;
         ok &= (sh3[a] >= -1 && sh3[a] <= 1);
@@ -848,17 +857,11 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       // reference adds the new position's D onto the G2P D of the old position
       // (it never resets it, :1524,1604,1729) and inverts half the sum (:1732),
       // so M = (0.5 (D_old + D_new))^-1.
-      AxisStencil st[2][3];
-      int lb[2][3];
+      AxisStencil st[3];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        st[0][a] = axis_stencil<-1>(xs[a]);
-        st[1][a] = axis_stencil<1>(xs[a]);
-        lb[0][a] = st[0][a].base - 4 * kk[a];
-        lb[1][a] = st[1][a].base - 4 * kk[a];
-      }
+      for (int a = 0; a < 3; ++a) st[a] = axis_stencil(x[a], inv_dx);
       float D6[6], Di6[6], Di[9], DT[9];
-      d_matrix(st, dx, D6);
+      d_matrix(st, D6);
 #pragma unroll
       for (int k = 0; k < 6; ++k) D6[k] = 0.5f * (Dold[k] + D6[k]);
       inv_sym3(D6[0], D6[1], D6[2], D6[3], D6[4], D6[5], Di6);
@@ -866,10 +869,10 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       matmul3(Di, tau, DT);
       float Ah[9];
       bool finite = true;
-      const float sA = ndt * vol_over_mass;
+      const float sA = ndt * vol_over_mass * inv_dx;
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
-        Ah[k] = (C[k] - sA * DT[k]) * dx;
+        Ah[k] = fmaf(-sA, DT[k], Cdx[k]);
         finite &= fabsf(Ah[k]) < kFixMaxValue;
       }
 #pragma unroll
@@ -878,7 +881,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         set_status(scal, kStatusNumeric);
         continue;
       }
-      p2g_scatter(ptile, st, lb, v, Ah);
+      p2g_scatter(ptile, st, key, v, Ah);
     }
     __syncthreads();
 
@@ -976,23 +979,19 @@ __global__ void __launch_bounds__(NT, 2) rasterize_kernel(SceneDev sc, ModelDev 
     const int kk[3] = {key.x, key.y, key.z};
     for (uint32_t q = threadIdx.x; q < n; q += NT) {
       const uint32_t i = start + q;
-      const float xs[3] = {s0.x[0][i] * inv_dx, s0.x[1][i] * inv_dx, s0.x[2][i] * inv_dx};
       const float v[3] = {md.vel_in[3 * i], md.vel_in[3 * i + 1], md.vel_in[3 * i + 2]};
-      AxisStencil st[2][3];
-      int lb[2][3];
+      AxisStencil st[3];
       bool ok = true;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        st[0][a] = axis_stencil<-1>(xs[a]);
-        st[1][a] = axis_stencil<1>(xs[a]);
-        lb[0][a] = st[0][a].base - 4 * kk[a];
-        lb[1][a] = st[1][a].base - 4 * kk[a];
-        ok &= lb[0][a] >= 0 && lb[0][a] <= 6 && lb[1][a] >= 0 && lb[1][a] <= 6;
+        st[a] = axis_stencil(s0.x[a][i], inv_dx);
+        const int l0 = st[a].b[0] - 4 * kk[a], l1 = st[a].b[1] - 4 * kk[a];
+        ok &= l0 >= 0 && l0 <= 6 && l1 >= 0 && l1 <= 6;
       }
       bool finite = fabsf(v[0]) < kFixMaxValue && fabsf(v[1]) < kFixMaxValue && fabsf(v[2]) < kFixMaxValue;
       if (!ok) set_status(scal, kStatusOutsideBlock);
       if (!finite) set_status(scal, kStatusNumeric);
-      if (ok && finite) p2g_scatter(ptile, st, lb, v, Z);
+      if (ok && finite) p2g_scatter(ptile, st, key, v, Z);
     }
     __syncthreads();
     flush_tile<NT>(sc, key, ptile, md.smat ? 1.0 : md.flush_ratio, gd.grid[0]);
@@ -1315,8 +1314,7 @@ __global__ void setup_bin_kernel(SceneDev sc, uint32_t n, const float* __restric
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float px = x[3 * i], py = x[3 * i + 1], pz = x[3 * i + 2];
-  const int cx = static_cast<int>(px * sc.inv_dx + 0.25f), cy = static_cast<int>(py * sc.inv_dx + 0.25f),
-            cz = static_cast<int>(pz * sc.inv_dx + 0.25f);
+  const int cx = cell_of(px, sc.inv_dx), cy = cell_of(py, sc.inv_dx), cz = cell_of(pz, sc.inv_dx);
   const int bx = trunc_div4(cx - 2), by = trunc_div4(cy - 2), bz = trunc_div4(cz - 2);
   uint32_t f = 0xFFFFFFFFu;
   const bool finite = isfinite(px) && isfinite(py) && isfinite(pz) && px >= 0.f && py >= 0.f && pz >= 0.f;
@@ -1450,9 +1448,9 @@ __global__ void __launch_bounds__(NT) setup_order_kernel(SceneDev sc, BlockListD
     // Cell of each particle within the block (the binning's +dx/4 cell).
     for (uint32_t i = threadIdx.x; i < n; i += NT) {
       const uint32_t p = s[i];
-      const int lx = (static_cast<int>(x[3 * p] * sc.inv_dx + 0.25f) - 2 - 4 * key.x) & 3;
-      const int ly = (static_cast<int>(x[3 * p + 1] * sc.inv_dx + 0.25f) - 2 - 4 * key.y) & 3;
-      const int lz = (static_cast<int>(x[3 * p + 2] * sc.inv_dx + 0.25f) - 2 - 4 * key.z) & 3;
+      const int lx = (cell_of(x[3 * p], sc.inv_dx) - 2 - 4 * key.x) & 3;
+      const int ly = (cell_of(x[3 * p + 1], sc.inv_dx) - 2 - 4 * key.y) & 3;
+      const int lz = (cell_of(x[3 * p + 2], sc.inv_dx) - 2 - 4 * key.z) & 3;
       cell[i] = static_cast<uint8_t>(lx * 16 + ly * 4 + lz);
     }
     __syncthreads();
@@ -1511,9 +1509,9 @@ __global__ void __launch_bounds__(NT, 4) reorder_gather_kernel(SceneDev sc, Mode
       }
       src_of[j] = iin;
       // the cell within the block, as setup_order_kernel numbers it ((c - 2) mod 4 per axis)
-      const int lx = (static_cast<int>(sin.x[0][iin] * sc.inv_dx + 0.25f) - 2) & 3;
-      const int ly = (static_cast<int>(sin.x[1][iin] * sc.inv_dx + 0.25f) - 2) & 3;
-      const int lz = (static_cast<int>(sin.x[2][iin] * sc.inv_dx + 0.25f) - 2) & 3;
+      const int lx = (cell_of(sin.x[0][iin], sc.inv_dx) - 2) & 3;
+      const int ly = (cell_of(sin.x[1][iin], sc.inv_dx) - 2) & 3;
+      const int lz = (cell_of(sin.x[2][iin], sc.inv_dx) - 2) & 3;
       cell[j] = static_cast<uint8_t>(lx * 16 + ly * 4 + lz);
     }
     __syncthreads();
@@ -1691,10 +1689,9 @@ __global__ void __launch_bounds__(NT) probe_kernel(SceneDev sc, ModelDev md, Gri
       if (oaux) oaux[o] = (material_has_aux(kind) && sin.aux) ? sin.aux[iin] : 0.f;
       if (oid) oid[o] = pid;
       if (ov) {
-        const float xs[3] = {x[0] * sc.inv_dx, x[1] * sc.inv_dx, x[2] * sc.inv_dx};
-        float v[3], C[9], D6[6];
+        float v[3], Cdx[9], D6[6];
         bool inside = true;
-        g2p(vtile, xs, key, sc.dx, v, C, inside, D6);
+        g2p(vtile, x, sc.inv_dx, key, v, Cdx, inside, D6);
         if (sc.rigid) {  // rigid particles report zero velocity (include/mpm_algorithm.cuh:1316-1325)
           const float f0 = (material_has_F(kind) && sin.F[0]) ? sin.F[0][iin] : 1.f;
           const float a = (material_has_aux(kind) && sin.aux) ? sin.aux[iin] : 1.f;

@@ -1,5 +1,5 @@
-// Device math for the CK-MPM substep: 3x3 helpers, the FP32 SVD, the compact
-// (CK) kernel weights and the three constitutive models on the hot path.
+// Device math for the CK-MPM substep: 3x3 helpers, the FP32 SVD, and
+// the constitutive models of the hot path.
 //
 // Matrices are row-major float[9] like the reference's Matrix<float,3,3>
 // (AppledoreM/CKMPM include/data_type.cuh:32-425).
@@ -12,9 +12,15 @@ namespace ckmpm {
 
 #define CKMPM_DEV __device__ __forceinline__
 
+// Sums of products are written as explicit fused multiply-adds: the compiler may
+// contract a b + c d either way, and not the same way in every instantiation of a
+// kernel, while results must not depend on the launch shape.
+CKMPM_DEV float dot2(float a, float b, float c, float d) { return fmaf(c, d, a * b); }
+CKMPM_DEV float dot3(float a, float b, float c, float d, float e, float f) { return fmaf(e, f, fmaf(c, d, a * b)); }
+
 CKMPM_DEV float det3(const float* a) {
-  return a[0] * (a[4] * a[8] - a[5] * a[7]) - a[1] * (a[3] * a[8] - a[5] * a[6]) +
-         a[2] * (a[3] * a[7] - a[4] * a[6]);
+  return dot3(a[0], dot2(a[4], a[8], -a[5], a[7]), -a[1], dot2(a[3], a[8], -a[5], a[6]), a[2],
+              dot2(a[3], a[7], -a[4], a[6]));
 }
 
 // Adjugate inverse (include/data_type.cuh:369-386).
@@ -34,17 +40,17 @@ CKMPM_DEV void inv3(const float* a, float* r) {
 // Inverse of a symmetric matrix given by its 6 unique entries
 // (d00, d11, d22, d01, d02, d12); writes the 6 unique entries of the inverse.
 CKMPM_DEV void inv_sym3(float d00, float d11, float d22, float d01, float d02, float d12, float* r) {
-  const float c00 = d11 * d22 - d12 * d12;
-  const float c01 = d02 * d12 - d01 * d22;
-  const float c02 = d01 * d12 - d02 * d11;
-  const float det = d00 * c00 + d01 * c01 + d02 * c02;
+  const float c00 = dot2(d11, d22, -d12, d12);
+  const float c01 = dot2(d02, d12, -d01, d22);
+  const float c02 = dot2(d01, d12, -d02, d11);
+  const float det = dot3(d00, c00, d01, c01, d02, c02);
   const float id = 1.0f / det;
   r[0] = id * c00;
-  r[1] = id * (d00 * d22 - d02 * d02);
-  r[2] = id * (d00 * d11 - d01 * d01);
+  r[1] = id * dot2(d00, d22, -d02, d02);
+  r[2] = id * dot2(d00, d11, -d01, d01);
   r[3] = id * c01;
   r[4] = id * c02;
-  r[5] = id * (d01 * d02 - d00 * d12);
+  r[5] = id * dot2(d01, d02, -d00, d12);
 }
 
 CKMPM_DEV void matmul3(const float* a, const float* b, float* r) {
@@ -52,7 +58,7 @@ CKMPM_DEV void matmul3(const float* a, const float* b, float* r) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) t[i * 3 + j] = a[i * 3] * b[j] + a[i * 3 + 1] * b[3 + j] + a[i * 3 + 2] * b[6 + j];
+    for (int j = 0; j < 3; ++j) t[i * 3 + j] = dot3(a[i * 3], b[j], a[i * 3 + 1], b[3 + j], a[i * 3 + 2], b[6 + j]);
 #pragma unroll
   for (int k = 0; k < 9; ++k) r[k] = t[k];
 }
@@ -189,16 +195,6 @@ CKMPM_DEV void svd3(const float* A, float* U, float* S, float* V) {
   S[0] = B[0];
   S[1] = B[4];
   S[2] = B[8];
-}
-
-// ------------------------------------------------------------------ CK weights
-// w0 = 1 - o + sin(2 pi o) / (2 pi) for offset o in [0, 1); node weights are
-// w0 and 1 - w0 along each axis (include/mpm_kernel.cuh:91-114, which also
-// evaluates the sine with the __sinf intrinsic).
-CKMPM_DEV float ck_w0(float o) {
-  const float kTwoPi = 6.283185307179586f;
-  const float kInvTwoPi = 0.15915494309189535f;
-  return 1.0f - o + kInvTwoPi * __sinf(kTwoPi * o);
 }
 
 // ------------------------------------------------------------------ materials
@@ -463,15 +459,13 @@ CKMPM_DEV void stress_linear(const float* C, float dt, const float* F, float* Q,
 // J-fluid: J += tr(C) dt J; p = bulk (J^-gamma - 1); tau = J (visc (C + C^T) - p I)
 // (include/mpm_algorithm.cuh:528-569, include/mpm_material.cuh:468-477).
 CKMPM_DEV void stress_fluid(float bulk, float gamma, float visc, const float* C, float dt, float& J, float* tau) {
-  J += (C[0] + C[4] + C[8]) * dt * J;
-  const float p = bulk * (powf(J, -gamma) - 1.0f);
+  J = fmaf((C[0] + C[4] + C[8]) * dt, J, J);
+  const float p = __fmul_rn(bulk, powf(J, -gamma) - 1.0f);
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) tau[r * 3 + c] = (C[r * 3 + c] + C[c * 3 + r]) * visc;
-  tau[0] -= p;
-  tau[4] -= p;
-  tau[8] -= p;
+    for (int c = 0; c < 3; ++c)
+      tau[r * 3 + c] = r == c ? fmaf(2.0f * C[r * 3 + c], visc, -p) : (C[r * 3 + c] + C[c * 3 + r]) * visc;
 #pragma unroll
   for (int k = 0; k < 9; ++k) tau[k] *= J;
 }
