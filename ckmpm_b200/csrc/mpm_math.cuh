@@ -197,6 +197,140 @@ CKMPM_DEV void svd3(const float* A, float* U, float* S, float* V) {
   S[2] = B[8];
 }
 
+// ------------------------------------------------------------------ left eigenvectors
+//
+// The isotropic stresses need F = U diag(S) V^T only through U, S and
+// F itself: tau = U diag(f(S)) U^T, and a return map that scales the
+// principal stretches by r_i gives F <- U diag(r) U^T F.  So the substep takes the
+// eigenvectors U of b = F F^T by the same cyclic Jacobi as svd3 and the stretches
+// as the column norms of W = F^T U (W_i = S_i V_i), and needs neither V, nor the
+// sorting, nor the QR of svd3.  Norms of F^T u_i keep S_i to rounding of |F|
+// where square roots of the eigenvalues would not.
+//
+// A pair is left unrotated when its off-diagonal is below kLeftNegligible times
+// the trace: leaving it changes U diag(f(S)) U^T by at most that fraction of f,
+// below the rounding of forming b.
+constexpr float kLeftNegligible = 1e-9f;
+
+// c = cos, s = sin and t = tan of the rotation that zeroes apq; (1, 0, 0) when
+// |apq| < tiny.
+CKMPM_DEV void jacobi_angle(float app, float aqq, float apq, float tiny, float& t, float& c, float& s) {
+  const float d = aqq - app, e = 2.0f * apq;
+  const float h2 = fmaf(d, d, e * e);
+  const float den = d + copysignf(h2 * rsqrtf(h2), d);
+  t = fabsf(apq) >= tiny ? __fdividef(e, den) : 0.0f;
+  c = rsqrt_refined(fmaf(t, t, 1.0f));
+  s = t * c;
+}
+
+CKMPM_DEV void left_rotate(float& app, float& aqq, float& apq, float& arp, float& arq, float tiny, float* U, int p,
+                           int q) {
+  if (!(fabsf(apq) >= tiny)) return;
+  float t, c, s;
+  jacobi_angle(app, aqq, apq, tiny, t, c, s);
+  app = fmaf(-t, apq, app);
+  aqq = fmaf(t, apq, aqq);
+  apq = 0.0f;
+  const float rp = arp, rq = arq;
+  arp = dot2(c, rp, -s, rq);
+  arq = dot2(s, rp, c, rq);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float up = U[k * 3 + p], uq = U[k * 3 + q];
+    U[k * 3 + p] = dot2(c, up, -s, uq);
+    U[k * 3 + q] = dot2(s, up, c, uq);
+  }
+}
+
+// U (columns: eigenvectors of F F^T, a proper rotation), W = F^T U and the
+// stretches S = |W_i| >= 0, in no order.
+CKMPM_DEV void left_stretch(const float* F, float* U, float* W, float* S) {
+  float m00 = dot3(F[0], F[0], F[1], F[1], F[2], F[2]);
+  float m11 = dot3(F[3], F[3], F[4], F[4], F[5], F[5]);
+  float m22 = dot3(F[6], F[6], F[7], F[7], F[8], F[8]);
+  float m01 = dot3(F[0], F[3], F[1], F[4], F[2], F[5]);
+  float m02 = dot3(F[0], F[6], F[1], F[7], F[2], F[8]);
+  float m12 = dot3(F[3], F[6], F[4], F[7], F[5], F[8]);
+  const float tiny = fmaxf(kLeftNegligible * (m00 + m11 + m22), 1e-18f);  // 1e-18 squared stays normal
+#pragma unroll
+  for (int k = 0; k < 9; ++k) U[k] = (k & 3) ? 0.0f : 1.0f;
+  if (!(fmaxf(fmaxf(fabsf(m01), fabsf(m02)), fabsf(m12)) < tiny)) {
+    // First sweep written out on U = I.
+    float t, c, s;
+    jacobi_angle(m00, m11, m01, tiny, t, c, s);
+    m00 = fmaf(-t, m01, m00);
+    m11 = fmaf(t, m01, m11);
+    const float q02 = dot2(c, m02, -s, m12), q12 = dot2(s, m02, c, m12);
+    float t2, c2, s2;
+    jacobi_angle(m00, m22, q02, tiny, t2, c2, s2);
+    m00 = fmaf(-t2, q02, m00);
+    m22 = fmaf(t2, q02, m22);
+    m01 = -s2 * q12;
+    m12 = c2 * q12;
+    U[0] = c2 * c;
+    U[3] = -c2 * s;
+    U[6] = -s2;
+    const float u02 = s2 * c, u12 = -s2 * s;
+    float t3, c3, s3;
+    jacobi_angle(m11, m22, m12, tiny, t3, c3, s3);
+    m11 = fmaf(-t3, m12, m11);
+    m22 = fmaf(t3, m12, m22);
+    m02 = s3 * m01;
+    m01 = c3 * m01;
+    m12 = 0.0f;
+    U[1] = dot2(c3, s, -s3, u02);
+    U[4] = dot2(c3, c, -s3, u12);
+    U[7] = -s3 * c2;
+    U[2] = dot2(s3, s, c3, u02);
+    U[5] = dot2(s3, c, c3, u12);
+    U[8] = c3 * c2;
+#pragma unroll
+    for (int sweep = 1; sweep < 3; ++sweep) {
+      left_rotate(m00, m11, m01, m02, m12, tiny, U, 0, 1);
+      left_rotate(m00, m22, m02, m01, m12, tiny, U, 0, 2);
+      left_rotate(m11, m22, m12, m01, m02, tiny, U, 1, 2);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) W[k * 3 + i] = dot3(F[k], U[i], F[3 + k], U[3 + i], F[6 + k], U[6 + i]);
+    const float n2 = dot3(W[i], W[i], W[3 + i], W[3 + i], W[6 + i], W[6 + i]);
+    S[i] = n2 > 0.0f ? n2 * rsqrt_refined(n2) : n2;
+  }
+}
+
+// U diag(d) U^T (symmetric).
+CKMPM_DEV void left_diag(const float* U, const float* d, float* r9) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const float a = U[r * 3] * d[0], b = U[r * 3 + 1] * d[1], e = U[r * 3 + 2] * d[2];
+#pragma unroll
+    for (int c = r; c < 3; ++c) {
+      const float v = dot3(a, U[c * 3], b, U[c * 3 + 1], e, U[c * 3 + 2]);
+      r9[r * 3 + c] = v;
+      r9[c * 3 + r] = v;
+    }
+  }
+}
+
+// F = U diag(r) W^T.
+CKMPM_DEV void left_rescale(const float* U, const float* r, const float* W, float* F) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float a = U[i * 3] * r[0], b = U[i * 3 + 1] * r[1], e = U[i * 3 + 2] * r[2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) F[i * 3 + k] = dot3(a, W[k * 3], b, W[k * 3 + 1], e, W[k * 3 + 2]);
+  }
+}
+
+// Whether the smallest stretch is large enough against the largest for W_i / S_i
+// to stand for V_i: the error of W_i is that of |F|, so V_i's is S_max / S_min
+// times rounding.  Beyond 4 (and for a NaN) the return maps take svd3's V.
+CKMPM_DEV bool left_well_conditioned(const float* S) {
+  return fminf(fminf(S[0], S[1]), S[2]) > 0.25f * fmaxf(fmaxf(S[0], S[1]), S[2]);
+}
+
 // ------------------------------------------------------------------ materials
 // Numbering of MPMConstitutiveModel (include/mpm_material.cuh:10-18).
 enum MaterialKind : int32_t {
@@ -218,33 +352,44 @@ struct MaterialParams {
 };
 
 // Fixed-corotated Kirchhoff stress, tau = U diag(2 mu s (s - 1) + lambda J (J - 1)) U^T
-// (include/mpm_material.cuh:320-357).
+// (include/mpm_material.cuh:320-357), where the smallest stretch takes the sign of det F.
 CKMPM_DEV void stress_fixed_corotated(float lambda, float mu, const float* F, float* tau) {
-  float U[9], S[3], V[9];
-  svd3(F, U, S, V);
-  const float J = S[0] * S[1] * S[2];
+  float U[9], W[9], S[3];
+  left_stretch(F, U, W, S);
+  const float J = det3(F);
+  if (J < 0.0f) {
+    const float least = fminf(fminf(S[0], S[1]), S[2]);
+    if (S[2] == least) S[2] = -S[2];
+    else if (S[1] == least) S[1] = -S[1];
+    else S[0] = -S[0];
+  }
   const float lj = lambda * J * (J - 1.0f);
   float sc[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) sc[i] = 2.0f * mu * S[i] * (S[i] - 1.0f) + lj;
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = r; c < 3; ++c) {
-      const float v = U[r * 3] * sc[0] * U[c * 3] + U[r * 3 + 1] * sc[1] * U[c * 3 + 1] + U[r * 3 + 2] * sc[2] * U[c * 3 + 2];
-      tau[r * 3 + c] = v;
-      tau[c * 3 + r] = v;
-    }
+  for (int i = 0; i < 3; ++i) sc[i] = fmaf(2.0f * mu * S[i], S[i] - 1.0f, lj);
+  left_diag(U, sc, tau);
 }
 
 // Drucker-Prager StVK-Hencky return map with the reference's constants:
 // zero cohesion, beta = 1, volume correction on, sin(phi) = 0.5
 // (include/mpm_material.cuh:362-464).  Updates F and logJp in place.
+//
+// The reference computes tau = U diag(p) V^T F^T with p = (2 mu log s + lambda tr log s) / s
+// after F <- U diag(s) V^T; V^T F^T = diag(s) U^T, so tau = U diag(2 mu log s + lambda tr log s) U^T,
+// and log s is known: 0 on the tension branch (s = 1), H elsewhere.
+// An elastic step (dg <= 0, stretches within the clamp) leaves F as it is.
 CKMPM_DEV void stress_drucker_prager(float lambda, float mu, float* F, float& logJp, float* tau) {
   const float kYs = 0.816496580927726f * 2.0f * 0.5f / (3.0f - 0.5f);
   const float smu = 2.0f * mu;
-  float U[9], S[3], V[9];
-  svd3(F, U, S, V);
+  float U[9], W[9], S[3];
+  left_stretch(F, U, W, S);
+  const bool good = left_well_conditioned(S) && S[0] > 4e-4f;
+  if (!good) {
+    float V[9];
+    svd3(F, U, S, V);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) W[i] = V[i];
+  }
   float eps[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) eps[i] = logf(fmaxf(fabsf(S[i]), 1e-4f));
@@ -252,100 +397,73 @@ CKMPM_DEV void stress_drucker_prager(float lambda, float mu, float* F, float& lo
   const float etr = esum + logJp;
   float eh[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) eh[i] = eps[i] - etr / 3.0f;
-  const float ehn = sqrtf(eh[0] * eh[0] + eh[1] * eh[1] + eh[2] * eh[2]);
-  float ns[3];
-  if (etr >= 0.0f) {
-    ns[0] = ns[1] = ns[2] = 1.0f;
-    logJp = esum + logJp;
-  } else {
-    logJp = 0.0f;
-    const float dg = ehn + (3.0f * lambda + smu) / smu * etr * kYs;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const float H = dg <= 0.0f ? eps[i] : eps[i] - (dg / ehn) * eh[i];
-      ns[i] = expf(H);
-    }
-  }
-  // F <- U diag(ns) V^T
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      F[r * 3 + c] = U[r * 3] * ns[0] * V[c * 3] + U[r * 3 + 1] * ns[1] * V[c * 3 + 1] + U[r * 3 + 2] * ns[2] * V[c * 3 + 2];
-  // tau = U diag(p) V^T F^T with p = (2 mu log s + lambda tr log s) / s (the reference's order,
-  // include/mpm_material.cuh:447-463).  With F = U diag(s) V^T and V orthogonal,
-  // V^T F^T = diag(s) U^T, so tau = U diag(2 mu log s + lambda tr log s) U^T: symmetric, and
-  // 36 multiply-adds and three divisions fewer per particle (1.7 % of the fused substep on the
-  // sand column).  log s is 0 on the tension branch (s = 1), and log(exp(H)) there otherwise.
+  for (int i = 0; i < 3; ++i) eh[i] = fmaf(etr, -1.0f / 3.0f, eps[i]);
+  const float ehn = sqrtf(dot3(eh[0], eh[0], eh[1], eh[1], eh[2], eh[2]));
+  const bool tension = etr >= 0.0f;
+  logJp = tension ? etr : 0.0f;
+  const float dg = fmaf(fmaf(3.0f, lambda, smu) / smu * kYs, etr, ehn);
+  const float k = !tension && dg > 0.0f ? dg / ehn : 0.0f;
   float h[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) h[i] = etr >= 0.0f ? 0.0f : logf(ns[i]);
+  for (int i = 0; i < 3; ++i) h[i] = tension ? 0.0f : fmaf(-k, eh[i], eps[i]);
+  if (tension || k > 0.0f || !good) {
+    // Ratio of the new stretch to |W_i| (S_i, or 1 where W holds V).
+    float r[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) r[i] = expf(good ? h[i] - eps[i] : h[i]);
+    left_rescale(U, r, W, F);
+  }
   const float trh = h[0] + h[1] + h[2];
   float sc[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) sc[i] = smu * h[i] + lambda * trh;
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = r; c < 3; ++c) {
-      const float v = U[r * 3] * sc[0] * U[c * 3] + U[r * 3 + 1] * sc[1] * U[c * 3 + 1] + U[r * 3 + 2] * sc[2] * U[c * 3 + 2];
-      tau[r * 3 + c] = v;
-      tau[c * 3 + r] = v;
-    }
+  for (int i = 0; i < 3; ++i) sc[i] = dot2(smu, h[i], lambda, trh);
+  left_diag(U, sc, tau);
 }
 
 // Von Mises plasticity on the Hencky strain of the trial elastic F, then the
-// StVK-Hencky stress of the projected F from its own SVD, as the reference
-// computes it (include/mpm_algorithm.cuh:404-520, include/mpm_material.cuh:480-518):
+// StVK-Hencky stress of the projected F (include/mpm_algorithm.cuh:404-520,
+// include/mpm_material.cuh:480-518):
 //   eps = log S, eps_hat = eps - tr(eps) / 3, f = |eps_hat| - yield / (2 mu);
 //   f > 0: S <- exp(eps - f eps_hat / |eps_hat|), Fe <- U diag(S) V^T;
-//   tau = U diag((2 mu log S + lambda tr log S) / S) V^T Fe^T.
-// Fe holds the trial elastic F on entry and the projected one on exit.
+//   tau = U diag((2 mu log S + lambda tr log S) / S) V^T Fe^T = U diag(2 mu log S + lambda tr log S) U^T.
+// The reference takes a second SVD for the projected Fe; its U and log S are
+// the ones at hand.  Fe holds the trial elastic F on entry and the projected one on exit.
+// An inverted Fe (S_2 < 0) has no Hencky strain: NaN, as log S gives.
 CKMPM_DEV void stress_von_mises(float mu, float lambda, float yield, float* Fe, float* tau) {
-  float U[9], S[3], V[9];
-  svd3(Fe, U, S, V);
+  float U[9], W[9], S[3];
+  left_stretch(Fe, U, W, S);
+  const bool good = left_well_conditioned(S) && det3(Fe) > 0.0f;
+  if (!good) {
+    float V[9];
+    svd3(Fe, U, S, V);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) W[i] = V[i];
+  }
   float eps[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) eps[i] = logf(S[i]);
   const float etr = eps[0] + eps[1] + eps[2];
   float eh[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) eh[i] = eps[i] - etr / 3.0f;
-  const float ehn = sqrtf(eh[0] * eh[0] + eh[1] * eh[1] + eh[2] * eh[2]);
+  for (int i = 0; i < 3; ++i) eh[i] = fmaf(etr, -1.0f / 3.0f, eps[i]);
+  const float ehn = sqrtf(dot3(eh[0], eh[0], eh[1], eh[1], eh[2], eh[2]));
   const float yf = ehn - yield / (2.0f * mu);
+  float h[3] = {eps[0], eps[1], eps[2]};
   if (yf > 0.0f) {
-    float ns[3];
+    const float k = yf / ehn;
+    float r[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) ns[i] = expf(eps[i] - yf * eh[i] / ehn);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        Fe[r * 3 + c] = U[r * 3] * ns[0] * V[c * 3] + U[r * 3 + 1] * ns[1] * V[c * 3 + 1] + U[r * 3 + 2] * ns[2] * V[c * 3 + 2];
+    for (int i = 0; i < 3; ++i) {
+      h[i] = fmaf(-k, eh[i], eps[i]);
+      r[i] = expf(good ? -k * eh[i] : h[i]);
+    }
+    left_rescale(U, r, W, Fe);
   }
-  svd3(Fe, U, S, V);
-  float ls[3];
+  const float trh = h[0] + h[1] + h[2];
+  float sc[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) ls[i] = logf(S[i]);
-  const float lsum = ls[0] + ls[1] + ls[2];
-  float ph[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const float inv = 1.0f / S[i];
-    ph[i] = 2.0f * mu * inv * ls[i] + lambda * lsum * inv;
-  }
-  float P[9];
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      P[r * 3 + c] = U[r * 3] * ph[0] * V[c * 3] + U[r * 3 + 1] * ph[1] * V[c * 3 + 1] + U[r * 3 + 2] * ph[2] * V[c * 3 + 2];
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      tau[r * 3 + c] = P[r * 3] * Fe[c * 3] + P[r * 3 + 1] * Fe[c * 3 + 1] + P[r * 3 + 2] * Fe[c * 3 + 2];
+  for (int i = 0; i < 3; ++i) sc[i] = dot2(2.0f * mu, h[i], lambda, trh);
+  left_diag(U, sc, tau);
 }
 
 // Non-associated Cam-clay (include/mpm_material.cuh:520-669, driven from
