@@ -440,6 +440,14 @@ def run_diff(args, rank, world, local_rank):
     return line
 
 
+def substep_launches(cfg, n_models: int, n_scenes: int = 1) -> int:
+    """Kernel launches of one substep: per model the fused kernel, the compaction (two kernels in a domain of more
+    than 16384 blocks) and the window zeroing, which the compaction of a small domain with few blocks includes; the
+    last launch also ends the substep."""
+    entries = n_scenes * int(np.prod(cfg.domain_blocks))
+    return n_models * (2 if entries <= 16384 else 4)
+
+
 def run_batched(args, rank, world, local_rank):
     """Batched form: this rank's shard of the 256 scenes in one SceneBatch
     (one persistent fused launch + rebinning per substep, CUDA graphs), launch
@@ -587,7 +595,7 @@ def run_batched(args, rank, world, local_rank):
                    "tuning": best, "tuning_candidates": len(tried),
                    "l2": "particle state ~560 MB > 126 MB L2: no flush"},
         "roofline": roofline, "e2e": e2e, "clocks": clocks,
-        "gpu_launches": 1 + args.steps * 5,
+        "gpu_launches": 1 + args.steps * substep_launches(cfg, 1, len(sub)),
     }
     if looped:
         line["looped_plain"] = looped
@@ -742,7 +750,7 @@ def run_ours(args, rank, world, local_rank):
                    "tuning": {k: tuning[k] for k in ("threads", "ctas_per_sm", "graph_chunk")},
                    "l2": "particle state ~190 MB > 126 MB L2: no flush"},
         "roofline": roofline, "e2e": e2e, "clocks": clocks,
-        "gpu_launches": 1 + args.steps * (4 * len(models) + 1),  # per model: fused, 2 compaction, zero; + end
+        "gpu_launches": 1 + args.steps * substep_launches(cfg, len(models)),
     }
     return line
 

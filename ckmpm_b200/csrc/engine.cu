@@ -87,8 +87,8 @@ struct ckmpm_scene {
   std::vector<std::pair<void*, size_t>> allocs;
   size_t n_state_allocs = 0;
   cudaGraphExec_t graph_chunk = nullptr;
-  cudaGraphExec_t graph_one = nullptr;
   uint64_t host_step = 0;
+  uint32_t nblocks0 = 0;   // active blocks at setup (the largest model's)
   // Substeps between re-layouts of the particles (reorder_gather_kernel); 0 = never.
   uint32_t reorder_every = kReorderEvery;
   uint64_t last_reorder = 0;
@@ -144,8 +144,7 @@ cudaError_t dalloc(ckmpm_scene* s, T** p, size_t count) {
 
 void free_graphs(ckmpm_scene* s) {
   if (s->graph_chunk) cudaGraphExecDestroy(s->graph_chunk);
-  if (s->graph_one) cudaGraphExecDestroy(s->graph_one);
-  s->graph_chunk = s->graph_one = nullptr;
+  s->graph_chunk = nullptr;
 }
 
 template <int KIND, int NT, bool RIGID>
@@ -242,13 +241,30 @@ cudaError_t fused_attributes(int device, int* occ4) {
   return cudaSuccess;
 }
 
-// Compaction of one model's next block list into list `out`.
-cudaError_t launch_compact(ckmpm_scene* s, const ModelHost& m, const BlockListDev& out) {
-  compact_reduce_kernel<<<m.ntiles, kCompactThreads, 0, s->stream>>>(s->sc, m.dev.dense_total, m.dev.tile_sums);
-  compact_scatter_kernel<<<m.ntiles, kCompactThreads, 0, s->stream>>>(s->sc, m.dev.dense_total, m.dev.tile_sums, out,
-                                                                       m.dev.cap_slots, m.dev.ticket, s->scal);
+// Compaction of one model's next block list, bl[list], from the totals of `parity`.
+// With `zero_grid` >= 0 it also zeroes the windows of its blocks in that grid (epoch
+// step + 2) and, `end`, ends the substep.
+cudaError_t launch_compact(const SceneDev& sc, const ModelDev& d, const GridDev& gd, Scalars* scal, uint32_t ntiles,
+                           cudaStream_t st, int list, int parity, int zero_grid = -1, bool end = false) {
+  if (sc.tile_shift == 10)
+    compact_reduce_kernel<4><<<ntiles, kCompactThreads, 0, st>>>(sc, d.dense_total[parity], d.tile_sums);
+  auto launch = [&](auto kernel) {
+    const int z = zero_grid < 0 ? 0 : zero_grid;
+    kernel<<<ntiles, kCompactThreads, 0, st>>>(sc, d.dense_total[parity], d.dense_total[parity ^ 1], d.tile_sums,
+                                               d.bl[list], d.cap_slots, d.ticket, scal, gd.grid[z], gd.stamp[z], 2,
+                                               end ? 1 : 0);
+  };
+  if (sc.tile_shift == 10) launch(compact_scatter_kernel<4, false>);
+  else if (zero_grid < 0) launch(compact_scatter_kernel<1, false>);
+  else launch(compact_scatter_kernel<1, true>);
   return cudaGetLastError();
 }
+
+cudaError_t launch_compact(ckmpm_scene* s, const ModelHost& m, int list, int parity, int zero_grid = -1, bool end = false) {
+  return launch_compact(s->sc, m.dev, s->grid, s->scal, m.ntiles, s->stream, list, parity, zero_grid, end);
+}
+
+uint32_t compact_tiles(const SceneDev& sc) { return (sc.nblocks_domain + (1u << sc.tile_shift) - 1) >> sc.tile_shift; }
 
 __global__ void set_next_dt_kernel(Scalars* scal, float dt) {
   if (threadIdx.x == 0) {
@@ -262,38 +278,50 @@ __global__ void set_frame_end_kernel(Scalars* scal, double frame_time) {
 }
 
 // Zero (and stamp with step + epoch_offset) the blocks of grid[grid_parity]
-// that a substep over block lists bl[list_parity] deposits into.
-cudaError_t launch_zero(ckmpm_scene* s, int list_parity, int grid_parity, int32_t epoch_offset) {
+// that a substep over block lists bl[list_parity] deposits into; with `end`, the
+// last model's launch also ends the substep.
+cudaError_t launch_zero(ckmpm_scene* s, int list_parity, int grid_parity, int32_t epoch_offset, bool end) {
   for (auto& m : s->models)
     zero_windows_kernel<<<s->sm_count * 4, 256, 0, s->stream>>>(s->sc, m.dev.bl[list_parity],
                                                                  s->grid.grid[grid_parity],
-                                                                 s->grid.stamp[grid_parity], s->scal, epoch_offset);
+                                                                 s->grid.stamp[grid_parity], s->scal, epoch_offset,
+                                                                 end && &m == &s->models.back() ? 1 : 0);
   return cudaGetLastError();
 }
 
-// Enqueue one substep for every model.  The compaction of each model writes
-// the block list the fused kernel did not read: that of the other parity.
-// Once every model's fused kernel has read grid[parity], its blocks that the
-// next substep deposits into are zeroed for it (epoch step + 2).
-cudaError_t enqueue_substep(ckmpm_scene* s, int parity_of_step) {
+// Whether the compaction also zeroes the next windows: in a small domain with few
+// blocks (a tile's CTA clears its own blocks' windows, up to 1 MB; spread over the whole
+// GPU by a kernel of its own that takes less time than the launch it costs only from
+// about a thousand blocks).
+bool folds_zero(const SceneDev& sc, uint32_t nblocks) { return sc.tile_shift == 8 && nblocks <= 1024u; }
+
+// Enqueue one substep for every model: two launches each (fused; compaction and
+// zeroing) in a small scene, else three in a small domain and four in a large one,
+// where the compaction is two.  The last launch also ends the substep.
+// The compaction of each model writes the block list the fused kernel did not
+// read: that of the other parity.  Once every model's fused kernel has read
+// grid[parity], its blocks that the next substep deposits into are zeroed for it
+// (epoch step + 2).
+cudaError_t enqueue_substep(ckmpm_scene* s, int parity) {
+  cudaError_t e = cudaSuccess;
+  const bool fold = folds_zero(s->sc, s->nblocks0);
   for (auto& m : s->models) {
-    cudaError_t e = launch_fused_any(s, m);
-    if (e != cudaSuccess) return e;
-    e = launch_compact(s, m, m.dev.bl[parity_of_step ^ 1]);
-    if (e != cudaSuccess) return e;
+    if (e == cudaSuccess) e = launch_fused_any(s, m);
+    if (e == cudaSuccess && !fold) e = launch_compact(s, m, parity ^ 1, parity);
   }
-  cudaError_t e = launch_zero(s, parity_of_step ^ 1, parity_of_step, 2);
-  if (e != cudaSuccess) return e;
-  end_substep_kernel<<<1, 32, 0, s->stream>>>(s->scal);
-  return cudaGetLastError();
+  if (!fold) return e == cudaSuccess ? launch_zero(s, parity ^ 1, parity, 2, true) : e;
+  for (auto& m : s->models)
+    if (e == cudaSuccess) e = launch_compact(s, m, parity ^ 1, parity, parity, &m == &s->models.back());
+  return e;
 }
 
-cudaError_t build_graph(ckmpm_scene* s, int nsub, int first_parity, cudaGraphExec_t* exec) {
+// A graph of nsub substeps, the first of even parity.
+cudaError_t build_graph(ckmpm_scene* s, int nsub, cudaGraphExec_t* exec) {
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return e;
   for (int i = 0; i < nsub; ++i) {
-    e = enqueue_substep(s, (first_parity + i) & 1);
+    e = enqueue_substep(s, i & 1);
     if (e != cudaSuccess) break;
   }
   cudaError_t e2 = cudaStreamEndCapture(s->stream, &g);
@@ -524,6 +552,7 @@ static void io_layout(ModelHost& m, bool track, Carve& c) {
 // block lists, the binning totals, compaction partials, the work ticket, the
 // sorted initial velocities and a batch's per-scene tables.
 static void state_layout(ModelHost& m, uint32_t nbd, bool track, Carve& c) {
+  const bool s_small = nbd <= kSmallDomain;
   ModelDev& d = m.dev;
   const size_t n = m.n;
   const bool batch = m.mat.kind == kMixedKind;
@@ -547,8 +576,10 @@ static void state_layout(ModelHost& m, uint32_t nbd, bool track, Carve& c) {
     bl.nblocks = c.take<uint32_t>(1);
     bl.nparticles = c.take<uint32_t>(1);
   }
-  d.dense_total = c.take<uint32_t>(nbd);
-  d.tile_sums = c.take<uint32_t>(2 * static_cast<size_t>(m.ntiles));
+  // A small domain's compaction clears the other parity's totals (compact_scatter_kernel).
+  d.dense_total[0] = c.take<uint32_t>(nbd);
+  d.dense_total[1] = s_small ? c.take<uint32_t>(nbd) : d.dense_total[0];
+  d.tile_sums = c.take<unsigned long long>(m.ntiles);
   d.ticket = c.take<uint32_t>(1);
   d.vel_in = c.take<float>(3 * n);
   d.smat = batch ? c.take<SceneMat>(m.smat.size()) : nullptr;
@@ -565,7 +596,7 @@ static cudaError_t alloc_state(ckmpm_scene* s, ModelHost& m) {
   const bool track = m.mat.kind == kMixedKind || (s->desc.flags & CKMPM_FLAG_TRACK_IDS) != 0;
   d.cap_particles = m.n;
   d.cap_slots = std::max<uint32_t>(1, std::min<uint32_t>(nbd, m.n));
-  m.ntiles = (nbd + kCompactTile - 1) / kCompactTile;
+  m.ntiles = compact_tiles(s->sc);
   Carve size;
   state_layout(m, nbd, track, size);
   void* arena = nullptr;
@@ -843,7 +874,7 @@ ckmpm_status ckmpm_setup(ckmpm_scene* s) {
       CK_CUDA(s, cudaMemsetAsync(d.bl[b].nblocks, 0, sizeof(uint32_t), s->stream));
       CK_CUDA(s, cudaMemsetAsync(d.bl[b].nparticles, 0, sizeof(uint32_t), s->stream));
     }
-    CK_CUDA(s, cudaMemsetAsync(d.dense_total, 0, sizeof(uint32_t) * nbd, s->stream));
+    for (int b = 0; b < 2; ++b) CK_CUDA(s, cudaMemsetAsync(d.dense_total[b], 0, sizeof(uint32_t) * nbd, s->stream));
     CK_CUDA(s, cudaMemsetAsync(d.ticket, 0, sizeof(uint32_t), s->stream));
     if (batch) {
       CK_CUDA(s, cudaMemcpyAsync(const_cast<SceneMat*>(d.smat), m.smat.data(), sizeof(SceneMat) * m.smat.size(),
@@ -860,8 +891,8 @@ ckmpm_status ckmpm_setup(ckmpm_scene* s) {
     uint32_t* flat = sort_array(m, 0);
     uint32_t* cursor = sort_array(m, 1);
     uint32_t* perm = sort_array(m, 2);
-    setup_bin_kernel<<<(n + 255) / 256, 256, 0, s->stream>>>(s->sc, n, m.ox, d.sstart, flat, d.dense_total);
-    CK_CUDA(s, launch_compact(s, m, d.bl[0]));
+    setup_bin_kernel<<<(n + 255) / 256, 256, 0, s->stream>>>(s->sc, n, m.ox, d.sstart, flat, d.dense_total[1]);
+    CK_CUDA(s, launch_compact(s, m, 0, 1));  // as if substep -1 had binned the input
     CK_CUDA(s, cudaMemsetAsync(cursor, 0, sizeof(uint32_t) * d.cap_slots, s->stream));
     setup_place_kernel<<<(n + 255) / 256, 256, 0, s->stream>>>(n, flat, d.bl[0], cursor, perm);
     setup_order_kernel<256><<<s->sm_count * 4, 256, 0, s->stream>>>(s->sc, d.bl[0], m.ox, perm, s->scal);
@@ -877,7 +908,7 @@ ckmpm_status ckmpm_setup(ckmpm_scene* s) {
   }
   // Initial grid: every model deposits mass and momentum into grid[0], epoch 0;
   // then the blocks substep 0 deposits into are zeroed in grid[1] (epoch 1).
-  CK_CUDA(s, launch_zero(s, 0, 0, 0));
+  CK_CUDA(s, launch_zero(s, 0, 0, 0, false));
   for (auto& m : s->models) {
     CK_CUDA(s, cudaMemsetAsync(m.dev.ticket, 0, sizeof(uint32_t), s->stream));
     rasterize_kernel<kFusedThreads><<<s->fused_ctas, kFusedThreads, kSmemFused, s->stream>>>(s->sc, m.dev, s->grid,
@@ -885,13 +916,16 @@ ckmpm_status ckmpm_setup(ckmpm_scene* s) {
     CK_CUDA(s, cudaGetLastError());
     CK_CUDA(s, cudaMemsetAsync(m.dev.ticket, 0, sizeof(uint32_t), s->stream));
   }
-  CK_CUDA(s, launch_zero(s, 0, 1, 1));
+  CK_CUDA(s, launch_zero(s, 0, 1, 1, false));
   // The scalars were zeroed at creation; setup's kernels may have raised status
   // bits in them, which ckmpm_setup then reports.
   finish_setup_kernel<<<1, 32, 0, s->stream>>>(s->scal, 0u, s->rigid_v[0], s->rigid_v[1], s->rigid_v[2]);
   CK_CUDA(s, cudaGetLastError());
   // The one wait of setup: the status word and each model's binned count.
-  std::vector<uint32_t> binned(s->models.size(), 0u);
+  std::vector<uint32_t> binned(s->models.size(), 0u), blocks(s->models.size(), 0u);
+  for (size_t i = 0; i < s->models.size(); ++i)
+    CK_CUDA(s, cudaMemcpyAsync(&blocks[i], s->models[i].dev.bl[0].nblocks, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                               s->stream));
   for (size_t i = 0; i < s->models.size(); ++i)
     CK_CUDA(s, cudaMemcpyAsync(&binned[i], s->models[i].dev.bl[0].nparticles, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                s->stream));
@@ -899,6 +933,7 @@ ckmpm_status ckmpm_setup(ckmpm_scene* s) {
   CK_CUDA(s, cudaMemcpyAsync(&r, s->scal, sizeof(Scalars), cudaMemcpyDeviceToHost, s->stream));
   CK_CUDA(s, cudaStreamSynchronize(s->stream));
   for (size_t i = 0; i < s->models.size(); ++i) s->models[i].n_valid = binned[i];
+  s->nblocks0 = *std::max_element(blocks.begin(), blocks.end());
   s->setup_done = true;
   s->host_step = 0;
   s->n_state_allocs = s->allocs.size();
@@ -978,7 +1013,7 @@ ckmpm_status ckmpm_step_async(ckmpm_scene* s, uint32_t nsteps, float dt) {
     const int parity = static_cast<int>(s->host_step & 1);
     const uint32_t chunk = s->tune.graph_chunk;
     if (parity == 0 && nsteps - done >= chunk && !reorder_inside(s, chunk)) {
-      if (!s->graph_chunk) CK_CUDA(s, build_graph(s, static_cast<int>(chunk), 0, &s->graph_chunk));
+      if (!s->graph_chunk) CK_CUDA(s, build_graph(s, static_cast<int>(chunk), &s->graph_chunk));
       CK_CUDA(s, cudaGraphLaunch(s->graph_chunk, s->stream));
       done += chunk;
       s->host_step += chunk;
@@ -1315,7 +1350,7 @@ ckmpm_status ckmpm_autotune(ckmpm_scene* s, uint32_t probe_steps, float dt, ckmp
   // Applying the pick dropped the graphs of the last probed shape: capture the
   // chosen shape's chunk graph now (capture runs nothing), so that the first
   // ckmpm_step_async after tuning does not pay for it.
-  CK_CUDA(s, build_graph(s, static_cast<int>(s->tune.graph_chunk), 0, &s->graph_chunk));
+  CK_CUDA(s, build_graph(s, static_cast<int>(s->tune.graph_chunk), &s->graph_chunk));
   return CKMPM_OK;
 }
 
@@ -1437,11 +1472,10 @@ ckmpm_status ckmpm_step_profiled(ckmpm_scene* s, uint32_t nsteps, float dt, doub
       CK_CUDA(s, cudaEventRecord(E[0], s->stream));
       CK_CUDA(s, launch_fused_any(s, m));
       CK_CUDA(s, cudaEventRecord(E[1], s->stream));
-      CK_CUDA(s, launch_compact(s, m, m.dev.bl[parity ^ 1]));
-      if (mi + 1 == nm) CK_CUDA(s, launch_zero(s, parity ^ 1, parity, 2));
+      CK_CUDA(s, launch_compact(s, m, parity ^ 1, parity));
+      if (mi + 1 == nm) CK_CUDA(s, launch_zero(s, parity ^ 1, parity, 2, true));
       CK_CUDA(s, cudaEventRecord(E[2], s->stream));
     }
-    end_substep_kernel<<<1, 32, 0, s->stream>>>(s->scal);
     ++s->host_step;
   }
   CK_CUDA(s, cudaStreamSynchronize(s->stream));

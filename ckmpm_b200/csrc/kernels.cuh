@@ -43,8 +43,11 @@ constexpr int kMaxParticlesPerBlock = 4096;  // u16 in-block index, 64 per cell 
 constexpr int kTileRow = 68;
 constexpr int kTileNodes = 2 * 8 * kTileRow;  // 2 grids x 8 x planes around a particle block
 constexpr int kCompactThreads = 256;
-constexpr int kCompactPerThread = 4;
-constexpr int kCompactTile = kCompactThreads * kCompactPerThread;
+// Traversal entries per thread of the compaction, and so per CTA: 4 (1024 a CTA), or 1
+// in a domain of at most kSmallDomain entries, which would otherwise fill a few SMs only.
+constexpr uint32_t kSmallDomain = 16384;
+constexpr uint32_t tile_shift_of(uint32_t entries) { return entries <= kSmallDomain ? 8u : 10u; }
+static_assert(kCompactThreads == 256, "tiles of 2^8 and 2^10 entries");
 constexpr float kFixScale = 68719476736.0f;        // 2^36: P2G fixed-point scale (per unit particle mass)
 constexpr float kFixInvScale = 1.4551915228366852e-11f;  // 2^-36
 constexpr float kFixMaxValue = 131072.0f;          // |contribution| bound per unit mass (2^17)
@@ -68,6 +71,7 @@ struct SceneDev {
   uint32_t ccount[8];    // blocks of each colour class in one domain
   uint32_t nstack;       // stacked domains (1 for a single scene, the scene count for a batch)
   uint32_t nblocks_domain;  // table entries over all stacked domains
+  uint32_t tile_shift;      // log2 of the compaction's tile
   float grid_unit;       // single scene: mass of one fixed-point unit (heaviest model's mass x 2^-36)
   int32_t rigid;         // rigid particles on (the velocity is Scalars::rigid_v)
   const uint8_t* brule;  // boundary == 2: per-cell rule (ckmpm_cell_rule), x-major over the domain's cells
@@ -99,13 +103,14 @@ struct Scalars {
   double cur_dt_d;     // cur_dt / next_dt in double, as the reference keeps its clock
   double next_dt_d;
   float rigid_v[3];    // velocity of rigid particles (when SceneDev::rigid)
+  uint32_t ctas_done;  // CTAs of the substep's last kernel that have finished (zero between kernels)
 };
 
 struct BlockListDev {
   int4* keys;           // block coordinate and colour
   uint32_t* start;      // first particle of the block in the state arrays
   uint32_t* count;      // particles in the block
-  int32_t* table;       // dense: block -> slot, -1 when inactive
+  int32_t* table;       // dense, by traversal index: block -> slot, -1 when inactive
   uint32_t* prefix28;   // per slot: prefix counts of outgoing directions (written by the fused kernel)
   uint16_t* idx;        // per particle: in-block position, grouped by outgoing direction
   uint32_t* nblocks;    // device scalar: active particle blocks
@@ -139,8 +144,8 @@ __host__ __device__ __forceinline__ float rigid_attribute(int kind, const float*
 struct ModelDev {
   StateDev st[2];
   BlockListDev bl[2];
-  uint32_t* dense_total;  // per domain block: particles binned into it (zero between uses)
-  uint32_t* tile_sums;    // compaction partials
+  uint32_t* dense_total[2];  // by traversal index and step parity: particles binned into the block (one array in large domains)
+  unsigned long long* tile_sums;  // per compaction tile: active blocks << 32 | particles (large domains)
   uint32_t* ticket;       // work counter of the fused kernel
   float* vel_in;          // setup: sorted initial velocities
   uint32_t cap_slots;
@@ -164,6 +169,7 @@ struct GridDev {
 inline void init_colour_classes(SceneDev& sc, uint32_t nstack) {
   sc.nstack = nstack;
   sc.nblocks_domain = nstack * static_cast<uint32_t>(sc.dims[0]) * sc.dims[1] * sc.dims[2];
+  sc.tile_shift = tile_shift_of(sc.nblocks_domain);
   uint32_t base = 0;
   for (int c = 0; c < 8; ++c) {
     const int par[3] = {(c >> 2) & 1, (c >> 1) & 1, c & 1};
@@ -198,6 +204,30 @@ __device__ __forceinline__ int scene_of(const uint32_t* sstart, uint32_t nstack,
 }
 
 __device__ __forceinline__ int colour_of(int x, int y, int z) { return ((x & 1) << 2) | ((y & 1) << 1) | (z & 1); }
+
+// First traversal index and blocks of each colour class, for lanes of different
+// classes to look up in shared memory (divergent constant loads serialise).
+struct ColourClasses {
+  uint32_t base[8], count[8];
+};
+
+__device__ __forceinline__ void load_classes(const SceneDev& sc, ColourClasses& c) {
+  if (threadIdx.x < 8) {
+    c.base[threadIdx.x] = sc.cbase[threadIdx.x];
+    c.count[threadIdx.x] = sc.ccount[threadIdx.x];
+  }
+}
+
+// Place of a block in the colour-major traversal (colour class, stacked domain,
+// lexicographic within the class).  The block table and the binning totals are
+// stored in this order, so the compaction reads and writes them coalesced.
+__device__ __forceinline__ uint32_t traversal_index(const SceneDev& sc, const ColourClasses& cc, int w, int x, int y,
+                                                    int z) {
+  const int c = colour_of(x, y, z);
+  const int ny = (sc.dims[1] + 1 - (y & 1)) >> 1, nz = (sc.dims[2] + 1 - (z & 1)) >> 1;
+  return cc.base[c] + static_cast<uint32_t>(w) * cc.count[c] +
+         static_cast<uint32_t>(((x >> 1) * ny + (y >> 1)) * nz + (z >> 1));
+}
 
 __device__ __forceinline__ int trunc_div4(int a) { return a / 4; }  // truncation toward zero, as the reference
 
@@ -557,29 +587,60 @@ __device__ __forceinline__ void flush_tile(const SceneDev& sc, int4 key, unsigne
   }
 }
 
+// The end of a substep (one thread): advance the substep counter and roll the dt
+// pair: currentDt = nextDt, then the clock advances by it (include/mpm_engine.cuh:869-871).
+__device__ __forceinline__ void end_substep(Scalars* scal) {
+  scal->step += 1;
+  scal->cur_dt = scal->next_dt;
+  scal->cur_dt_d = scal->next_dt_d;
+  scal->time += scal->cur_dt_d;
+}
+
+// Flat index of the grid block at corner e of a particle block's 2x2x2 window if the
+// caller is the first to stamp it with `epoch`, else -1.
+__device__ __forceinline__ int64_t claim_window(const SceneDev& sc, int4 key, int e, int32_t* stamp, int32_t epoch) {
+  const int x = key.x + (e >> 2), y = key.y + ((e >> 1) & 1), z = key.z + (e & 1);
+  if (!in_domain(sc, x, y, z)) return -1;
+  const int64_t f = flat_block(sc, key.w, x, y, z);
+  return atomicExch(stamp + f, epoch) == epoch ? -1 : f;
+}
+
+// The warp zeroes the grid blocks its lanes claimed.
+__device__ __forceinline__ void clear_claimed(int64_t f, long long* __restrict__ g) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t won = __ballot_sync(0xffffffffu, f >= 0); won; won &= won - 1u) {
+    const int64_t b = __shfl_sync(0xffffffffu, f, __ffs(won) - 1);
+    longlong2* p = reinterpret_cast<longlong2*>(g + b * 512);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p[i * 32 + lane] = make_longlong2(0, 0);
+  }
+}
+
+// The last CTA to get here ends the substep (by then every CTA has read the step); the
+// count is left at zero.
+__device__ __forceinline__ void end_substep_by_last_cta(Scalars* scal) {
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&scal->ctas_done, 1u) == gridDim.x - 1) {
+    scal->ctas_done = 0u;
+    end_substep(scal);
+  }
+}
+
 // Zero the grid blocks that the next substep deposits into -- the 2x2x2
 // window of every block of `list` -- and stamp them with `epoch`, each block
-// once (the first warp to swap its stamp zeroes it).  One warp per (block,
-// window corner).  Runs after every kernel that reads the buffer.
+// once (the first lane to swap its stamp claims it).  One warp per block of the
+// list: its first 8 lanes claim the window's blocks at once, then the warp clears
+// the claimed ones, so a block waits for one atomic's latency instead of a chain.
+// Runs after every kernel that reads the buffer.  With `end` it also ends the substep.
 __global__ void zero_windows_kernel(SceneDev sc, BlockListDev list, long long* __restrict__ g, int32_t* stamp,
-                                    const Scalars* __restrict__ scal, int32_t epoch_offset) {
+                                    Scalars* __restrict__ scal, int32_t epoch_offset, int end) {
   const uint32_t nb = *list.nblocks;
   const int32_t epoch = scal->step + epoch_offset;
   const int lane = threadIdx.x & 31;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nb * 8u; t += nwarps) {
-    const int4 key = list.keys[t >> 3];
-    const int e = static_cast<int>(t & 7u);
-    const int x = key.x + (e >> 2), y = key.y + ((e >> 1) & 1), z = key.z + (e & 1);
-    if (!in_domain(sc, x, y, z)) continue;
-    const int64_t f = flat_block(sc, key.w, x, y, z);
-    int won = 0;
-    if (lane == 0) won = atomicExch(stamp + f, epoch) != epoch ? 1 : 0;
-    won = __shfl_sync(0xffffffffu, won, 0);
-    if (!won) continue;
-    longlong2* p = reinterpret_cast<longlong2*>(g + f * 512);
-    for (int i = lane; i < 256; i += 32) p[i] = make_longlong2(0, 0);
-  }
+  for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nb; t += nwarps)
+    clear_claimed(lane < 8 ? claim_window(sc, list.keys[t], lane, stamp, epoch) : -1, g);
+  if (end) end_substep_by_last_cta(scal);
 }
 
 // Incoming particle groups of block `key` (run by warp 0): for each of the
@@ -587,14 +648,15 @@ __global__ void zero_windows_kernel(SceneDev sc, BlockListDev list, long long* _
 // particles that moved here.  s_off: exclusive prefix over directions (28),
 // s_idx: where the group's in-block indices start in prev.idx, s_src: the
 // source block's first particle in the state arrays.
-__device__ __forceinline__ void incoming_groups(const SceneDev& sc, const BlockListDev& prev, int4 key, uint32_t* s_off,
+__device__ __forceinline__ void incoming_groups(const SceneDev& sc, const ColourClasses& classes,
+                                                const BlockListDev& prev, int4 key, uint32_t* s_off,
                                                 uint32_t* s_idx, uint32_t* s_src) {
   const int lane = threadIdx.x & 31;
   uint32_t c = 0, ib = 0, ss = 0;
   if (lane < 27) {
     const int x = key.x + lane / 9 - 1, y = key.y + (lane / 3) % 3 - 1, z = key.z + lane % 3 - 1;
     if (in_domain(sc, x, y, z)) {
-      const int32_t s = prev.table[flat_block(sc, key.w, x, y, z)];
+      const int32_t s = prev.table[traversal_index(sc, classes, key.w, x, y, z)];
       if (s >= 0) {
         const uint32_t a = prev.prefix28[s * 28 + lane], b = prev.prefix28[s * 28 + lane + 1];
         c = b - a;
@@ -637,6 +699,7 @@ __device__ __forceinline__ int find_group(const uint32_t* s_off, uint32_t q) {
 __device__ __forceinline__ uint32_t o_slot(uint32_t start, uint32_t q) { return start + q; }
 
 struct SharedSmall {
+  ColourClasses classes;
   int64_t blk[8];
   uint32_t item;
   uint32_t off[28];
@@ -661,8 +724,8 @@ constexpr size_t kSmemFused = kSmemVTile + kSmemPTile + kSmemCodes;
 // compiles the rigid-particle test in (scenes with rigid particles on; the
 // test alone cost 1.7 % on the sand column).  Register
 // budget: 64 per thread at 256 threads (4 CTAs per SM); at 128 threads the
-// shared-memory footprint allows 5 CTAs per SM, so up to 102 registers; at
-// 1024 threads one CTA fills the SM (for small scenes, where a few hundred
+// shared-memory footprint allows 5 CTAs per SM, so up to 102 registers.
+// At 1024 threads one CTA fills the SM (for small scenes, where a few hundred
 // blocks cannot fill 148 SMs and the fullest block sets the launch's length).
 template <int NT>
 constexpr int fused_min_ctas() { return NT == 128 ? 5 : 1024 / NT; }
@@ -676,7 +739,7 @@ struct RankCounts {
 template <int KIND, int NT, bool RIGID = false>
 __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     g2p2g_kernel(SceneDev sc, ModelDev md, GridDev gd, Scalars* __restrict__ scal) {
-  static_assert(NT % 32 == 0 && NT / 32 <= 32 && NT >= 64, "block size");
+  static_assert(NT % 32 == 0 && NT / 32 <= 32 && NT >= 96, "block size");
   extern __shared__ __align__(16) unsigned char smem[];
   float4* vtile = reinterpret_cast<float4*>(smem);
   unsigned* ptile = reinterpret_cast<unsigned*>(smem + kSmemVTile);
@@ -700,6 +763,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
   const float dtdx = dt * inv_dx;
   const uint32_t maxp = min(md.max_per_block, static_cast<uint32_t>(kMaxParticlesPerBlock));
 
+  load_classes(sc, sh.classes);
   for (int i = threadIdx.x; i < 2 * kTilePlane / 4; i += NT)
     reinterpret_cast<uint4*>(ptile)[i] = make_uint4(0u, 0u, 0u, 0u);
   for (;;) {
@@ -729,12 +793,12 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     }
 
     if (threadIdx.x < 32)
-      incoming_groups(sc, prev, key, sh.off, sh.idx, sh.src);
+      incoming_groups(sc, sh.classes, prev, key, sh.off, sh.idx, sh.src);
     else if (threadIdx.x < 40)
       window_blocks(sc, stin, read_epoch, key, sh.blk, threadIdx.x - 32);
+    __syncthreads();
     for (int i = threadIdx.x; i < static_cast<int>(sizeof(rk.wcnt) / sizeof(uint32_t)); i += NT)
       (&rk.wcnt[0][0])[i] = 0u;
-    __syncthreads();
     load_velocity_tile<NT>(sc, gin, sh.blk, key, unit, dt, vtile);
     __syncthreads();
     // The block's output slots [start, start + n) must lie in the state arrays;
@@ -868,13 +932,12 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       sym_to_full(Di6, Di);
       matmul3(Di, tau, DT);
       float Ah[9];
-      bool finite = true;
       const float sA = ndt * vol_over_mass * inv_dx;
 #pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        Ah[k] = fmaf(-sA, DT[k], Cdx[k]);
-        finite &= fabsf(Ah[k]) < kFixMaxValue;
-      }
+      for (int k = 0; k < 9; ++k) Ah[k] = fmaf(-sA, DT[k], Cdx[k]);
+      bool finite = true;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) finite &= fabsf(Ah[k]) < kFixMaxValue;
 #pragma unroll
       for (int r = 0; r < 3; ++r) finite &= fabsf(v[r]) < kFixMaxValue;
       if (!finite) {
@@ -890,63 +953,64 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     // group counts, then prefix over warps and directions, then ranks), the
     // index list, this block's 28 group prefixes and the next step's per-block
     // totals.
-    {
-      constexpr int kWarps = NT / 32;
-      const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-      const uint32_t span = ((n + kWarps * 32 - 1) / (kWarps * 32)) * 32;
-      const uint32_t q0 = wid * span, q1 = min(q0 + span, n);
-      const uint32_t lt = (1u << lane) - 1u;
-      for (uint32_t b = q0; b < q1; b += 32) {
-        const uint32_t q = b + lane;
-        const int code = q < q1 ? dcode[q] : 255;
-        const uint32_t mask = __match_any_sync(0xffffffffu, code);
-        if (code < 28 && lane == 31 - __clz(mask)) rk.wcnt[wid][code] += __popc(mask);
-        __syncwarp();
-      }
-      __syncthreads();
-      if (threadIdx.x < 32) {
-        uint32_t c = 0;
-        if (lane < 28) {
+    constexpr int kWarps = NT / 32;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t span = ((n + kWarps * 32 - 1) / (kWarps * 32)) * 32;
+    const uint32_t p0 = min(wid * span, n), p1 = min(p0 + span, n);
+    for (uint32_t b = p0; b < p1; b += 32) {
+      const uint32_t p = b + lane;
+      const int code = p < p1 ? dcode[p] : 255;
+      const uint32_t mask = __match_any_sync(0xffffffffu, code);
+      if (code < 28 && lane == 31 - __clz(mask)) rk.wcnt[wid][code] += __popc(mask);
+      __syncwarp();
+    }
+    __syncthreads();
+    uint32_t total = 0;  // in direction `lane`
+    if (threadIdx.x < 28) {
 #pragma unroll
-          for (int w = 0; w < kWarps; ++w) {
-            const uint32_t t = rk.wcnt[w][lane];
-            rk.wcnt[w][lane] = c;
-            c += t;
-          }
-        }
-        const uint32_t cv = lane < 27 ? c : 0u;
-        uint32_t incl = cv;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += t;
-        }
-        if (lane < 27) {
-          const uint32_t pre = incl - cv;
-#pragma unroll
-          for (int w = 0; w < kWarps; ++w) rk.wcnt[w][lane] += pre;
-          cur.prefix28[item * 28 + lane] = pre;
-          if (c > 0) {
-            const int x = key.x - (lane / 9 - 1), y = key.y - ((lane / 3) % 3 - 1), z = key.z - (lane % 3 - 1);
-            atomicAdd(md.dense_total + flat_block(sc, key.w, x, y, z), c);
-          }
-        }
-        if (lane == 26) cur.prefix28[item * 28 + 27] = incl;
-        if (lane == 27 && c > 0) atomicAdd(&scal->lost, c);
+      for (int w = 0; w < kWarps; ++w) {
+        const uint32_t t = rk.wcnt[w][lane];
+        rk.wcnt[w][lane] = total;
+        total += t;
       }
-      __syncthreads();
-      for (uint32_t b = q0; b < q1; b += 32) {
-        const uint32_t q = b + lane;
-        const int code = q < q1 ? dcode[q] : 255;
-        const uint32_t mask = __match_any_sync(0xffffffffu, code);
-        if (code < 27) {
-          const uint32_t r = rk.wcnt[wid][code] + __popc(mask & lt);
-          if (start + r < md.cap_particles) cur.idx[start + r] = static_cast<uint16_t>(q);
-        }
-        __syncwarp();
-        if (code < 27 && lane == 31 - __clz(mask)) rk.wcnt[wid][code] += __popc(mask);
-        __syncwarp();
+    }
+    if (threadIdx.x < 32) {
+      const uint32_t cv = lane < 27 ? total : 0u;
+      uint32_t incl = cv;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
       }
+      if (lane < 27) {
+        const uint32_t pre = incl - cv;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) rk.wcnt[w][lane] += pre;
+        cur.prefix28[item * 28 + lane] = pre;
+      }
+      if (lane == 26) cur.prefix28[item * 28 + 27] = incl;
+    }
+    __syncthreads();
+    // The next list's totals.
+    if (threadIdx.x < 28 && total > 0) {
+      if (lane == 27) {
+        atomicAdd(&scal->lost, total);
+      } else {
+        const int x = key.x - (lane / 9 - 1), y = key.y - ((lane / 3) % 3 - 1), z = key.z - (lane % 3 - 1);
+        atomicAdd(md.dense_total[parity] + traversal_index(sc, sh.classes, key.w, x, y, z), total);
+      }
+    }
+    for (uint32_t b = p0; b < p1; b += 32) {
+      const uint32_t p = b + lane;
+      const int code = p < p1 ? dcode[p] : 255;
+      const uint32_t mask = __match_any_sync(0xffffffffu, code);
+      if (code < 27) {
+        const uint32_t r = rk.wcnt[wid][code] + __popc(mask & ((1u << lane) - 1u));
+        if (start + r < md.cap_particles) cur.idx[start + r] = static_cast<uint16_t>(p);
+      }
+      __syncwarp();
+      if (code < 27 && lane == 31 - __clz(mask)) rk.wcnt[wid][code] += __popc(mask);
+      __syncwarp();
     }
     flush_tile<NT>(sc, key, ptile, ratio, gout);
   }
@@ -1082,88 +1146,153 @@ __device__ __forceinline__ void block_scan2(uint32_t a, uint32_t b, uint32_t& ea
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kCompactThreads) compact_reduce_kernel(SceneDev sc, const uint32_t* __restrict__ total,
-                                                                          uint32_t* __restrict__ tile_sums) {
-  __shared__ uint32_t scratch[128];
-  const uint32_t t0 = blockIdx.x * kCompactTile + threadIdx.x * kCompactPerThread;
-  uint32_t nblk = 0, npart = 0;
-  for (int k = 0; k < kCompactPerThread; ++k) {
-    const uint32_t t = t0 + k;
-    if (t >= sc.nblocks_domain) break;
-    const int4 key = traversal_key(sc, t);
-    const uint32_t c = total[flat_block(sc, key.w, key.x, key.y, key.z)];
-    nblk += c > 0 ? 1u : 0u;
-    npart += c;
+// Block-wide inclusive work of the compaction with one barrier: the sum of `pre`
+// over the CTA, and the exclusive scan of `v` over its threads (both pairs of 32-bit
+// counts packed as active blocks << 32 | particles; neither half can carry, the
+// particle total stays below 2^32).
+__device__ __forceinline__ void block_sum_scan(unsigned long long pre, unsigned long long v, unsigned long long& sum,
+                                               unsigned long long& excl, unsigned long long* scratch) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    pre += __shfl_xor_sync(0xffffffffu, pre, o);
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
   }
-  nblk = block_reduce_sum(nblk, scratch);
-  npart = block_reduce_sum(npart, scratch);
-  if (threadIdx.x == 0) {
-    tile_sums[2 * blockIdx.x] = nblk;
-    tile_sums[2 * blockIdx.x + 1] = npart;
+  if (lane == 31) {
+    scratch[w] = pre;
+    scratch[kCompactThreads / 32 + w] = incl;
+  }
+  __syncthreads();
+  sum = 0;
+  excl = incl - v;
+#pragma unroll
+  for (int k = 0; k < kCompactThreads / 32; ++k) {
+    sum += scratch[k];
+    if (k < w) excl += scratch[kCompactThreads / 32 + k];
   }
 }
 
+// The caller's PER entries of an array in traversal order (zero past the end).
+template <int PER>
+__device__ __forceinline__ void load_totals(const uint32_t* total, uint32_t t0, uint32_t n, uint32_t* c) {
+  if (PER == 4 && t0 + 4 <= n) {
+    const uint4 v = *reinterpret_cast<const uint4*>(total + t0);
+    c[0] = v.x;
+    c[PER > 1 ? 1 : 0] = PER > 1 ? v.y : v.x;
+    c[PER > 2 ? 2 : 0] = PER > 2 ? v.z : v.x;
+    c[PER > 3 ? 3 : 0] = PER > 3 ? v.w : v.x;
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < PER; ++k) c[k] = t0 + k < n ? total[t0 + k] : 0u;
+}
+
+// The tile sums of a large domain.
+template <int PER>
+__global__ void __launch_bounds__(kCompactThreads) compact_reduce_kernel(SceneDev sc, const uint32_t* __restrict__ total,
+                                                                          unsigned long long* __restrict__ tile_sums) {
+  __shared__ unsigned long long scratch[2 * kCompactThreads / 32];
+  uint32_t c[PER];
+  load_totals<PER>(total, (blockIdx.x * kCompactThreads + threadIdx.x) * PER, sc.nblocks_domain, c);
+  unsigned long long v = 0, sum, unused;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) v += (c[k] ? 1ull << 32 : 0ull) + c[k];
+  block_sum_scan(v, 0ull, sum, unused, scratch);
+  if (threadIdx.x == 0) tile_sums[blockIdx.x] = sum;
+}
+
+// One CTA per tile of kCompactThreads x PER traversal entries.  A tile takes its first
+// slot and particle from the tiles before it: in a large domain (PER 4) from their sums,
+// and an empty tile (most of a sparse domain) only marks its table entries; in a small one
+// (PER 1), without a reduce launch, from the totals themselves, at most 16 loads a thread.
+// The totals are left at zero: a large domain's in place, a small one's by the next
+// compaction (`clear`, the other parity's), since other tiles still read them here.
+// ZERO also does zero_windows_kernel's work for the tile's blocks and, with `end`, ends
+// the substep: one launch less, for scenes whose few blocks a tile's CTA clears in no
+// time (a 16^3-block domain has 16 tiles).
+// Bound: latency; one 16-byte load and store per 4 entries.
+template <int PER, bool ZERO>
 __global__ void __launch_bounds__(kCompactThreads)
-    compact_scatter_kernel(SceneDev sc, uint32_t* __restrict__ total, const uint32_t* __restrict__ tile_sums,
-                           BlockListDev out, uint32_t cap_slots, uint32_t* ticket, Scalars* scal) {
-  __shared__ uint32_t scratch[128];
-  uint32_t pb = 0, pp = 0;
-  for (uint32_t t = threadIdx.x; t < blockIdx.x; t += blockDim.x) {
-    pb += tile_sums[2 * t];
-    pp += tile_sums[2 * t + 1];
-  }
-  pb = block_reduce_sum(pb, scratch);
-  pp = block_reduce_sum(pp, scratch);
-  const uint32_t t0 = blockIdx.x * kCompactTile + threadIdx.x * kCompactPerThread;
-  uint32_t c[kCompactPerThread];
-  int64_t fb[kCompactPerThread];
-  int4 keys[kCompactPerThread];
-  uint32_t nblk = 0, npart = 0;
+    compact_scatter_kernel(SceneDev sc, uint32_t* __restrict__ total, uint32_t* __restrict__ clear,
+                           const unsigned long long* __restrict__ tile_sums, BlockListDev out, uint32_t cap_slots,
+                           uint32_t* ticket, Scalars* scal, long long* __restrict__ g, int32_t* stamp,
+                           int32_t epoch_offset, int end) {
+  __shared__ unsigned long long scratch[2 * kCompactThreads / 32];
+  __shared__ int4 active[ZERO ? kCompactThreads * PER : 1];
+  __shared__ uint32_t n_active;
+  const uint32_t n = sc.nblocks_domain;
+  const uint32_t t0 = (blockIdx.x * kCompactThreads + threadIdx.x) * PER;
+  const bool last = blockIdx.x == gridDim.x - 1;
+  const int32_t epoch = ZERO ? scal->step + epoch_offset : 0;
+  if (threadIdx.x == 0) n_active = 0u;
+  int slots[PER];
 #pragma unroll
-  for (int k = 0; k < kCompactPerThread; ++k) {
-    const uint32_t t = t0 + k;
-    c[k] = 0;
-    fb[k] = -1;
-    if (t < sc.nblocks_domain) {
-      keys[k] = traversal_key(sc, t);
-      fb[k] = flat_block(sc, keys[k].w, keys[k].x, keys[k].y, keys[k].z);
-      c[k] = total[fb[k]];
-      nblk += c[k] > 0 ? 1u : 0u;
-      npart += c[k];
+  for (int k = 0; k < PER; ++k) slots[k] = -1;
+  if (PER == 1 || last || tile_sums[blockIdx.x]) {
+    unsigned long long pre = 0;
+    if (PER == 1) {
+      for (uint32_t t = 4 * threadIdx.x; t < blockIdx.x * kCompactThreads; t += 4 * kCompactThreads) {
+        const uint4 q = *reinterpret_cast<const uint4*>(total + t);
+        pre += (static_cast<unsigned long long>((q.x > 0u) + (q.y > 0u) + (q.z > 0u) + (q.w > 0u)) << 32) +
+               (q.x + q.y + q.z + q.w);
+      }
+    } else {
+      for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kCompactThreads) pre += tile_sums[t];
     }
-  }
-  uint32_t eb, ep;
-  block_scan2(nblk, npart, eb, ep, scratch);
-  uint32_t slot = pb + eb, part = pp + ep;
-  bool overflow = false;
+    uint32_t c[PER];
+    load_totals<PER>(total, t0, n, c);
+    unsigned long long v = 0;
 #pragma unroll
-  for (int k = 0; k < kCompactPerThread; ++k) {
-    if (fb[k] < 0) continue;
-    if (c[k] > 0) {
+    for (int k = 0; k < PER; ++k) v += (c[k] ? 1ull << 32 : 0ull) + c[k];
+    unsigned long long before, excl;
+    block_sum_scan(pre, v, before, excl, scratch);
+    uint32_t slot = static_cast<uint32_t>((before + excl) >> 32), part = static_cast<uint32_t>(before + excl);
+    bool overflow = false;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      if (!c[k]) continue;
       if (slot < cap_slots) {
-        out.keys[slot] = keys[k];
+        const int4 key = traversal_key(sc, t0 + k);
+        out.keys[slot] = key;
         out.start[slot] = part;
         out.count[slot] = c[k];
-        out.table[fb[k]] = static_cast<int32_t>(slot);
+        slots[k] = static_cast<int>(slot);
+        if (ZERO) active[atomicAdd(&n_active, 1u)] = key;
       } else {
-        out.table[fb[k]] = -1;
         overflow = true;
       }
       ++slot;
       part += c[k];
-      total[fb[k]] = 0;
-    } else {
-      out.table[fb[k]] = -1;
+      if (PER == 4) total[t0 + k] = 0u;
     }
-  }
-  if (overflow) set_status(scal, kStatusCapacity);
-  if (blockIdx.x == gridDim.x - 1) {
-    const uint32_t tb = block_reduce_sum(nblk, scratch), tp = block_reduce_sum(npart, scratch);
-    if (threadIdx.x == 0) {
-      *out.nblocks = min(pb + tb, cap_slots);
-      *out.nparticles = pp + tp;
+    if (overflow) set_status(scal, kStatusCapacity);
+    if (last && threadIdx.x == kCompactThreads - 1) {
+      *out.nblocks = min(slot, cap_slots);
+      *out.nparticles = part;
       *ticket = 0;
     }
+  }
+  if (PER == 1 && t0 < n) clear[t0] = 0u;
+  if (PER == 4 && t0 + 4 <= n) {
+    *reinterpret_cast<int4*>(out.table + t0) =
+        make_int4(slots[0], slots[PER > 1 ? 1 : 0], slots[PER > 2 ? 2 : 0], slots[PER > 3 ? 3 : 0]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+      if (t0 + k < n) out.table[t0 + k] = slots[k];
+  }
+  if constexpr (ZERO) {
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (uint32_t base = threadIdx.x & ~31u; base < n_active * 8u; base += kCompactThreads) {
+      const uint32_t t = base + lane;
+      int64_t f = -1;
+      if (t < n_active * 8u) f = claim_window(sc, active[t >> 3], static_cast<int>(t & 7u), stamp, epoch);
+      clear_claimed(f, g);
+    }
+    if (end) end_substep_by_last_cta(scal);
   }
 }
 
@@ -1223,8 +1352,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
   }
 }
 
-// Advance the substep counter and roll the dt pair: currentDt = nextDt, then
-// the clock advances by it (include/mpm_engine.cuh:869-871).
 // End of setup: the particles dropped while binning and the rigid velocity.
 // The other fields keep what setup's kernels left (zero, and any status bits
 // they raised: a non-finite initial velocity, a full block).
@@ -1234,15 +1361,6 @@ __global__ void finish_setup_kernel(Scalars* scal, uint32_t lost, float rx, floa
     scal->rigid_v[0] = rx;
     scal->rigid_v[1] = ry;
     scal->rigid_v[2] = rz;
-  }
-}
-
-__global__ void end_substep_kernel(Scalars* scal) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    scal->step += 1;
-    scal->cur_dt = scal->next_dt;
-    scal->cur_dt_d = scal->next_dt_d;
-    scal->time += scal->cur_dt_d;
   }
 }
 
@@ -1304,13 +1422,15 @@ __global__ void adaptive_dt_kernel(Scalars* scal, float dx, float cfl, float dt_
 }
 
 // ------------------------------------------------------------------ setup
-// Initial binning of every particle: its block's flat index in the dense
-// table (0xFFFFFFFF outside the domain or not finite), and the per-block
+// Initial binning of every particle: its block's traversal index (0xFFFFFFFF outside the domain or not finite), and the per-block
 // count.  With the compaction, setup_place_kernel and setup_order_kernel it
 // replaces ActivateBlocksWithParticles + BuildParticleCellBucket
 // (include/mpm_algorithm.cuh:586-626,713-736).
 __global__ void setup_bin_kernel(SceneDev sc, uint32_t n, const float* __restrict__ x, const uint32_t* __restrict__ sstart,
                                  uint32_t* __restrict__ flat, uint32_t* __restrict__ total) {
+  __shared__ ColourClasses classes;
+  load_classes(sc, classes);
+  __syncthreads();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float px = x[3 * i], py = x[3 * i + 1], pz = x[3 * i + 2];
@@ -1320,7 +1440,7 @@ __global__ void setup_bin_kernel(SceneDev sc, uint32_t n, const float* __restric
   const bool finite = isfinite(px) && isfinite(py) && isfinite(pz) && px >= 0.f && py >= 0.f && pz >= 0.f;
   if (finite && in_domain(sc, bx, by, bz)) {
     const int w = sstart ? scene_of(sstart, sc.nstack, i) : 0;
-    f = static_cast<uint32_t>(flat_block(sc, w, bx, by, bz));
+    f = traversal_index(sc, classes, w, bx, by, bz);
     atomicAdd(total + f, 1u);
   }
   flat[i] = f;
@@ -1487,10 +1607,12 @@ __global__ void __launch_bounds__(NT, 4) reorder_gather_kernel(SceneDev sc, Mode
   const StateDev sin = md.st[parity];
   const StateDev sdst = md.st[parity ^ 1];
   const uint32_t nb = *cur.nblocks;
+  load_classes(sc, sh.classes);
+  __syncthreads();
   for (uint32_t slot = blockIdx.x; slot < nb; slot += gridDim.x) {
     const int4 k4 = cur.keys[slot];
     const uint32_t start = cur.start[slot];
-    if (threadIdx.x < 32) incoming_groups(sc, prev, k4, sh.off, sh.idx, sh.src);
+    if (threadIdx.x < 32) incoming_groups(sc, sh.classes, prev, k4, sh.off, sh.idx, sh.src);
     __syncthreads();
     const uint32_t room = start < md.cap_particles ? md.cap_particles - start : 0u;
     const uint32_t n = min(min(cur.count[slot], sh.off[27]), room);
@@ -1651,13 +1773,15 @@ __global__ void __launch_bounds__(NT) probe_kernel(SceneDev sc, ModelDev md, Gri
   const StateDev sin = md.st[parity];
   const uint32_t nb = *cur.nblocks;
   const float dt = scal->cur_dt;
+  load_classes(sc, sh.classes);
+  __syncthreads();
   for (uint32_t item = blockIdx.x; item < nb; item += gridDim.x) {
     const int4 key = cur.keys[item];
     const uint32_t start = cur.start[item];
     const uint32_t n = cur.count[item];
     const int kind = md.smat ? md.smat[key.w].kind : md.mat.kind;
     if (threadIdx.x < 32)
-      incoming_groups(sc, prev, key, sh.off, sh.idx, sh.src);
+      incoming_groups(sc, sh.classes, prev, key, sh.off, sh.idx, sh.src);
     else if (threadIdx.x < 40)
       window_blocks(sc, gd.stamp[parity], step, key, sh.blk, threadIdx.x - 32);
     __syncthreads();

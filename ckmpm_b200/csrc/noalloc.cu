@@ -41,6 +41,7 @@ constexpr size_t kNaGrid = na_align(sizeof(long long) * 512 * kNoAllocMaxDomainB
 constexpr size_t kNaDomainU32 = na_align(sizeof(uint32_t) * kNoAllocMaxDomainBlocks);
 constexpr size_t kNaParticleU32 = na_align(sizeof(uint32_t) * kNoAllocMaxParticles);
 constexpr size_t kNaParticleU16 = na_align(sizeof(uint16_t) * kNoAllocMaxParticles);
+static_assert(tile_shift_of(kNoAllocMaxDomainBlocks) == 8, "the compaction's small tiles");
 constexpr size_t kNaSlots = kNoAllocMaxDomainBlocks;  // slots <= min(domain blocks, particles)
 constexpr size_t kNaBlockList = na_align(sizeof(int4) * kNaSlots) + 2 * na_align(sizeof(uint32_t) * kNaSlots) +
                                 kNaDomainU32 + na_align(sizeof(uint32_t) * 28 * kNaSlots) + kNaParticleU16 +
@@ -48,7 +49,7 @@ constexpr size_t kNaBlockList = na_align(sizeof(int4) * kNaSlots) + 2 * na_align
 constexpr size_t kNaState = 14 * kNaParticleU32;  // x[3], F[9], aux, id
 constexpr size_t kNoAllocScratchBytes =
     2 * kNaGrid + 2 * kNaDomainU32 + na_align(sizeof(Scalars)) + 2 * kNaState + 2 * kNaBlockList +
-    kNaDomainU32 /*dense totals*/ + na_align(sizeof(uint32_t) * 2 * 64) /*tile sums*/ + na_align(4) /*ticket*/ +
+    2 * kNaDomainU32 /*dense totals*/ + na_align(4) /*ticket*/ +
     3 * kNaParticleU32 /*initial velocities*/ +
     3 * kNaParticleU32 /*setup: flat block indices, placement cursors, particle order*/ +
     18 * kNaParticleU32 /*export*/;
@@ -239,8 +240,7 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
     bl.nblocks = cv.take<uint32_t>(1);
     bl.nparticles = cv.take<uint32_t>(1);
   }
-  d.dense_total = cv.take<uint32_t>(kNoAllocMaxDomainBlocks);
-  d.tile_sums = cv.take<uint32_t>(2 * 64);
+  for (int b = 0; b < 2; ++b) d.dense_total[b] = cv.take<uint32_t>(kNoAllocMaxDomainBlocks);
   d.ticket = cv.take<uint32_t>(1);
   d.vel_in = cv.take<float>(3 * size_t(kNoAllocMaxParticles));
   uint32_t* flat = cv.take<uint32_t>(kNoAllocMaxParticles);
@@ -263,7 +263,7 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
   d.mass = mass;
   d.vol = volume;
   d.flush_ratio = 1.0;
-  const uint32_t ntiles = (nbd + kCompactTile - 1) / kCompactTile;
+  const uint32_t ntiles = compact_tiles(sc);
 
 #define NA_CUDA(call)                                                   \
   do {                                                                  \
@@ -277,15 +277,13 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
     NA_CUDA(cudaMemsetAsync(d.bl[b].nblocks, 0, sizeof(uint32_t), st));
     NA_CUDA(cudaMemsetAsync(d.bl[b].nparticles, 0, sizeof(uint32_t), st));
   }
-  NA_CUDA(cudaMemsetAsync(d.dense_total, 0, sizeof(uint32_t) * nbd, st));
+  for (int b = 0; b < 2; ++b) NA_CUDA(cudaMemsetAsync(d.dense_total[b], 0, sizeof(uint32_t) * nbd, st));
   NA_CUDA(cudaMemsetAsync(d.ticket, 0, sizeof(uint32_t), st));
 
   // Setup: bin, compact, place and order each block's particles, gather,
   // identity previous step, initial grid -- the sequence of ckmpm_setup.
-  setup_bin_kernel<<<(n + 255) / 256, 256, 0, st>>>(sc, n, x, nullptr, flat, d.dense_total);
-  compact_reduce_kernel<<<ntiles, kCompactThreads, 0, st>>>(sc, d.dense_total, d.tile_sums);
-  compact_scatter_kernel<<<ntiles, kCompactThreads, 0, st>>>(sc, d.dense_total, d.tile_sums, d.bl[0], d.cap_slots,
-                                                             d.ticket, scal);
+  setup_bin_kernel<<<(n + 255) / 256, 256, 0, st>>>(sc, n, x, nullptr, flat, d.dense_total[1]);
+  NA_CUDA(launch_compact(sc, d, grid, scal, ntiles, st, 0, 1));
   NA_CUDA(cudaMemsetAsync(cursor, 0, sizeof(uint32_t) * d.cap_slots, st));
   setup_place_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, flat, d.bl[0], cursor, perm);
   setup_order_kernel<256><<<ctas, 256, 0, st>>>(sc, d.bl[0], x, perm, scal);
@@ -309,14 +307,15 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
   NA_CUDA(cudaMemsetAsync(d.ticket, 0, sizeof(uint32_t), st));
   int sms = 0;
   NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, desc->device));
-  zero_windows_kernel<<<sms * 4, 256, 0, st>>>(sc, d.bl[0], grid.grid[0], grid.stamp[0], scal, 0);
+  zero_windows_kernel<<<sms * 4, 256, 0, st>>>(sc, d.bl[0], grid.grid[0], grid.stamp[0], scal, 0, 0);
   rasterize_kernel<kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, d, grid, scal);
   NA_CUDA(cudaMemsetAsync(d.ticket, 0, sizeof(uint32_t), st));
-  zero_windows_kernel<<<sms * 4, 256, 0, st>>>(sc, d.bl[0], grid.grid[1], grid.stamp[1], scal, 1);
+  zero_windows_kernel<<<sms * 4, 256, 0, st>>>(sc, d.bl[0], grid.grid[1], grid.stamp[1], scal, 1, 0);
   finish_setup_kernel<<<1, 32, 0, st>>>(scal, n - n_valid, 0.f, 0.f, 0.f);  // keeps setup's status bits
   NA_CUDA(cudaGetLastError());
 
   // Substeps: the launch sequence of ckmpm_step without graphs.
+  const bool fold = folds_zero(sc, counts[0]);
   if (nsteps > 0) set_next_dt_kernel<<<1, 32, 0, st>>>(scal, dt);
   for (uint32_t i = 0; i < nsteps; ++i) {
     const int parity = static_cast<int>(i & 1);
@@ -336,11 +335,10 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
       default:
         g2p2g_kernel<kFluid, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, d, grid, scal);
     }
-    compact_reduce_kernel<<<ntiles, kCompactThreads, 0, st>>>(sc, d.dense_total, d.tile_sums);
-    compact_scatter_kernel<<<ntiles, kCompactThreads, 0, st>>>(sc, d.dense_total, d.tile_sums, d.bl[parity ^ 1],
-                                                               d.cap_slots, d.ticket, scal);
-    zero_windows_kernel<<<sms * 4, 256, 0, st>>>(sc, d.bl[parity ^ 1], grid.grid[parity], grid.stamp[parity], scal, 2);
-    end_substep_kernel<<<1, 32, 0, st>>>(scal);
+    NA_CUDA(launch_compact(sc, d, grid, scal, ntiles, st, parity ^ 1, parity, fold ? parity : -1, true));
+    if (!fold)
+      zero_windows_kernel<<<sms * 4, 256, 0, st>>>(sc, d.bl[parity ^ 1], grid.grid[parity], grid.stamp[parity], scal, 2,
+                                                   1);
   }
   NA_CUDA(cudaGetLastError());
 

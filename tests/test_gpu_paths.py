@@ -1,0 +1,172 @@
+"""Edges of the engine's dispatch: launch shapes by block count, domain sizes of the
+compaction, the stresses' fallback, adaptive graphs, and the differentiable rollout's
+particle order and tiles.  Where two routes compute the same thing, they are
+compared bit for bit; the stresses against the FP64 oracle."""
+import math
+
+import numpy as np
+import pytest
+
+from ckmpm_b200 import Scene, scenes
+from ckmpm_b200 import _capi as capi
+from ckmpm_b200.engine import MPMConfig, MPMMaterial, MPMModel, compute_lame_parameters
+
+pytestmark = pytest.mark.gpu
+
+
+def rotations(rng, n):
+    q, _ = np.linalg.qr(rng.normal(size=(n, 3, 3)))
+    q[np.linalg.det(q) < 0, :, 0] *= -1
+    return q
+
+
+def box_scene(n, blocks, dx=1 / 64, ppc=8, kind="fixed_corotated", seed=0, v0=(0.4, -1.0, 0.3)):
+    """A jittered cube of about n particles in the middle of a domain of `blocks`, at cell size dx."""
+    rng = np.random.default_rng(seed)
+    half = 0.5 * (n / ppc) ** (1 / 3) * dx
+    c = 2.0 * np.asarray(blocks) * dx + 0.1 * dx
+    x = scenes.box_particles(c - half, c + half, dx, ppc, rng)
+    lam, mu = compute_lame_parameters(5e4, 0.3)
+    mat = MPMMaterial.fluid(1e4, 7.15, 0.1) if kind == "fluid" else getattr(MPMMaterial, kind)(lam, mu)
+    vol = dx ** 3 / ppc
+    v = (np.asarray(v0) + 4.0 * (x - c)[:, [1, 2, 0]]).astype(np.float32)
+    return MPMConfig(dx=dx, domain_blocks=tuple(blocks)), [MPMModel(1000 * vol, vol, x, v, mat)]
+
+
+def run(cfg, models, steps, tuning=None, dt=1e-4):
+    s = Scene(cfg)
+    for m in models:
+        s.add_model(m)
+    if tuning:
+        s.set_tuning(*tuning)
+    s.setup()
+    s.step(steps, dt)
+    return s
+
+
+def assert_same(a, b, what):
+    for name in ("x", "v", "F", "aux"):
+        p, q = getattr(a, name), getattr(b, name)
+        assert np.array_equal(p.view(np.uint32), q.view(np.uint32)), (what, name)
+    assert np.array_equal(a.id, b.id), what
+
+
+@pytest.mark.parametrize("kind", ["fixed_corotated", "drucker_prager", "fluid"])
+@pytest.mark.parametrize("n,blocks", [(40, 12), (17000, 12), (45000, 14), (100000, 16)])
+def test_split_blocks_give_the_same_bits(engine_lib, kind, n, blocks):
+    """The default shape (blocks split over clusters of 4 or 2 CTAs, or not, by their number)
+    against one CTA per block, with the particles crossing block faces."""
+    cfg, models = box_scene(n, (blocks,) * 3, kind=kind)
+    a = run(cfg, models, 33)
+    b = run(cfg, models, 33, (256, 4, 8))
+    c = run(cfg, models, 33, (1024, 1, 8))
+    assert_same(a.state(0), b.state(0), "default")
+    assert_same(c.state(0), b.state(0), "clusters")
+    for which in (0, 1, 2):
+        for p, q in zip(a.blocks(0, which), b.blocks(0, which)):
+            assert np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("dims", [(9, 11, 13), (25, 25, 26), (26, 26, 26), (64, 17, 16)])
+def test_domain_size_does_not_matter(engine_lib, dims):
+    """The compaction's small and large tiles, odd extents among them: the same body far from
+    any wall moves alike in every domain (positions are taken relative to its block)."""
+    cfg, models = box_scene(5000, (10, 10, 10))
+    ref = run(cfg, models, 40, (256, 4, 8))
+    big = MPMConfig(dx=cfg.dx, domain_blocks=dims)
+    s = run(big, models, 40)
+    assert_same(s.state(0), ref.state(0), dims)
+    for p, q in zip(s.blocks(0, 0), ref.blocks(0, 0)):
+        assert np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("kind", [capi.FIXED_COROTATED, capi.DRUCKER_PRAGER, capi.VON_MISES])
+def test_stress_of_ill_conditioned_deformation(engine_lib, oracle_mod, kind):
+    """Stretches from well within to far beyond the ratio of 4 at which the return maps go back to
+    the full SVD, and inverted ones for the fixed-corotated model.  The stretches are known to
+    rounding of the largest, so log s to 2^-23 s_max / s_min: the tolerance on tau is
+    8 of those times the stiffness."""
+    rng = np.random.default_rng(11)
+    n = 384
+    ratio = np.exp(rng.uniform(0, math.log(40.0), n))
+    s = np.stack([np.ones(n), ratio ** -rng.uniform(0, 1, n), 1 / ratio], 1) * np.exp(rng.uniform(-0.3, 0.3, (n, 1)))
+    if kind == capi.FIXED_COROTATED:
+        s[::7, 2] *= -1
+    F = (rotations(rng, n) * s[:, None, :]) @ rotations(rng, n).transpose(0, 2, 1)
+    F = F.astype(np.float32)
+    lam, mu = 2.0e4, 3.0e4
+    params = {capi.VON_MISES: [mu, lam, 500.0, 0.0]}.get(kind, [lam, mu, 0.0, 0.0])
+    mat = capi.Material()
+    mat.kind = kind
+    for i, p in enumerate(params):
+        mat.p[i] = p
+    aux = np.full(n, 1.0 if kind == capi.VON_MISES else 0.0, np.float32)
+    Fg, ag, tau = F.copy(), aux.copy(), np.zeros_like(F)
+    C = np.zeros((n, 3, 3), np.float32)
+    capi.check(engine_lib.ckmpm_debug_constitutive(mat, n, capi.fptr(C), 0.0, capi.fptr(Fg), capi.fptr(ag),
+                                                   capi.fptr(tau), None, None, None), "debug")
+    for i in range(n):
+        Fo, ao, to = oracle_mod.constitutive(kind, params, np.zeros((3, 3)), 0.0, F[i].astype(np.float64), float(aux[i]))
+        eps = 2.0 ** -23 * float(ratio[i])
+        assert np.abs(tau[i] - to).max() <= 8 * eps * 5 * max(lam, mu) + 2e-5 * np.abs(to).max(), i
+        assert np.abs(Fg[i] - Fo).max() <= 16 * eps + 2e-6, i
+
+
+@pytest.mark.parametrize("boundary", ["sticky_blocks", "slip_floor"])
+def test_adaptive_frame_equals_its_substeps(engine_lib, boundary):
+    """A frame in one call (substeps replayed from graphs, the dt taken on the device) against the
+    same frame one substep per call, and two frames of different bounds on one scene."""
+    cfg, models = box_scene(6000, (12,) * 3, v0=(3.0, -4.0, 2.0))
+    cfg.boundary = boundary
+    whole, single = Scene(cfg), Scene(cfg)
+    for s in (whole, single):
+        s.add_model(models[0])
+        s.setup()
+    for dt, cfl, frame in ((1e-4, 0.02, 2.3e-3), (7e-5, 0.5, 1.7e-3)):
+        whole.step_adaptive(1 << 20, dt, cfl, frame)
+        left = frame
+        while True:
+            single.step_adaptive(1, dt, cfl, left)
+            left = 0.0
+            t, end = single.time()
+            if not end - t > 0.0:
+                break
+        assert whole.counters()["steps"] == single.counters()["steps"]
+        assert whole.time() == single.time()
+    assert_same(whole.state(0), single.state(0), boundary)
+
+
+@pytest.mark.parametrize("n,spread,every", [(1, 0.0, 1), (129, 0.02, 1), (700, 0.3, 4), (3000, 0.1, 1), (3000, 0.1, 7)])
+def test_rollout_does_not_depend_on_the_particle_order(engine_lib, n, spread, every):
+    """The rollout sorts its particles and deposits through per-CTA tiles, or directly where a CTA's
+    particles lie too far apart (a sparse cloud): permuted inputs give permuted outputs and gradients,
+    bit for bit, for every checkpoint interval."""
+    torch = pytest.importorskip("torch")
+    from ckmpm_b200.diff import DiffRollout
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(n)
+    cfg = MPMConfig(dx=1 / 64, domain_blocks=(16,) * 3)
+    x = (0.5 + spread * (rng.random((n, 3)) * 2 - 1)).astype(np.float32)
+    v = rng.normal(scale=0.5, size=(n, 3)).astype(np.float32)
+    logE = (math.log(5e4) + 0.2 * rng.standard_normal(n)).astype(np.float32)
+    gx, gF = rng.normal(size=(n, 3)).astype(np.float32), rng.normal(size=(n, 3, 3)).astype(np.float32)
+    vol = (1 / 64) ** 3 / 8
+
+    def outputs(order, k):
+        t = [torch.from_numpy(np.ascontiguousarray(a[order])).to(dev) for a in (x, v, logE, gx, gF)]
+        sim = DiffRollout(cfg, n, 1000 * vol, vol, nu=0.3, nsteps=9, dt=1e-4, checkpoint_every=k)
+        res = []
+        for _ in range(2):  # the second pass finds every sum as the first left it
+            out = sim.forward(*t[:3])
+            res.append([a.cpu().numpy() for a in (*out, *sim.backward(t[3], t[4], dev))])
+        for a, b in zip(*res):
+            assert np.array_equal(a, b)
+        sim.close()
+        return res[1]
+
+    ref = outputs(np.arange(n), every)
+    order = rng.permutation(n)
+    for a, b in zip(ref, outputs(order, every)):
+        assert np.array_equal(a[order], b)
+    for a, b in zip(ref, outputs(np.arange(n), 2)):
+        assert np.array_equal(a, b)
