@@ -148,35 +148,36 @@ void free_graphs(ckmpm_scene* s) {
 }
 
 template <int KIND, int NT, bool RIGID>
-cudaError_t launch_fused(ckmpm_scene* s, const ModelHost& m) {
-  g2p2g_kernel<KIND, NT, RIGID><<<s->fused_ctas, NT, kSmemFused, s->stream>>>(s->sc, m.dev, s->grid, s->scal);
+cudaError_t launch_fused(ckmpm_scene* s, const ModelHost& m, int parity) {
+  g2p2g_kernel<KIND, NT, RIGID><<<s->fused_ctas, NT, kSmemFused, s->stream>>>(
+      s->sc, for_substep(m.dev, parity), for_substep(s->grid, parity), s->scal);
   return cudaGetLastError();
 }
 
 template <int NT, bool RIGID>
-cudaError_t launch_fused_kind(ckmpm_scene* s, const ModelHost& m) {
+cudaError_t launch_fused_kind(ckmpm_scene* s, const ModelHost& m, int parity) {
   switch (m.mat.kind) {
-    case CKMPM_FIXED_COROTATED: return launch_fused<kFixedCorotated, NT, RIGID>(s, m);
-    case CKMPM_LINEAR: return launch_fused<kLinear, NT, RIGID>(s, m);
-    case CKMPM_DRUCKER_PRAGER: return launch_fused<kDruckerPrager, NT, RIGID>(s, m);
-    case CKMPM_VON_MISES: return launch_fused<kVonMises, NT, RIGID>(s, m);
-    case CKMPM_NACC: return launch_fused<kNacc, NT, RIGID>(s, m);
-    default: return launch_fused<kFluid, NT, RIGID>(s, m);
+    case CKMPM_FIXED_COROTATED: return launch_fused<kFixedCorotated, NT, RIGID>(s, m, parity);
+    case CKMPM_LINEAR: return launch_fused<kLinear, NT, RIGID>(s, m, parity);
+    case CKMPM_DRUCKER_PRAGER: return launch_fused<kDruckerPrager, NT, RIGID>(s, m, parity);
+    case CKMPM_VON_MISES: return launch_fused<kVonMises, NT, RIGID>(s, m, parity);
+    case CKMPM_NACC: return launch_fused<kNacc, NT, RIGID>(s, m, parity);
+    default: return launch_fused<kFluid, NT, RIGID>(s, m, parity);
   }
 }
 
 template <int NT>
-cudaError_t launch_fused_nt(ckmpm_scene* s, const ModelHost& m) {
-  if (m.mat.kind == kMixedKind) return launch_fused<kMixed, NT, false>(s, m);  // batches have no rigid particles
-  return s->sc.rigid ? launch_fused_kind<NT, true>(s, m) : launch_fused_kind<NT, false>(s, m);
+cudaError_t launch_fused_nt(ckmpm_scene* s, const ModelHost& m, int parity) {
+  if (m.mat.kind == kMixedKind) return launch_fused<kMixed, NT, false>(s, m, parity);  // batches have no rigid particles
+  return s->sc.rigid ? launch_fused_kind<NT, true>(s, m, parity) : launch_fused_kind<NT, false>(s, m, parity);
 }
 
-cudaError_t launch_fused_any(ckmpm_scene* s, const ModelHost& m) {
+cudaError_t launch_fused_any(ckmpm_scene* s, const ModelHost& m, int parity) {
   switch (s->tune.threads) {
-    case 128: return launch_fused_nt<128>(s, m);
-    case 192: return launch_fused_nt<192>(s, m);
-    case 1024: return launch_fused_nt<1024>(s, m);
-    default: return launch_fused_nt<256>(s, m);
+    case 128: return launch_fused_nt<128>(s, m, parity);
+    case 192: return launch_fused_nt<192>(s, m, parity);
+    case 1024: return launch_fused_nt<1024>(s, m, parity);
+    default: return launch_fused_nt<256>(s, m, parity);
   }
 }
 
@@ -306,7 +307,7 @@ cudaError_t enqueue_substep(ckmpm_scene* s, int parity) {
   cudaError_t e = cudaSuccess;
   const bool fold = folds_zero(s->sc, s->nblocks0);
   for (auto& m : s->models) {
-    if (e == cudaSuccess) e = launch_fused_any(s, m);
+    if (e == cudaSuccess) e = launch_fused_any(s, m, parity);
     if (e == cudaSuccess && !fold) e = launch_compact(s, m, parity ^ 1, parity);
   }
   if (!fold) return e == cudaSuccess ? launch_zero(s, parity ^ 1, parity, 2, true) : e;
@@ -1470,7 +1471,7 @@ ckmpm_status ckmpm_step_profiled(ckmpm_scene* s, uint32_t nsteps, float dt, doub
       auto& m = s->models[mi];
       cudaEvent_t* E = &ev[(i * nm + mi) * 3];
       CK_CUDA(s, cudaEventRecord(E[0], s->stream));
-      CK_CUDA(s, launch_fused_any(s, m));
+      CK_CUDA(s, launch_fused_any(s, m, parity));
       CK_CUDA(s, cudaEventRecord(E[1], s->stream));
       CK_CUDA(s, launch_compact(s, m, parity ^ 1, parity));
       if (mi + 1 == nm) CK_CUDA(s, launch_zero(s, parity ^ 1, parity, 2, true));

@@ -29,6 +29,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "mpm_math.cuh"
 
 namespace ckmpm {
@@ -163,6 +165,24 @@ struct GridDev {
   long long* grid[2];
   int32_t* stamp[2];
 };
+
+// The double-buffered arrays as a substep of step parity `p` sees them: [0] read, [1] written.
+inline ModelDev for_substep(ModelDev m, int p) {
+  if (p) {
+    std::swap(m.st[0], m.st[1]);
+    std::swap(m.bl[0], m.bl[1]);
+    std::swap(m.dense_total[0], m.dense_total[1]);
+  }
+  return m;
+}
+
+inline GridDev for_substep(GridDev g, int p) {
+  if (p) {
+    std::swap(g.grid[0], g.grid[1]);
+    std::swap(g.stamp[0], g.stamp[1]);
+  }
+  return g;
+}
 
 // Colour classes of the traversal over `nstack` stacked domains of sc.dims
 // blocks: class c holds the blocks whose coordinate parities are the bits of c.
@@ -747,17 +767,18 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
   __shared__ SharedSmall sh;
   __shared__ RankCounts<NT> rk;
 
-  const int32_t step = scal->step;
-  const int parity = step & 1;
-  const int32_t read_epoch = step;
+  // md and gd are the host's for_substep copies: entry 0 of every pair is the one this
+  // substep reads, so the arrays' addresses are plain kernel parameters (indexed by the
+  // step's parity they cost a constant load each, every time).
+  const int32_t read_epoch = scal->step;
   const float dt = scal->cur_dt, ndt = scal->next_dt;
-  const BlockListDev cur = md.bl[parity];
-  const BlockListDev prev = md.bl[parity ^ 1];
-  const StateDev sin = md.st[parity];
-  const StateDev sout = md.st[parity ^ 1];
-  const long long* __restrict__ gin = gd.grid[parity];
-  long long* __restrict__ gout = gd.grid[parity ^ 1];
-  const int32_t* __restrict__ stin = gd.stamp[parity];
+  const BlockListDev& cur = md.bl[0];
+  const BlockListDev& prev = md.bl[1];
+  const StateDev& sin = md.st[0];
+  const StateDev& sout = md.st[1];
+  const long long* __restrict__ gin = gd.grid[0];
+  long long* __restrict__ gout = gd.grid[1];
+  const int32_t* __restrict__ stin = gd.stamp[0];
   const uint32_t nb = *cur.nblocks;
   const float inv_dx = sc.inv_dx;
   const float dtdx = dt * inv_dx;
@@ -997,7 +1018,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         atomicAdd(&scal->lost, total);
       } else {
         const int x = key.x - (lane / 9 - 1), y = key.y - ((lane / 3) % 3 - 1), z = key.z - (lane % 3 - 1);
-        atomicAdd(md.dense_total[parity] + traversal_index(sc, sh.classes, key.w, x, y, z), total);
+        atomicAdd(md.dense_total[0] + traversal_index(sc, sh.classes, key.w, x, y, z), total);
       }
     }
     for (uint32_t b = p0; b < p1; b += 32) {

@@ -319,21 +319,23 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
   if (nsteps > 0) set_next_dt_kernel<<<1, 32, 0, st>>>(scal, dt);
   for (uint32_t i = 0; i < nsteps; ++i) {
     const int parity = static_cast<int>(i & 1);
+    const ModelDev md = for_substep(d, parity);
+    const GridDev gd = for_substep(grid, parity);
     switch (material->kind) {
       case CKMPM_FIXED_COROTATED:
-        g2p2g_kernel<kFixedCorotated, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, d, grid, scal);
+        g2p2g_kernel<kFixedCorotated, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
         break;
       case CKMPM_DRUCKER_PRAGER:
-        g2p2g_kernel<kDruckerPrager, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, d, grid, scal);
+        g2p2g_kernel<kDruckerPrager, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
         break;
       case CKMPM_VON_MISES:
-        g2p2g_kernel<kVonMises, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, d, grid, scal);
+        g2p2g_kernel<kVonMises, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
         break;
       case CKMPM_NACC:
-        g2p2g_kernel<kNacc, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, d, grid, scal);
+        g2p2g_kernel<kNacc, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
         break;
       default:
-        g2p2g_kernel<kFluid, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, d, grid, scal);
+        g2p2g_kernel<kFluid, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
     }
     NA_CUDA(launch_compact(sc, d, grid, scal, ntiles, st, parity ^ 1, parity, fold ? parity : -1, true));
     if (!fold)
