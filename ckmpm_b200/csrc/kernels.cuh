@@ -26,6 +26,7 @@
 // of the blocks the next substep deposits into.  No host sync.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -745,8 +746,12 @@ constexpr size_t kSmemFused = kSmemVTile + kSmemPTile + kSmemCodes;
 // test alone cost 1.7 % on the sand column).  Register
 // budget: 64 per thread at 256 threads (4 CTAs per SM); at 128 threads the
 // shared-memory footprint allows 5 CTAs per SM, so up to 102 registers.
-// At 1024 threads one CTA fills the SM (for small scenes, where a few hundred
-// blocks cannot fill 148 SMs and the fullest block sets the launch's length).
+// CLUSTER splits every block over the CTAs of a thread-block cluster, for small
+// scenes, whose few hundred blocks cannot fill 148 SMs and whose fullest block sets
+// the launch's length: each CTA takes a contiguous part of the block's particles
+// with tiles of its own, flushed into the grid like any others (the sums are
+// exact), and only the direction counts of the rebin ranking cross CTAs, through
+// distributed shared memory.  The particles' order, and every bit, stays the same.
 template <int NT>
 constexpr int fused_min_ctas() { return NT == 128 ? 5 : 1024 / NT; }
 
@@ -756,7 +761,13 @@ struct RankCounts {
   uint32_t wcnt[NT / 32][28];
 };
 
-template <int KIND, int NT, bool RIGID = false>
+// Clusters: this CTA's particles by direction, read by the cluster's other CTAs.
+template <bool CLUSTER>
+struct PartCounts {
+  uint32_t count[CLUSTER ? 28 : 1];
+};
+
+template <int KIND, int NT, bool RIGID = false, bool CLUSTER = false>
 __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     g2p2g_kernel(SceneDev sc, ModelDev md, GridDev gd, Scalars* __restrict__ scal) {
   static_assert(NT % 32 == 0 && NT / 32 <= 32 && NT >= 96, "block size");
@@ -766,6 +777,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
   uint8_t* dcode = smem + kSmemVTile + kSmemPTile;
   __shared__ SharedSmall sh;
   __shared__ RankCounts<NT> rk;
+  __shared__ PartCounts<CLUSTER> pc;
 
   // md and gd are the host's for_substep copies: entry 0 of every pair is the one this
   // substep reads, so the arrays' addresses are plain kernel parameters (indexed by the
@@ -784,13 +796,24 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
   const float dtdx = dt * inv_dx;
   const uint32_t maxp = min(md.max_per_block, static_cast<uint32_t>(kMaxParticlesPerBlock));
 
+  // Cluster of nparts CTAs per block (1 without CLUSTER), this one taking part `part`.
+  namespace cg = cooperative_groups;
+  const uint32_t nparts = CLUSTER ? cg::this_cluster().num_blocks() : 1u;
+  const uint32_t part = CLUSTER ? cg::this_cluster().block_rank() : 0u;
+  const uint32_t first = blockIdx.x / nparts, nworkers = gridDim.x / nparts;
+  if (first >= nb) return;
   load_classes(sc, sh.classes);
   for (int i = threadIdx.x; i < 2 * kTilePlane / 4; i += NT)
     reinterpret_cast<uint4*>(ptile)[i] = make_uint4(0u, 0u, 0u, 0u);
-  for (;;) {
-    if (threadIdx.x == 0) sh.item = atomicAdd(md.ticket, 1u);
-    __syncthreads();
-    const uint32_t item = sh.item;
+  // Blocks come from the ticket, one at a time when a CTA is free (taking the next one
+  // early lengthens the launch's tail: 6 % on the sand column); clusters, which
+  // seldom have a second block, stride.
+  for (uint32_t item = first;; item += nworkers) {
+    if constexpr (!CLUSTER) {
+      if (threadIdx.x == 0) sh.item = atomicAdd(md.ticket, 1u);
+      __syncthreads();
+      item = sh.item;
+    }
     if (item >= nb) break;
     const int4 key = cur.keys[item];
     const uint32_t start = cur.start[item];
@@ -825,7 +848,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     // The block's output slots [start, start + n) must lie in the state arrays;
     // counts that say otherwise are flagged and clamped, never written past.
     const uint32_t room = start < md.cap_particles ? md.cap_particles - start : 0u;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && part == 0) {
       uint32_t flags = 0;
       if (sh.off[27] != n || n > room) flags |= kStatusConsistency;
       if (n > maxp) flags |= kStatusCapacity;
@@ -833,7 +856,14 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     }
     n = min(min(min(n, sh.off[27]), maxp), room);
 
-    for (uint32_t q = threadIdx.x; q < n; q += NT) {
+    // This CTA's particles [q0, q1) of the block, whole warps of them.
+    uint32_t q0 = 0, q1 = n;
+    if (CLUSTER) {
+      const uint32_t each = (((n + 31) >> 5) + nparts - 1) / nparts * 32;
+      q0 = min(part * each, n);
+      q1 = min(q0 + each, n);
+    }
+    for (uint32_t q = q0 + threadIdx.x; q < q1; q += NT) {
       const int d = find_group(sh.off, q);
       const uint32_t ii = sh.idx[d] + (q - sh.off[d]);
       uint32_t iin = ii < md.cap_particles ? sh.src[d] + prev.idx[ii] : 0xFFFFFFFFu;
@@ -930,7 +960,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       }
       ok &= in_domain(sc, kk[0] - sh3[0], kk[1] - sh3[1], kk[2] - sh3[2]);
       const int code = ok ? (sh3[0] + 1) * 9 + (sh3[1] + 1) * 3 + (sh3[2] + 1) : 27;
-      dcode[q] = static_cast<uint8_t>(code);
+      dcode[q - q0] = static_cast<uint8_t>(code);
       if (!inside) set_status(scal, kStatusOutsideBlock);
       if (!win) {
         atomicAdd(&scal->window_skips, 1u);
@@ -973,11 +1003,12 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     // direction groups, in two passes over warp-contiguous ranges (per-warp
     // group counts, then prefix over warps and directions, then ranks), the
     // index list, this block's 28 group prefixes and the next step's per-block
-    // totals.
+    // totals.  The parts of a cluster read each other's counts from shared memory.
     constexpr int kWarps = NT / 32;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint32_t span = ((n + kWarps * 32 - 1) / (kWarps * 32)) * 32;
-    const uint32_t p0 = min(wid * span, n), p1 = min(p0 + span, n);
+    const uint32_t m = q1 - q0;
+    const uint32_t span = ((m + kWarps * 32 - 1) / (kWarps * 32)) * 32;
+    const uint32_t p0 = min(wid * span, m), p1 = min(p0 + span, m);
     for (uint32_t b = p0; b < p1; b += 32) {
       const uint32_t p = b + lane;
       const int code = p < p1 ? dcode[p] : 255;
@@ -986,16 +1017,27 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       __syncwarp();
     }
     __syncthreads();
-    uint32_t total = 0;  // in direction `lane`
+    uint32_t mine = 0;
     if (threadIdx.x < 28) {
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) {
         const uint32_t t = rk.wcnt[w][lane];
-        rk.wcnt[w][lane] = total;
-        total += t;
+        rk.wcnt[w][lane] = mine;
+        mine += t;
       }
+      if constexpr (CLUSTER) pc.count[lane] = mine;
     }
+    if (CLUSTER) cg::this_cluster().sync();
+    uint32_t total = mine;  // of the block, in direction `lane`
     if (threadIdx.x < 32) {
+      uint32_t before = 0;  // in the parts before this one
+      if constexpr (CLUSTER) {
+        for (uint32_t r = 0; r < nparts; ++r) {
+          const uint32_t t = r == part || lane >= 28 ? 0u : cg::this_cluster().map_shared_rank(pc.count, r)[lane];
+          total += t;
+          before += r < part ? t : 0u;
+        }
+      }
       const uint32_t cv = lane < 27 ? total : 0u;
       uint32_t incl = cv;
 #pragma unroll
@@ -1006,14 +1048,16 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       if (lane < 27) {
         const uint32_t pre = incl - cv;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) rk.wcnt[w][lane] += pre;
-        cur.prefix28[item * 28 + lane] = pre;
+        for (int w = 0; w < kWarps; ++w) rk.wcnt[w][lane] += pre + before;
+        if (part == 0) cur.prefix28[item * 28 + lane] = pre;
       }
-      if (lane == 26) cur.prefix28[item * 28 + 27] = incl;
+      if (lane == 26 && part == 0) cur.prefix28[item * 28 + 27] = incl;
     }
     __syncthreads();
+    // The parts' counts have been read: the next block may overwrite them once all arrive.
+    if (CLUSTER) cg::this_cluster().barrier_arrive();
     // The next list's totals.
-    if (threadIdx.x < 28 && total > 0) {
+    if (threadIdx.x < 28 && part == 0 && total > 0) {
       if (lane == 27) {
         atomicAdd(&scal->lost, total);
       } else {
@@ -1027,13 +1071,14 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       const uint32_t mask = __match_any_sync(0xffffffffu, code);
       if (code < 27) {
         const uint32_t r = rk.wcnt[wid][code] + __popc(mask & ((1u << lane) - 1u));
-        if (start + r < md.cap_particles) cur.idx[start + r] = static_cast<uint16_t>(p);
+        if (start + r < md.cap_particles) cur.idx[start + r] = static_cast<uint16_t>(q0 + p);
       }
       __syncwarp();
       if (code < 27 && lane == 31 - __clz(mask)) rk.wcnt[wid][code] += __popc(mask);
       __syncwarp();
     }
     flush_tile<NT>(sc, key, ptile, ratio, gout);
+    if (CLUSTER) cg::this_cluster().barrier_wait();
   }
 }
 

@@ -139,6 +139,17 @@ __global__ void noalloc_fill_kernel(uint32_t n, float* x, float* v, float* F, fl
   if (aux) aux[i] = nan;
 }
 
+template <bool CLUSTER>
+FusedFn na_fused(int32_t kind) {
+  switch (kind) {
+    case CKMPM_FIXED_COROTATED: return g2p2g_kernel<kFixedCorotated, kFusedThreads, false, CLUSTER>;
+    case CKMPM_DRUCKER_PRAGER: return g2p2g_kernel<kDruckerPrager, kFusedThreads, false, CLUSTER>;
+    case CKMPM_VON_MISES: return g2p2g_kernel<kVonMises, kFusedThreads, false, CLUSTER>;
+    case CKMPM_NACC: return g2p2g_kernel<kNacc, kFusedThreads, false, CLUSTER>;
+    default: return g2p2g_kernel<kFluid, kFusedThreads, false, CLUSTER>;
+  }
+}
+
 ckmpm_status na_fail(const char** message, ckmpm_status code, const char* text) {
   if (message) *message = text;
   return code;
@@ -314,29 +325,19 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
   finish_setup_kernel<<<1, 32, 0, st>>>(scal, n - n_valid, 0.f, 0.f, 0.f);  // keeps setup's status bits
   NA_CUDA(cudaGetLastError());
 
-  // Substeps: the launch sequence of ckmpm_step without graphs.
+  // Substeps: the launch sequence of ckmpm_step without graphs, in its launch shape.
+  const uint32_t parts = cluster_parts(sms, counts[0]);
   const bool fold = folds_zero(sc, counts[0]);
+  const FusedFn fused = parts > 1 ? na_fused<true>(material->kind) : na_fused<false>(material->kind);
   if (nsteps > 0) set_next_dt_kernel<<<1, 32, 0, st>>>(scal, dt);
   for (uint32_t i = 0; i < nsteps; ++i) {
     const int parity = static_cast<int>(i & 1);
     const ModelDev md = for_substep(d, parity);
     const GridDev gd = for_substep(grid, parity);
-    switch (material->kind) {
-      case CKMPM_FIXED_COROTATED:
-        g2p2g_kernel<kFixedCorotated, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
-        break;
-      case CKMPM_DRUCKER_PRAGER:
-        g2p2g_kernel<kDruckerPrager, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
-        break;
-      case CKMPM_VON_MISES:
-        g2p2g_kernel<kVonMises, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
-        break;
-      case CKMPM_NACC:
-        g2p2g_kernel<kNacc, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
-        break;
-      default:
-        g2p2g_kernel<kFluid, kFusedThreads><<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
-    }
+    if (parts > 1)
+      NA_CUDA(launch_clusters(fused, cluster_ctas(sms), kFusedThreads, parts, st, sc, md, gd, scal));
+    else
+      fused<<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
     NA_CUDA(launch_compact(sc, d, grid, scal, ntiles, st, parity ^ 1, parity, fold ? parity : -1, true));
     if (!fold)
       zero_windows_kernel<<<sms * 4, 256, 0, st>>>(sc, d.bl[parity ^ 1], grid.grid[parity], grid.stamp[parity], scal, 2,
