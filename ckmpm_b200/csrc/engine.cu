@@ -90,6 +90,9 @@ struct ckmpm_scene {
   std::vector<std::pair<void*, size_t>> allocs;
   size_t n_state_allocs = 0;
   cudaGraphExec_t graph_chunk = nullptr;
+  // A chunk of adaptive substeps, captured for these bounds (ckmpm_step_adaptive).
+  cudaGraphExec_t graph_adaptive = nullptr;
+  float adaptive_dt_max = 0.f, adaptive_cfl = 0.f;
   uint64_t host_step = 0;
   uint32_t nblocks0 = 0;   // active blocks at setup (the largest model's)
   // Substeps between re-layouts of the particles (reorder_gather_kernel); 0 = never.
@@ -147,7 +150,8 @@ cudaError_t dalloc(ckmpm_scene* s, T** p, size_t count) {
 
 void free_graphs(ckmpm_scene* s) {
   if (s->graph_chunk) cudaGraphExecDestroy(s->graph_chunk);
-  s->graph_chunk = nullptr;
+  if (s->graph_adaptive) cudaGraphExecDestroy(s->graph_adaptive);
+  s->graph_chunk = s->graph_adaptive = nullptr;
 }
 
 // Launches a fused kernel of the cluster shape: `parts` CTAs per cluster.
@@ -359,13 +363,26 @@ cudaError_t enqueue_substep(ckmpm_scene* s, int parity) {
   return e;
 }
 
+// One adaptive substep: the CFL dt from the grid it reads, then the substep.
+cudaError_t enqueue_adaptive_substep(ckmpm_scene* s, int parity_of_step) {
+  float mass_floor = 0.f;
+  for (const auto& m : s->models) mass_floor = (mass_floor == 0.f) ? m.mass : std::min(mass_floor, m.mass);
+  mass_floor *= 1.52587890625e-05f;  // 2^-16
+  const uint32_t ctas = std::min<uint32_t>((s->sc.nblocks_domain + kMaxvBlocks - 1) / kMaxvBlocks,
+                                           static_cast<uint32_t>(s->sm_count) * 16u);
+  grid_maxv_kernel<<<ctas, kMaxvThreads, 0, s->stream>>>(s->sc, s->grid, s->scal, mass_floor, s->adaptive_cfl,
+                                                         s->adaptive_dt_max);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? enqueue_substep(s, parity_of_step) : e;
+}
+
 // A graph of nsub substeps, the first of even parity.
-cudaError_t build_graph(ckmpm_scene* s, int nsub, cudaGraphExec_t* exec) {
+cudaError_t build_graph(ckmpm_scene* s, int nsub, bool adaptive, cudaGraphExec_t* exec) {
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return e;
   for (int i = 0; i < nsub; ++i) {
-    e = enqueue_substep(s, i & 1);
+    e = adaptive ? enqueue_adaptive_substep(s, i & 1) : enqueue_substep(s, i & 1);
     if (e != cudaSuccess) break;
   }
   cudaError_t e2 = cudaStreamEndCapture(s->stream, &g);
@@ -1073,7 +1090,7 @@ ckmpm_status ckmpm_step_async(ckmpm_scene* s, uint32_t nsteps, float dt) {
     const int parity = static_cast<int>(s->host_step & 1);
     const uint32_t chunk = s->tune.graph_chunk;
     if (parity == 0 && nsteps - done >= chunk && !reorder_inside(s, chunk)) {
-      if (!s->graph_chunk) CK_CUDA(s, build_graph(s, static_cast<int>(chunk), &s->graph_chunk));
+      if (!s->graph_chunk) CK_CUDA(s, build_graph(s, static_cast<int>(chunk), false, &s->graph_chunk));
       CK_CUDA(s, cudaGraphLaunch(s->graph_chunk, s->stream));
       done += chunk;
       s->host_step += chunk;
@@ -1114,10 +1131,13 @@ ckmpm_status ckmpm_step_adaptive(ckmpm_scene* s, uint32_t nsteps, float dt_max, 
   // steps one substep at a time, e.g. to record per-substep diagnostics).
   const double t0 = h.time, t_end = frame_time > 0.0 ? h.time + frame_time : h.frame_end;
   if (frame_time > 0.0) set_frame_end_kernel<<<1, 32, 0, s->stream>>>(s->scal, frame_time);
-  const int maxv_ctas = s->sm_count * 8;
-  float mass_floor = 0.f;
-  for (const auto& m : s->models) mass_floor = (mass_floor == 0.f) ? m.mass : std::min(mass_floor, m.mass);
-  mass_floor *= 1.52587890625e-05f;  // 2^-16
+  // The stream is idle here: a graph captured for other bounds can go.
+  if (s->graph_adaptive && (s->adaptive_dt_max != dt_max || s->adaptive_cfl != cfl)) {
+    cudaGraphExecDestroy(s->graph_adaptive);
+    s->graph_adaptive = nullptr;
+  }
+  s->adaptive_dt_max = dt_max;
+  s->adaptive_cfl = cfl;
   uint32_t taken = 0;
   // Each substep advances by at most dt_max, so floor(remaining / dt_max)
   // substeps never pass the frame end; the last one is clipped to it on the
@@ -1127,13 +1147,20 @@ ckmpm_status ckmpm_step_adaptive(ckmpm_scene* s, uint32_t nsteps, float dt_max, 
     if (!(remaining > 0.0) || taken >= nsteps) break;
     uint32_t k = static_cast<uint32_t>(remaining / static_cast<double>(dt_max));
     k = std::max<uint32_t>(1u, std::min<uint32_t>(k, nsteps - taken));
-    for (uint32_t i = 0; i < k; ++i) {
+    for (uint32_t i = 0; i < k;) {
       if (reorder_due(s)) CK_CUDA(s, enqueue_reorder(s));
       const int parity = static_cast<int>(s->host_step & 1);
-      grid_maxv_kernel<<<maxv_ctas, 256, 0, s->stream>>>(s->sc, s->grid, s->scal, mass_floor);
-      adaptive_dt_kernel<<<1, 32, 0, s->stream>>>(s->scal, s->sc.dx, cfl, dt_max);
-      CK_CUDA(s, enqueue_substep(s, parity));
-      ++s->host_step;
+      const uint32_t chunk = s->tune.graph_chunk;
+      if (parity == 0 && k - i >= chunk && !reorder_inside(s, chunk)) {
+        if (!s->graph_adaptive) CK_CUDA(s, build_graph(s, static_cast<int>(chunk), true, &s->graph_adaptive));
+        CK_CUDA(s, cudaGraphLaunch(s->graph_adaptive, s->stream));
+        i += chunk;
+        s->host_step += chunk;
+      } else {
+        CK_CUDA(s, enqueue_adaptive_substep(s, parity));
+        ++i;
+        ++s->host_step;
+      }
     }
     taken += k;
     CK_CUDA(s, cudaMemcpyAsync(&h, s->scal, sizeof(Scalars), cudaMemcpyDeviceToHost, s->stream));
@@ -1411,7 +1438,7 @@ ckmpm_status ckmpm_autotune(ckmpm_scene* s, uint32_t probe_steps, float dt, ckmp
   // Applying the pick dropped the graphs of the last probed shape: capture the
   // chosen shape's chunk graph now (capture runs nothing), so that the first
   // ckmpm_step_async after tuning does not pay for it.
-  CK_CUDA(s, build_graph(s, static_cast<int>(s->tune.graph_chunk), &s->graph_chunk));
+  CK_CUDA(s, build_graph(s, static_cast<int>(s->tune.graph_chunk), false, &s->graph_chunk));
   return CKMPM_OK;
 }
 
