@@ -64,6 +64,7 @@ struct ModelHost {
   std::vector<SceneMat> smat;
   std::vector<uint32_t> sstart;
   std::vector<int32_t> skind;
+  bool core = false;  // batch: every scene is fixed-corotated, Drucker-Prager or fluid
 };
 
 }  // namespace
@@ -201,7 +202,7 @@ template <int NT, bool CLUSTER = false>
 cudaError_t launch_fused_nt(ckmpm_scene* s, const ModelHost& m, int parity) {
   // batches have no rigid particles
   if (m.mat.kind == kMixedKind)
-    return launch_fused<kMixed, NT, false, CLUSTER>(s, m, parity);
+    return m.core ? launch_fused<kMixedCore, NT, false, CLUSTER>(s, m, parity) : launch_fused<kMixed, NT, false, CLUSTER>(s, m, parity);
   return s->sc.rigid ? launch_fused_kind<NT, true, CLUSTER>(s, m, parity) : launch_fused_kind<NT, false, CLUSTER>(s, m, parity);
 }
 
@@ -234,7 +235,8 @@ int shape_index(uint32_t threads) {
 
 template <int NT, bool CLUSTER>
 cudaError_t set_fused_attributes(int* occ) {
-  const void* fns[13] = {reinterpret_cast<const void*>(g2p2g_kernel<kFixedCorotated, NT, false, CLUSTER>),
+  const void* fns[14] = {reinterpret_cast<const void*>(g2p2g_kernel<kMixedCore, NT, false, CLUSTER>),
+                         reinterpret_cast<const void*>(g2p2g_kernel<kFixedCorotated, NT, false, CLUSTER>),
                          reinterpret_cast<const void*>(g2p2g_kernel<kLinear, NT, false, CLUSTER>),
                          reinterpret_cast<const void*>(g2p2g_kernel<kDruckerPrager, NT, false, CLUSTER>),
                          reinterpret_cast<const void*>(g2p2g_kernel<kFluid, NT, false, CLUSTER>),
@@ -767,6 +769,9 @@ ckmpm_status ckmpm_add_batch(ckmpm_scene* s, uint32_t nscenes, const ckmpm_batch
   if (total == 0 || total > 0xFFFFFFF0ull) return fail(s, CKMPM_ERR_INVALID, "batch particle count out of range");
   m.sstart[nscenes] = static_cast<uint32_t>(total);
   m.n = static_cast<uint32_t>(total);
+  m.core = std::all_of(m.skind.begin(), m.skind.end(), [](int32_t k) {
+    return k == CKMPM_FIXED_COROTATED || k == CKMPM_DRUCKER_PRAGER || k == CKMPM_FLUID;
+  });
   m.nv = m.n;
   m.mass = lightest;  // only the adaptive-dt mass floor reads it for a batch
   m.vol = 1.f;

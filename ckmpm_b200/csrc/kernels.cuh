@@ -91,6 +91,10 @@ struct SceneMat {
 };
 
 constexpr int kMixed = 7;  // material kind read per work item from the scene's SceneMat
+// The same for batches of fixed-corotated, Drucker-Prager and fluid scenes only: without
+// the other materials' code the kernel needs fewer registers than it has to spill.
+constexpr int kMixedCore = 8;
+constexpr bool is_mixed(int kind) { return kind == kMixed || kind == kMixedCore; }
 
 struct Scalars {
   int32_t step;        // substeps taken; epoch of the grid that the next substep reads
@@ -825,7 +829,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     // an ulp), so both forms start from the same constants.
     float vol_over_mass = __fdiv_rn(md.vol, md.mass), unit = sc.grid_unit;
     double ratio = md.flush_ratio;
-    if (KIND == kMixed) {
+    if (is_mixed(KIND)) {
       const SceneMat& sm = md.smat[key.w];
       kind = sm.kind;
       mp0 = sm.p[0];
@@ -914,23 +918,25 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
           stress_fixed_corotated(mp0, mp1, F, tau);
         } else if (kind == kDruckerPrager) {
           stress_drucker_prager(mp0, mp1, F, aux, tau);
-        } else if (kind == kVonMises) {
-          stress_von_mises(mp0, mp1, mp2, F, tau);
-        } else if (kind == kNacc) {
-          float prm[kMaterialParams];
+        } else if constexpr (KIND != kMixedCore) {
+          if (kind == kVonMises) {
+            stress_von_mises(mp0, mp1, mp2, F, tau);
+          } else if (kind == kNacc) {
+            float prm[kMaterialParams];
 #pragma unroll
-          for (int k = 0; k < kMaterialParams; ++k) prm[k] = KIND == kMixed ? md.smat[key.w].p[k] : md.mat.p[k];
-          stress_nacc(prm, F, aux, tau);
-        } else {  // kLinear
-          float Q[9], C[9];
+            for (int k = 0; k < kMaterialParams; ++k) prm[k] = KIND == kMixed ? md.smat[key.w].p[k] : md.mat.p[k];
+            stress_nacc(prm, F, aux, tau);
+          } else {  // kLinear
+            float Q[9], C[9];
 #pragma unroll
-          for (int k = 0; k < 9; ++k) {
-            Q[k] = sin.Q[k][iin];
-            C[k] = __fmul_rn(Cdx[k], inv_dx);
+            for (int k = 0; k < 9; ++k) {
+              Q[k] = sin.Q[k][iin];
+              C[k] = __fmul_rn(Cdx[k], inv_dx);
+            }
+            stress_linear(C, dt, F, Q, tau);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) sout.Q[k][o_slot(start, q)] = Q[k];
           }
-          stress_linear(C, dt, F, Q, tau);
-#pragma unroll
-          for (int k = 0; k < 9; ++k) sout.Q[k][o_slot(start, q)] = Q[k];
         }
       }
 
