@@ -1196,7 +1196,9 @@ static cudaError_t ensure_export_buffers(ckmpm_scene*, ModelHost& m) {
 
 // Enqueues the gather of the requested per-particle arrays into the model's
 // export buffers (input order when ids are tracked).  n_upper bounds the live
-// count; n_dev, when given, is the device copy of it.
+// count; n_dev, when given, is the device copy of it, else n_upper is the count.
+// While no particle has been lost, input order is the order of the ids, and the
+// passes that place live ids are left out (or, the count not known here, do nothing).
 static cudaError_t enqueue_export(ckmpm_scene* s, ModelHost& m, bool x, bool v, bool F, bool aux, bool id,
                                   uint32_t n_upper, const uint32_t* n_dev) {
   const size_t cap_p = m.dev.cap_particles;
@@ -1204,10 +1206,11 @@ static cudaError_t enqueue_export(ckmpm_scene* s, ModelHost& m, bool x, bool v, 
   const uint32_t* dest = nullptr;
   cudaError_t e;
   if (m.copy_pending && (e = cudaStreamWaitEvent(s->stream, m.ev_copied, 0)) != cudaSuccess) return e;
-  if (m.dev.track_ids) {
+  const bool all_live = m.dev.track_ids && !n_dev && n_upper == m.dev.cap_particles;
+  if (m.dev.track_ids && !all_live) {
     // ids in block order, then the position of each live id in input order
     probe_kernel<kProbeThreads><<<pg, pb, kSmemVTile, s->stream>>>(s->sc, m.dev, s->grid, s->scal, nullptr, nullptr,
-                                                                 nullptr, nullptr, m.oid, nullptr);
+                                                                 nullptr, nullptr, m.oid, nullptr, 0, 1);
     if ((e = cudaMemsetAsync(m.oflag, 0, sizeof(uint32_t) * cap_p, s->stream)) != cudaSuccess) return e;
     if (n_upper)
       mark_ids_kernel<<<(n_upper + 255) / 256, 256, 0, s->stream>>>(n_upper, m.oid, m.oflag,
@@ -1220,7 +1223,8 @@ static cudaError_t enqueue_export(ckmpm_scene* s, ModelHost& m, bool x, bool v, 
   }
   probe_kernel<kProbeThreads><<<pg, pb, kSmemVTile, s->stream>>>(s->sc, m.dev, s->grid, s->scal, x ? m.ox : nullptr,
                                                                v ? m.ov : nullptr, F ? m.oF : nullptr,
-                                                               aux ? m.oaux : nullptr, id ? m.oid : nullptr, dest);
+                                                               aux ? m.oaux : nullptr, id ? m.oid : nullptr, dest,
+                                                               all_live ? 1 : 0, 0);
   return cudaGetLastError();
 }
 

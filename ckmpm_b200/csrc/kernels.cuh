@@ -1848,12 +1848,15 @@ __global__ void dd_unpack_kernel(long long* __restrict__ g, int32_t* __restrict_
 // Gathers the current state (x, F, aux, id) and interpolates v at each
 // particle from the current grid with the grid update applied, as the next
 // G2P will (include/mpm_algorithm.cuh:1306-1331).  Output slot: block order,
-// or dest[id] when dest is given (ids tracked).  Materials without F write
-// the identity, without aux zero (per scene in a batch).
+// or by id: dest[id] when dest is given (ids tracked), the id itself when every
+// particle is live (nothing lost: `all_live`, or as many live as the model's capacity
+// when `dest` is given).  skip_all_live: the pass that lists ids for the scan, which
+// has nothing to do then.  Materials without F write the identity, without aux zero
+// (per scene in a batch).
 template <int NT>
 __global__ void __launch_bounds__(NT) probe_kernel(SceneDev sc, ModelDev md, GridDev gd, Scalars* scal, float* ox,
                                                   float* ov, float* oF, float* oaux, uint32_t* oid,
-                                                  const uint32_t* __restrict__ dest) {
+                                                  const uint32_t* __restrict__ dest, int all_live, int skip_all_live) {
   extern __shared__ __align__(16) unsigned char smem[];
   float4* vtile = reinterpret_cast<float4*>(smem);
   __shared__ SharedSmall sh;
@@ -1864,6 +1867,9 @@ __global__ void __launch_bounds__(NT) probe_kernel(SceneDev sc, ModelDev md, Gri
   const StateDev sin = md.st[parity];
   const uint32_t nb = *cur.nblocks;
   const float dt = scal->cur_dt;
+  const bool complete = *cur.nparticles == md.cap_particles;
+  if (skip_all_live && complete) return;
+  const bool by_id = all_live || (dest && complete);
   load_classes(sc, sh.classes);
   __syncthreads();
   for (uint32_t item = blockIdx.x; item < nb; item += gridDim.x) {
@@ -1889,7 +1895,7 @@ __global__ void __launch_bounds__(NT) probe_kernel(SceneDev sc, ModelDev md, Gri
         iin = 0;
       }
       const uint32_t pid = sin.id ? sin.id[iin] : start + q;
-      const uint32_t o = dest ? dest[pid] : start + q;
+      const uint32_t o = by_id ? pid : dest ? dest[pid] : start + q;
       const float x[3] = {sin.x[0][iin], sin.x[1][iin], sin.x[2][iin]};
       if (ox) {
         ox[3 * o] = x[0];
@@ -1930,6 +1936,7 @@ __global__ void mark_ids_kernel(uint32_t n, const uint32_t* __restrict__ ids, ui
                                uint32_t cap, const uint32_t* __restrict__ n_dev) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t live = n_dev ? min(n, *n_dev) : n;
+  if (live == cap) return;  // every particle is live: no list was written and none is needed
   if (i < live && ids[i] < cap) flag[ids[i]] = 1u;
 }
 

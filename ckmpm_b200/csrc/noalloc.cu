@@ -350,7 +350,7 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
   uint32_t live = 0;
   NA_CUDA(cudaMemcpyAsync(&live, cur.nparticles, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   probe_kernel<kProbeThreads><<<sms * 4, kProbeThreads, kSmemVTile, st>>>(sc, d, grid, scal, ex, ev, hasF ? eF : nullptr,
-                                                                         hasAux ? ea : nullptr, eid, nullptr);
+                                                                         hasAux ? ea : nullptr, eid, nullptr, 0, 0);
   NA_CUDA(cudaStreamSynchronize(st));
   if (x_out || v_out || F_out || aux_out) {
     noalloc_fill_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, x_out, v_out, F_out, aux_out);
