@@ -426,11 +426,11 @@ def run_diff(args, rank, world, local_rank):
         "train_step_particle_substeps_per_s": n * nsteps / (ms / 1e3),
         "gradcheck": gradcheck, "loss": float(loss.item()), "clocks": clocks, "roofline": roofline,
         "cpu_baseline": cpu,
-        # per training step: forward (init, box reset, raster, grid + particle per substep, last grid
-        # update, 2 layout copies: 2 nsteps + 6), backward (2 layout copies, seed max, scale; grid and
+        # per training step: forward (5 ordering kernels, init, box reset, raster, grid + particle per
+        # substep, last grid update, 2 layout copies: 2 nsteps + 11), backward (2 layout copies, seed max, scale; grid and
         # particle kernels of the recomputed substeps, 2 (len - 1) per segment; grid and particle
         # adjoint per substep; finish: 4 nsteps - 2 nseg + 5)
-        "gpu_launches": steps * (6 * nsteps - 2 * (-(-nsteps // d["checkpoint_every"])) + 11),
+        "gpu_launches": steps * (6 * nsteps - 2 * (-(-nsteps // d["checkpoint_every"])) + 16),
         "e2e": {"value": n * nsteps / (e2e_ms / 1e3), "unit": METRIC, "h2d_bytes_per_step": n * (12 + 12 + 4),
                 "d2h_bytes_per_step": 4 + n * (12 + 4),
                 "includes": "per step: x0, v0, log E uploaded from pinned host memory, forward + adjoint rollout "

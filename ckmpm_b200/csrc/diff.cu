@@ -56,89 +56,228 @@ __device__ __forceinline__ void box_reset(int* b) {
   b[3] = b[4] = b[5] = INT_MIN;
 }
 
-// Block-reduce a node box and merge it into b.
-__device__ __forceinline__ void box_merge(int* b, int lo0, int lo1, int lo2, int hi0, int hi1, int hi2) {
-  __shared__ int s[6];
-  if (threadIdx.x < 3) s[threadIdx.x] = INT_MAX;
-  else if (threadIdx.x < 6) s[threadIdx.x] = INT_MIN;
-  __syncthreads();
-  if (lo0 <= hi0) {
-    atomicMin(&s[0], lo0);
-    atomicMin(&s[1], lo1);
-    atomicMin(&s[2], lo2);
-    atomicMax(&s[3], hi0);
-    atomicMax(&s[4], hi1);
-    atomicMax(&s[5], hi2);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && s[0] <= s[3]) {
-    atomicMin(&b[0], s[0]);
-    atomicMin(&b[1], s[1]);
-    atomicMin(&b[2], s[2]);
-    atomicMax(&b[3], s[3]);
-    atomicMax(&b[4], s[4]);
-    atomicMax(&b[5], s[5]);
+// ---- Particle order
+//
+// The rollout keeps its particles in an order of its own, made from x0 by every
+// forward: pencils of 2 x 2 cells in x and y, run through in z, neighbouring
+// pencils in opposite directions, so that the kThreads particles of a CTA lie in
+// a few cells of one pencil.  Their stencils then read the same nodes (L1 hits
+// instead of L2 gathers) and their deposits fit a small shared tile.  Nothing
+// depends on the order: every particle computes by itself and the node sums are
+// exact.  Within a chunk of kThreads, particle j of the sorted order takes place
+// (j % 4) * 32 + j / 4: a warp's lanes then spread over the whole chunk's cells,
+// so fewer of them add to the same words at once.
+__host__ __device__ __forceinline__ uint32_t order_bins(const DenseGrid& G) {
+  return static_cast<uint32_t>(G.n[0] / 2) * static_cast<uint32_t>(G.n[1] / 2) * static_cast<uint32_t>(G.n[2]);
+}
+
+__device__ __forceinline__ uint32_t order_bin(const Dev& d, const float* x) {
+  int c[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) c[a] = min(max(static_cast<int>(x[a] * d.inv_dx), 0), d.G.n[a] - 1);
+  const int px = c[0] >> 1, py = c[1] >> 1, ny = d.G.n[1] >> 1;
+  const int y = (px & 1) ? ny - 1 - py : py;
+  const int z = ((px * ny + y) & 1) ? d.G.n[2] - 1 - c[2] : c[2];
+  return static_cast<uint32_t>((px * ny + y) * d.G.n[2] + z);
+}
+
+__global__ void order_count_kernel(Dev d, const float* __restrict__ x0, uint32_t* __restrict__ bins,
+                                   uint32_t* __restrict__ bin, uint32_t* __restrict__ rank) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= d.n) return;
+  const uint32_t b = order_bin(d, x0 + 3 * static_cast<size_t>(p));
+  bin[p] = b;
+  rank[p] = atomicAdd(bins + b, 1u);
+}
+
+__global__ void order_place_kernel(uint32_t n, const uint32_t* __restrict__ first, const uint32_t* __restrict__ bin,
+                                   const uint32_t* __restrict__ rank, uint32_t* __restrict__ perm) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  uint32_t j = first[bin[p]] + rank[p];
+  const uint32_t chunk = j / kThreads * kThreads;
+  if (chunk + kThreads <= n) j = chunk + ((j - chunk) % 4) * (kThreads / 4) + (j - chunk) / 4;
+  perm[j] = p;
+}
+
+// ---- CTA tile
+//
+// Box of base cells (both grids) of the CTA's particles and the nodes they reach.
+// Deposits go to a shared tile of exact 64-bit sums over that box, two native
+// 32-bit atomics per value with the carry from the low word (as the substep's
+// P2G tile), and from there to the grid, one reduction per touched node and
+// channel; a box of more than kTileNodes nodes deposits into the grid directly.
+// The sums are exact either way.  Bound before: 64 global 64-bit reductions per
+// particle, 3.2 M a launch on the 50k-particle cube.
+constexpr int kTileCap = 1024;  // nodes of both grids
+
+struct CtaBox {
+  int lo[3], e[3];  // first node, nodes per axis (one grid)
+  int nodes;        // of both grids; 0: no tile
+};
+
+__device__ __forceinline__ void cta_box_merge(int* s_box, bool use, const int* lo, const int* hi) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int l = __reduce_min_sync(0xffffffffu, use ? lo[a] : INT_MAX);
+    const int h = __reduce_max_sync(0xffffffffu, use ? hi[a] : INT_MIN);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(s_box + a, l);
+      atomicMax(s_box + 3 + a, h);
+    }
   }
 }
 
-__device__ __forceinline__ void fixed_add64(unsigned long long* p, float v) {
-  atomicAdd(p, static_cast<unsigned long long>(__float2ll_rn(v * kScale)));
+__device__ __forceinline__ CtaBox cta_box(const int* s_box) {
+  CtaBox b;
+  int64_t v = 2;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    b.lo[a] = s_box[a];
+    b.e[a] = s_box[3 + a] >= s_box[a] ? s_box[3 + a] - s_box[a] + 1 : 0;
+    v *= b.e[a];
+  }
+  b.nodes = v <= kTileCap ? static_cast<int>(v) : 0;
+  return b;
 }
 
-// Deposit nodes of one particle (per unit mass) into gsum; returns its node box.
-__device__ __forceinline__ void deposit(const Dev& d, const Fwd<float>& f, unsigned long long* gsum, int* lo, int* hi) {
-  diff::particle_deposit(f, d.dx, d.inv_dx, [&](int g, int cx, int cy, int cz, float w, const float* wv) {
-    if (!diff::node_in_grid(d.G, cx, cy, cz)) {
+__device__ __forceinline__ void tile_zero(unsigned* tile, int words) {
+  for (int i = threadIdx.x; i < words / 4; i += kThreads) reinterpret_cast<uint4*>(tile)[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Exact add to word pair `lo_word`, its high word `plane` words later.
+__device__ __forceinline__ void tile_add(unsigned* lo_word, int plane, long long v) {
+  const unsigned lo = static_cast<unsigned>(v);
+  const unsigned old = atomicAdd(lo_word, lo);
+  atomicAdd(lo_word + plane, static_cast<unsigned>(v >> 32) + (old + lo < lo ? 1u : 0u));
+}
+
+// Adds the tile's touched words to the grid arrays (kCh channels per node).
+template <int kCh>
+__device__ __forceinline__ void tile_flush(const Dev& d, const CtaBox& b, const unsigned* tile,
+                                           unsigned long long* __restrict__ out) {
+  const int per = b.nodes >> 1, plane = kCh * kTileCap;
+  for (int i = threadIdx.x; i < b.nodes; i += kThreads) {
+    const int g = i >= per ? 1 : 0, j = i - g * per;
+    const int z = j % b.e[2], xy = j / b.e[2], y = xy % b.e[1], x = xy / b.e[1];
+    unsigned long long* q = out + kCh * diff::node_index(d.G, g, b.lo[0] + x, b.lo[1] + y, b.lo[2] + z);
+#pragma unroll
+    for (int c = 0; c < kCh; ++c) {
+      const unsigned long long v = static_cast<unsigned long long>(tile[c * kTileCap + i]) |
+                                   (static_cast<unsigned long long>(tile[c * kTileCap + i + plane]) << 32);
+      if (v) atomicAdd(q + c, v);
+    }
+  }
+}
+
+// First and last node of a particle's stencils over both grids.  A position far
+// outside (or infinite) saturates the base cells, so `hi` may wrap: box_in_grid
+// bounds both ends.
+__device__ __forceinline__ void stencil_box(const diff::Stencil<float>& st, int* lo, int* hi) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = min(st.a[0][a].base, st.a[1][a].base);
+    hi[a] = max(st.a[0][a].base, st.a[1][a].base) + 1;
+  }
+}
+
+__device__ __forceinline__ bool box_in_grid(const DenseGrid& G, const int* lo, const int* hi) {
+  bool in = true;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) in &= lo[a] >= 0 && lo[a] < G.n[a] && hi[a] >= lo[a] && hi[a] < G.n[a];
+  return in;
+}
+
+// Deposits of the CTA's particles (per unit mass) into gsum and the merge of their
+// node box into `box`.  Collective; s_box holds an empty box on entry and the tile
+// zeros (both before the caller's last barrier).  A particle whose stencil leaves
+// the grid is reported and deposits the nodes it has inside.
+__device__ __forceinline__ void cta_deposit(const Dev& d, bool active, const Fwd<float>& f, unsigned* tile, int* s_box,
+                                            unsigned long long* __restrict__ gsum, int* box) {
+  int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+  bool inside = false;
+  if (active) {
+    stencil_box(f.stn, lo, hi);
+    inside = box_in_grid(d.G, lo, hi);
+    if (!inside) {
       atomicOr(d.status, kErrOutside);
-      return;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {  // the part of the stencil that is in the grid
+        lo[a] = min(max(lo[a], 0), d.G.n[a] - 1);
+        hi[a] = min(max(hi[a], 0), d.G.n[a] - 1);
+      }
     }
-    if (!(fabsf(wv[0]) < kMaxValue && fabsf(wv[1]) < kMaxValue && fabsf(wv[2]) < kMaxValue)) {
-      atomicOr(d.status, kErrRange);
-      return;
-    }
-    unsigned long long* q = gsum + 4 * diff::node_index(d.G, g, cx, cy, cz);
-    fixed_add64(q, w);
-    fixed_add64(q + 1, wv[0]);
-    fixed_add64(q + 2, wv[1]);
-    fixed_add64(q + 3, wv[2]);
-    lo[0] = min(lo[0], cx);
-    lo[1] = min(lo[1], cy);
-    lo[2] = min(lo[2], cz);
-    hi[0] = max(hi[0], cx);
-    hi[1] = max(hi[1], cy);
-    hi[2] = max(hi[2], cz);
-  });
+  }
+  cta_box_merge(s_box, active, lo, hi);
+  __syncthreads();
+  const CtaBox b = cta_box(s_box);
+  if (threadIdx.x < 3 && b.e[0] > 0 && b.e[1] > 0 && b.e[2] > 0) {
+    atomicMin(box + threadIdx.x, s_box[threadIdx.x]);
+    atomicMax(box + 3 + threadIdx.x, s_box[3 + threadIdx.x]);
+  }
+  if (active) {
+    const int per = b.nodes >> 1;
+    diff::particle_deposit(f, d.dx, d.inv_dx, [&](int g, int cx, int cy, int cz, float w, const float* wv) {
+      if (!inside && !diff::node_in_grid(d.G, cx, cy, cz)) return;
+      if (!(fabsf(wv[0]) < kMaxValue && fabsf(wv[1]) < kMaxValue && fabsf(wv[2]) < kMaxValue)) {
+        atomicOr(d.status, kErrRange);
+        return;
+      }
+      const long long v[4] = {__float2ll_rn(w * kScale), __float2ll_rn(wv[0] * kScale), __float2ll_rn(wv[1] * kScale),
+                              __float2ll_rn(wv[2] * kScale)};
+      if (per) {
+        unsigned* q = tile + g * per + ((cx - b.lo[0]) * b.e[1] + cy - b.lo[1]) * b.e[2] + cz - b.lo[2];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tile_add(q + c * kTileCap, 4 * kTileCap, v[c]);
+      } else {
+        unsigned long long* q = gsum + 4 * diff::node_index(d.G, g, cx, cy, cz);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) atomicAdd(q + c, static_cast<unsigned long long>(v[c]));
+      }
+    });
+  }
+  __syncthreads();
+  tile_flush<4>(d, b, tile, gsum);
 }
+
+constexpr size_t kDepositTile = sizeof(unsigned) * 2 * 4 * kTileCap;  // 32 KB
+constexpr size_t kAdjointTile = sizeof(unsigned) * 2 * 3 * kTileCap;  // 24 KB
 
 // AoS inputs -> SoA state; lambda / mu from log E; F = I.
 __global__ void init_kernel(Dev d, const float* __restrict__ x0, const float* __restrict__ logE, float nu,
-                            float* __restrict__ x, float* __restrict__ F, float* __restrict__ lam,
-                            float* __restrict__ mu) {
+                            const uint32_t* __restrict__ perm, float* __restrict__ x, float* __restrict__ F,
+                            float* __restrict__ lam, float* __restrict__ mu) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= d.n) return;
-  for (int a = 0; a < 3; ++a) x[a * d.n + p] = x0[3 * p + a];
+  const uint32_t u = perm[p];
+  for (int a = 0; a < 3; ++a) x[a * d.n + p] = x0[3 * u + a];
   for (int k = 0; k < 9; ++k) F[k * d.n + p] = (k & 3) ? 0.f : 1.f;
-  const float E = expf(logE[p]);
+  const float E = expf(logE[u]);
   mu[p] = E / (2.f * (1.f + nu));
   lam[p] = E * nu / ((1.f + nu) * (1.f - 2.f * nu));
 }
 
-__global__ void raster_kernel(Dev d, const float* __restrict__ x, const float* __restrict__ v0,
-                              unsigned long long* __restrict__ gsum, int* box) {
+__global__ void __launch_bounds__(kThreads) raster_kernel(Dev d, const float* __restrict__ x, const float* __restrict__ v0,
+                                                          const uint32_t* __restrict__ perm,
+                                                          unsigned long long* __restrict__ gsum, int* box) {
+  extern __shared__ __align__(16) unsigned tile[];
+  __shared__ int s_box[6];
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+  tile_zero(tile, 8 * kTileCap);
+  if (threadIdx.x == 0) box_reset(s_box);
+  Fwd<float> f;
   if (p < d.n) {
-    Fwd<float> f;
+    const uint32_t u = perm[p];
     const float xp[3] = {x[p], x[d.n + p], x[2 * d.n + p]};
     for (int a = 0; a < 3; ++a) {
       f.xn[a] = xp[a];
-      f.v[a] = v0[3 * p + a];
+      f.v[a] = v0[3 * u + a];
     }
     for (int k = 0; k < 9; ++k) f.A[k] = 0.f;
     diff::make_stencil(xp, d.inv_dx, f.stn);
-    deposit(d, f, gsum, lo, hi);
   }
-  box_merge(box, lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]);
+  __syncthreads();
+  cta_deposit(d, p < d.n, f, tile, s_box, gsum, box);
 }
 
 // Every substep's box starts empty; deposits widen it.  A recomputed segment
@@ -175,17 +314,34 @@ __global__ void grid_kernel(Dev d, unsigned long long* __restrict__ gsum, const 
   }
 }
 
-struct VelReader {
-  const DenseGrid* G;
-  const float4* vel;
-  uint32_t* status;
+// Reads a float4 per node of a particle's 16; the grid's bounds are checked once
+// for the whole stencil, per node only where it leaves the grid.
+struct NodeReader {
+  const Dev* d;
+  const float4* nodes;
+  bool inside;
+  __device__ NodeReader(const Dev& dev, const float4* q, const diff::Stencil<float>& st) : d(&dev), nodes(q) {
+    int lo[3], hi[3];
+    stencil_box(st, lo, hi);
+    inside = box_in_grid(dev.G, lo, hi);
+  }
+  __device__ bool get(int g, int cx, int cy, int cz, float4& q) const {
+    if (!inside && !diff::node_in_grid(d->G, cx, cy, cz)) return false;
+    q = nodes[diff::node_index(d->G, g, cx, cy, cz)];
+    return true;
+  }
+};
+
+struct VelReader : NodeReader {
+  __device__ VelReader(const Dev& dev, const float4* vel, const float* x) : NodeReader(dev, vel, stencil_at(dev, x)) {}
+  static __device__ diff::Stencil<float> stencil_at(const Dev& dev, const float* x) {
+    diff::Stencil<float> st;
+    diff::make_stencil(x, dev.inv_dx, st);
+    return st;
+  }
   __device__ void operator()(int g, int cx, int cy, int cz, float* v) const {
-    if (!diff::node_in_grid(*G, cx, cy, cz)) {
-      atomicOr(status, kErrOutside);
-      v[0] = v[1] = v[2] = 0.f;
-      return;
-    }
-    const float4 q = vel[diff::node_index(*G, g, cx, cy, cz)];
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!get(g, cx, cy, cz, q)) atomicOr(d->status, kErrOutside);
     v[0] = q.x;
     v[1] = q.y;
     v[2] = q.z;
@@ -209,20 +365,23 @@ __global__ void __launch_bounds__(kThreads) particle_kernel(Dev d, const float* 
                                                             const float* __restrict__ mu, const float4* __restrict__ vel,
                                                             float dt, float ndt, unsigned long long* __restrict__ gsum,
                                                             int* bnext, float* __restrict__ xo, float* __restrict__ Fo) {
+  extern __shared__ __align__(16) unsigned tile[];
+  __shared__ int s_box[6];
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+  tile_zero(tile, 8 * kTileCap);
+  if (threadIdx.x == 0) box_reset(s_box);
+  Fwd<float> f;
   if (p < d.n) {
     Particle<float> pp;
     load_particle(d, x, F, p, pp);
-    Fwd<float> f;
     float U[9], S[3], V[9];
-    VelReader vr{&d.G, vel, d.status};
+    VelReader vr(d, vel, pp.x);
     diff::particle_forward(pp, lam[p], mu[p], d.vol_over_mass, dt, ndt, d.dx, d.inv_dx, vr, Svd{}, f, U, S, V);
-    deposit(d, f, gsum, lo, hi);
     for (int a = 0; a < 3; ++a) xo[a * d.n + p] = f.xn[a];
     for (int k = 0; k < 9; ++k) Fo[k * d.n + p] = f.Fn[k];
   }
-  box_merge(bnext, lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]);
+  __syncthreads();
+  cta_deposit(d, p < d.n, f, tile, s_box, gsum, bnext);
 }
 
 // Adjoint of one substep for every particle.  xb / Fb hold the adjoints of the
@@ -252,50 +411,77 @@ __global__ void __launch_bounds__(kThreads, 3) particle_adjoint_kernel(
     const float* __restrict__ mu, const float4* __restrict__ vel, float dt, float ndt, const float4* __restrict__ gadj,
     float* __restrict__ xb, float* __restrict__ Fb, float* __restrict__ mub, float* __restrict__ lamb,
     unsigned long long* __restrict__ vbar) {
+  extern __shared__ __align__(16) unsigned tile[];
+  __shared__ int s_box[6];
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= d.n) return;
+  const bool active = p < d.n;
+  tile_zero(tile, 6 * kTileCap);
+  if (threadIdx.x == 0) box_reset(s_box);
+  __syncthreads();
+  // The box of the nodes that G2P reads at x, where the velocity adjoints go.
   Particle<float> pp;
-  load_particle(d, x, F, p, pp);
-  Fwd<float> f;
-  float U[9], S[3], V[9];
-  VelReader vr{&d.G, vel, d.status};
-  diff::particle_forward(pp, lam[p], mu[p], d.vol_over_mass, dt, ndt, d.dx, d.inv_dx, vr, Svd{}, f, U, S, V);
-  const DenseGrid& G = d.G;
-  auto ga = [&](int g, int cx, int cy, int cz, float* out) {
-    if (!gadj || !diff::node_in_grid(G, cx, cy, cz)) {
-      out[0] = out[1] = out[2] = out[3] = 0.f;
-      return;
-    }
-    const float4 q = gadj[diff::node_index(G, g, cx, cy, cz)];
-    out[0] = q.x;
-    out[1] = q.y;
-    out[2] = q.z;
-    out[3] = q.w;
-  };
-  const float units = d.adj_scale[0];
-  auto vs = [&](int g, int cx, int cy, int cz, const float* vb) {
-    if (!diff::node_in_grid(G, cx, cy, cz)) return;
-    unsigned long long* q = vbar + 3 * diff::node_index(G, g, cx, cy, cz);
+  int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+  bool inside = false;
+  if (active) {
+    load_particle(d, x, F, p, pp);
+    diff::Stencil<float> st;
+    diff::make_stencil(pp.x, d.inv_dx, st);
+    stencil_box(st, lo, hi);
+    inside = box_in_grid(d.G, lo, hi);
+  }
+  cta_box_merge(s_box, inside, lo, hi);
+  __syncthreads();
+  const CtaBox b = cta_box(s_box);
+  if (active) {
+    Fwd<float> f;
+    float U[9], S[3], V[9];
+    VelReader vr(d, vel, pp.x);
+    diff::particle_forward(pp, lam[p], mu[p], d.vol_over_mass, dt, ndt, d.dx, d.inv_dx, vr, Svd{}, f, U, S, V);
+    const NodeReader gr(d, gadj, f.stn);
+    auto ga = [&](int g, int cx, int cy, int cz, float* out) {
+      float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (gadj) gr.get(g, cx, cy, cz, q);
+      out[0] = q.x;
+      out[1] = q.y;
+      out[2] = q.z;
+      out[3] = q.w;
+    };
+    const float units = d.adj_scale[0];
+    const int per = b.nodes >> 1;
+    auto vs = [&](int g, int cx, int cy, int cz, const float* vb) {
+      if (!inside && !diff::node_in_grid(d.G, cx, cy, cz)) return;
+      long long u[3];
+      bool ok = true;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const float u = vb[c] * units;
-      if (!(fabsf(u) < kAdjMaxUnits)) {
-        atomicOr(d.status, kErrRange);
-        continue;
+      for (int c = 0; c < 3; ++c) {
+        const float t = vb[c] * units;
+        ok &= fabsf(t) < kAdjMaxUnits;
+        u[c] = fabsf(t) < kAdjMaxUnits ? __float2ll_rn(t) : 0ll;
       }
-      atomicAdd(q + c, static_cast<unsigned long long>(__float2ll_rn(u)));
-    }
-  };
-  float xnb[3], Fnb[9], xo[3], Fo[9];
-  for (int a = 0; a < 3; ++a) xnb[a] = xb[a * d.n + p];
-  for (int k = 0; k < 9; ++k) Fnb[k] = Fb[k * d.n + p];
-  float mb = mub[p], lb = lamb[p];
-  diff::particle_adjoint(pp, f, U, S, V, d.mass, lam[p], mu[p], d.vol_over_mass, dt, ndt, d.dx, d.inv_dx, vr, ga, vs,
-                         xnb, Fnb, xo, Fo, mb, lb);
-  for (int a = 0; a < 3; ++a) xb[a * d.n + p] = xo[a];
-  for (int k = 0; k < 9; ++k) Fb[k * d.n + p] = Fo[k];
-  mub[p] = mb;
-  lamb[p] = lb;
+      if (!ok) atomicOr(d.status, kErrRange);
+      if (per && inside) {
+        unsigned* q = tile + g * per + ((cx - b.lo[0]) * b.e[1] + cy - b.lo[1]) * b.e[2] + cz - b.lo[2];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) tile_add(q + c * kTileCap, 3 * kTileCap, u[c]);
+      } else {
+        unsigned long long* q = vbar + 3 * diff::node_index(d.G, g, cx, cy, cz);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) atomicAdd(q + c, static_cast<unsigned long long>(u[c]));
+      }
+    };
+    float xnb[3], Fnb[9], xo[3], Fo[9];
+    for (int a = 0; a < 3; ++a) xnb[a] = xb[a * d.n + p];
+    for (int k = 0; k < 9; ++k) Fnb[k] = Fb[k * d.n + p];
+    float mb = mub[p], lb = lamb[p];
+    diff::particle_adjoint(pp, f, U, S, V, d.mass, lam[p], mu[p], d.vol_over_mass, dt, ndt, d.dx, d.inv_dx, vr, ga, vs,
+                           xnb, Fnb, xo, Fo, mb, lb);
+    for (int a = 0; a < 3; ++a) xb[a * d.n + p] = xo[a];
+    for (int k = 0; k < 9; ++k) Fb[k * d.n + p] = Fo[k];
+    mub[p] = mb;
+    lamb[p] = lb;
+  }
+  __syncthreads();
+  tile_flush<3>(d, b, tile, vbar);
 }
 
 // Grid-update adjoint over box b: node velocity adjoint -> (mbar, mvbar); zeroes vbar.
@@ -329,12 +515,14 @@ __global__ void grid_adjoint_kernel(Dev d, const int* __restrict__ b, const floa
 __global__ void finish_kernel(Dev d, const float* __restrict__ x, const float* __restrict__ v0,
                               const float4* __restrict__ gadj, const float* __restrict__ xb,
                               const float* __restrict__ lam, const float* __restrict__ mu,
-                              const float* __restrict__ mub, const float* __restrict__ lamb, float* __restrict__ gx0,
+                              const float* __restrict__ mub, const float* __restrict__ lamb,
+                              const uint32_t* __restrict__ perm, float* __restrict__ gx0,
                               float* __restrict__ gv0, float* __restrict__ glogE) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= d.n) return;
   const float xp[3] = {x[p], x[d.n + p], x[2 * d.n + p]};
-  const float vp[3] = {v0[3 * p], v0[3 * p + 1], v0[3 * p + 2]};
+  const uint32_t u = perm[p];
+  const float vp[3] = {v0[3 * u], v0[3 * u + 1], v0[3 * u + 2]};
   float xo[3] = {xb[p], xb[d.n + p], xb[2 * d.n + p]}, vo[3] = {0.f, 0.f, 0.f};
   const DenseGrid& G = d.G;
   diff::raster_adjoint(xp, vp, d.mass, d.inv_dx,
@@ -351,23 +539,27 @@ __global__ void finish_kernel(Dev d, const float* __restrict__ x, const float* _
                        },
                        xo, vo);
   for (int a = 0; a < 3; ++a) {
-    gx0[3 * p + a] = xo[a];
-    gv0[3 * p + a] = vo[a];
+    gx0[3 * u + a] = xo[a];
+    gv0[3 * u + a] = vo[a];
   }
-  glogE[p] = mub[p] * mu[p] + lamb[p] * lam[p];
+  glogE[u] = mub[p] * mu[p] + lamb[p] * lam[p];
 }
 
-// SoA <-> AoS for the outputs and the incoming adjoints.
-__global__ void soa_to_aos_kernel(uint32_t n, int w, const float* __restrict__ soa, float* __restrict__ aos) {
+// SoA (rollout order) <-> AoS (the caller's order) for the outputs and the incoming adjoints.
+__global__ void soa_to_aos_kernel(uint32_t n, int w, const uint32_t* __restrict__ perm, const float* __restrict__ soa,
+                                  float* __restrict__ aos) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  for (int k = 0; k < w; ++k) aos[static_cast<size_t>(w) * p + k] = soa[static_cast<size_t>(k) * n + p];
+  const size_t u = perm[p];
+  for (int k = 0; k < w; ++k) aos[static_cast<size_t>(w) * u + k] = soa[static_cast<size_t>(k) * n + p];
 }
 
-__global__ void aos_to_soa_kernel(uint32_t n, int w, const float* __restrict__ aos, float* __restrict__ soa) {
+__global__ void aos_to_soa_kernel(uint32_t n, int w, const uint32_t* __restrict__ perm, const float* __restrict__ aos,
+                                  float* __restrict__ soa) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  for (int k = 0; k < w; ++k) soa[static_cast<size_t>(k) * n + p] = aos ? aos[static_cast<size_t>(w) * p + k] : 0.f;
+  const size_t u = perm[p];
+  for (int k = 0; k < w; ++k) soa[static_cast<size_t>(k) * n + p] = aos[static_cast<size_t>(w) * u + k];
 }
 
 }  // namespace diffk
@@ -398,6 +590,8 @@ struct ckmpm_diff {
   float *xb = nullptr, *Fb = nullptr, *mub = nullptr, *lamb = nullptr;
   unsigned long long* vbar = nullptr;
   float4* gadj = nullptr;
+  // Particle order: perm[slot] = input particle; bins and their scan, each particle's bin and place in it.
+  uint32_t *perm = nullptr, *bins = nullptr, *first = nullptr, *scan = nullptr, *bin = nullptr, *rank = nullptr;
   cudaGraphExec_t gfwd = nullptr, gbwd = nullptr;
   uint64_t generation = 0;
   bool have_forward = false;
@@ -512,7 +706,11 @@ ckmpm_status ckmpm_diff_create(const ckmpm_scene_desc* desc, uint32_t n, float m
             dk_alloc(h, &h->xb, 3 * n) == cudaSuccess && dk_alloc(h, &h->Fb, 9 * n) == cudaSuccess &&
             dk_alloc(h, &h->mub, n) == cudaSuccess && dk_alloc(h, &h->lamb, n) == cudaSuccess &&
             dk_alloc(h, &h->vbar, 3 * nn) == cudaSuccess && dk_alloc(h, &h->gadj, nn) == cudaSuccess &&
-            dk_alloc(h, &h->d.adj_scale, 4) == cudaSuccess;
+            dk_alloc(h, &h->d.adj_scale, 4) == cudaSuccess && dk_alloc(h, &h->perm, n) == cudaSuccess &&
+            dk_alloc(h, &h->bin, n) == cudaSuccess && dk_alloc(h, &h->rank, n) == cudaSuccess &&
+            dk_alloc(h, &h->bins, order_bins(d.G)) == cudaSuccess &&
+            dk_alloc(h, &h->first, order_bins(d.G)) == cudaSuccess &&
+            dk_alloc(h, &h->scan, scan_tiles(order_bins(d.G))) == cudaSuccess;
   if (!ok) return bail(dfail(h, CKMPM_ERR_CUDA, "device allocation failed"));
   // Sums and velocity adjoints start (and are always left) at zero inside every box.
   if (cudaMemsetAsync(h->gsum[0], 0, 32 * nn, h->stream) != cudaSuccess ||
@@ -563,10 +761,19 @@ cudaError_t enqueue_rollout(ckmpm_diff* h) {
     return (s < h->nsteps && s % h->every == 0) ? h->ck + static_cast<size_t>(s / h->every) * 12 * n
                                                  : h->xs[s & 1];
   };
-  init_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, h->x0, h->logE, h->nu, state(0), state(0) + 3 * n, h->lam,
-                                                  h->mu);
+  // The rollout's particle order.
+  const uint32_t nbins = order_bins(d.G), ntiles = scan_tiles(nbins);
+  e = cudaMemsetAsync(h->bins, 0, sizeof(uint32_t) * nbins, st);
+  if (e != cudaSuccess) return e;
+  order_count_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, h->x0, h->bins, h->bin, h->rank);
+  ckmpm::scan_reduce_kernel<<<ntiles, ckmpm::kScanThreads, 0, st>>>(h->bins, nbins, h->scan);
+  ckmpm::scan_sums_kernel<<<1, ckmpm::kScanThreads, 0, st>>>(h->scan, ntiles);
+  ckmpm::scan_apply_kernel<<<ntiles, ckmpm::kScanThreads, 0, st>>>(h->bins, nbins, h->scan, h->first);
+  order_place_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, h->first, h->bin, h->rank, h->perm);
+  init_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, h->x0, h->logE, h->nu, h->perm, state(0), state(0) + 3 * n,
+                                                  h->lam, h->mu);
   box_init_kernel<<<(h->nsteps + 1 + 127) / 128, 128, 0, st>>>(h->box, h->nsteps + 1);
-  raster_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, state(0), h->v0, h->gsum[0], h->box);
+  raster_kernel<<<blocks_for(n), kThreads, kDepositTile, st>>>(d, state(0), h->v0, h->perm, h->gsum[0], h->box);
   for (uint32_t s = 0; s < h->nsteps; ++s) {
     const float cdt = s == 0 ? 0.f : h->dt, ndt = h->dt;
     const bool ck = (s % h->every) == 0;
@@ -576,15 +783,15 @@ cudaError_t enqueue_rollout(ckmpm_diff* h) {
     grid_kernel<<<ctas, 256, 0, st>>>(d, h->gsum[s & 1], h->box + 6 * s, cdt, vs);
     float* in = state(s);
     float* outp = state(s + 1);
-    particle_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, in, in + 3 * n, h->lam, h->mu, vs, cdt, ndt,
+    particle_kernel<<<blocks_for(n), kThreads, kDepositTile, st>>>(d, in, in + 3 * n, h->lam, h->mu, vs, cdt, ndt,
                                                         h->gsum[(s + 1) & 1], h->box + 6 * (s + 1), outp,
                                                         outp + 3 * n);
   }
   // Leave the last deposit's sums at zero (they are never read).
   grid_kernel<<<ctas, 256, 0, st>>>(d, h->gsum[h->nsteps & 1], h->box + 6 * h->nsteps, h->dt, h->vel);
   const float* fin = state(h->nsteps);
-  soa_to_aos_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 3, fin, h->xT);
-  soa_to_aos_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 9, fin + 3 * n, h->FT);
+  soa_to_aos_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 3, h->perm, fin, h->xT);
+  soa_to_aos_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 9, h->perm, fin + 3 * n, h->FT);
   return cudaGetLastError();
 }
 
@@ -596,8 +803,8 @@ cudaError_t enqueue_backward(ckmpm_diff* h) {
   const size_t nn = h->nn;
   const int ctas = grid_ctas(h);
   cudaStream_t st = h->stream;
-  aos_to_soa_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 3, h->gxT, h->xb);
-  aos_to_soa_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 9, h->gFT, h->Fb);
+  aos_to_soa_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 3, h->perm, h->gxT, h->xb);
+  aos_to_soa_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 9, h->perm, h->gFT, h->Fb);
   cudaError_t e = cudaMemsetAsync(h->d.adj_scale + 2, 0, sizeof(float), st);
   if (e != cudaSuccess) return e;
   adj_seed_max_kernel<<<ctas, 256, 0, st>>>(n, h->xb, h->Fb, h->d.adj_scale);
@@ -625,7 +832,7 @@ cudaError_t enqueue_backward(ckmpm_diff* h) {
         grid_kernel<<<ctas, 256, 0, st>>>(d, h->gsum[s & 1], h->box + 6 * s, cdt, velp(s));
       if (s + 1 < s1) {
         float* outp = statep(s + 1);
-        particle_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, in, in + 3 * n, h->lam, h->mu, velp(s), cdt, ndt,
+        particle_kernel<<<blocks_for(n), kThreads, kDepositTile, st>>>(d, in, in + 3 * n, h->lam, h->mu, velp(s), cdt, ndt,
                                                             h->gsum[(s + 1) & 1], h->box + 6 * (s + 1), outp,
                                                             outp + 3 * n);
       }
@@ -634,7 +841,7 @@ cudaError_t enqueue_backward(ckmpm_diff* h) {
     for (int s = static_cast<int>(s1) - 1; s >= static_cast<int>(s0); --s) {
       const float cdt = s == 0 ? 0.f : h->dt, ndt = h->dt;
       const float* in = statep(static_cast<uint32_t>(s));
-      particle_adjoint_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, in, in + 3 * n, h->lam, h->mu, velp(s), cdt, ndt,
+      particle_adjoint_kernel<<<blocks_for(n), kThreads, kAdjointTile, st>>>(d, in, in + 3 * n, h->lam, h->mu, velp(s), cdt, ndt,
                                                                   first ? nullptr : h->gadj, h->xb, h->Fb, h->mub,
                                                                   h->lamb, h->vbar);
       first = false;
@@ -642,7 +849,7 @@ cudaError_t enqueue_backward(ckmpm_diff* h) {
     }
   }
   finish_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, h->ck, h->v0, h->gadj, h->xb, h->lam, h->mu, h->mub, h->lamb,
-                                                    h->gx0, h->gv0, h->glogE);
+                                                    h->perm, h->gx0, h->gv0, h->glogE);
   return cudaGetLastError();
 }
 

@@ -330,8 +330,9 @@ CKD bool node_active_block(const DenseGrid& G, int cx, int cy, int cz) {
   return !(bx < 2 || bx + 2 >= G.nb[0] || bz < 2 || bz + 2 >= G.nb[2] || by + 2 >= G.nb[1]);
 }
 
-CKD int64_t node_index(const DenseGrid& G, int g, int cx, int cy, int cz) {
-  return ((static_cast<int64_t>(g) * G.n[0] + cx) * G.n[1] + cy) * G.n[2] + cz;
+// At most 2 x 256^3 nodes (64 blocks per axis): 32 bits hold every index.
+CKD int node_index(const DenseGrid& G, int g, int cx, int cy, int cz) {
+  return ((g * G.n[0] + cx) * G.n[1] + cy) * G.n[2] + cz;
 }
 
 CKD bool node_in_grid(const DenseGrid& G, int cx, int cy, int cz) {
@@ -363,28 +364,37 @@ CKD void particle_forward(const Particle<T>& p, T lambda, T mu, T vol_over_mass,
   for (int k = 0; k < 9; ++k) f.B[k] = T(0);
   CKD_UNROLL
   for (int a = 0; a < 3; ++a) f.v[a] = T(0);
+  // Separable sums, one axis at a time (z, y, x): S = sum w v and T_a = sum over the
+  // nodes with d_a = 1 of w v give B_a = (T_a - o_a S) dx.
   CKD_UNROLL
-  for (int g = 0; g < 2; ++g)
+  for (int g = 0; g < 2; ++g) {
+    const Axis<T>*ax = &f.st.a[g][0], *ay = &f.st.a[g][1], *az = &f.st.a[g][2];
+    const T wx0 = ax->w0, wx1 = T(1) - wx0, wy0 = ay->w0, wy1 = T(1) - wy0, wz0 = az->w0, wz1 = T(1) - wz0;
+    T Sy[2][3], Ty[2][3], Tz[2][3];
     CKD_UNROLL
-    for (int n = 0; n < 8; ++n) {
-      const T w = node_weight(f.st, g, n, inv_dx, static_cast<T*>(nullptr));
-      int c[3];
-      T r[3];
+    for (int i = 0; i < 2; ++i) {
+      T a0[3], a1[3], b0[3], b1[3];
+      vel(g, ax->base + i, ay->base, az->base, a0);
+      vel(g, ax->base + i, ay->base, az->base + 1, a1);
+      vel(g, ax->base + i, ay->base + 1, az->base, b0);
+      vel(g, ax->base + i, ay->base + 1, az->base + 1, b1);
       CKD_UNROLL
-      for (int a = 0; a < 3; ++a) {
-        const int d = (n >> (2 - a)) & 1;
-        c[a] = f.st.a[g][a].base + d;
-        r[a] = (static_cast<T>(d) - f.st.a[g][a].o) * dx;
-      }
-      T vi[3];
-      vel(g, c[0], c[1], c[2], vi);
-      CKD_UNROLL
-      for (int i = 0; i < 3; ++i) {
-        f.v[i] += w * vi[i];
-        CKD_UNROLL
-        for (int a = 0; a < 3; ++a) f.B[i * 3 + a] += w * vi[i] * r[a];
+      for (int r = 0; r < 3; ++r) {
+        const T ta = wz1 * a1[r], tb = wz1 * b1[r];
+        Ty[i][r] = wy1 * (wz0 * b0[r] + tb);
+        Sy[i][r] = wy0 * (wz0 * a0[r] + ta) + Ty[i][r];
+        Tz[i][r] = wy0 * ta + wy1 * tb;
       }
     }
+    CKD_UNROLL
+    for (int r = 0; r < 3; ++r) {
+      const T Tx = wx1 * Sy[1][r], Sr = wx0 * Sy[0][r] + Tx;
+      f.v[r] += Sr;
+      f.B[r * 3] += (Tx - ax->o * Sr) * dx;
+      f.B[r * 3 + 1] += (wx0 * Ty[0][r] + wx1 * Ty[1][r] - ay->o * Sr) * dx;
+      f.B[r * 3 + 2] += (wx0 * Tz[0][r] + wx1 * Tz[1][r] - az->o * Sr) * dx;
+    }
+  }
   CKD_UNROLL
   for (int i = 0; i < 3; ++i) f.v[i] *= T(0.5);
   T D6[6], Di6[6];
