@@ -426,11 +426,7 @@ def run_diff(args, rank, world, local_rank):
         "train_step_particle_substeps_per_s": n * nsteps / (ms / 1e3),
         "gradcheck": gradcheck, "loss": float(loss.item()), "clocks": clocks, "roofline": roofline,
         "cpu_baseline": cpu,
-        # per training step: forward (5 ordering kernels, init, box reset, raster, grid + particle per
-        # substep, last grid update, 2 layout copies: 2 nsteps + 11), backward (2 layout copies, seed max, scale; grid and
-        # particle kernels of the recomputed substeps, 2 (len - 1) per segment; grid and particle
-        # adjoint per substep; finish: 4 nsteps - 2 nseg + 5)
-        "gpu_launches": steps * (6 * nsteps - 2 * (-(-nsteps // d["checkpoint_every"])) + 16),
+        "gpu_launches": steps * rollout_launches(nsteps, d["checkpoint_every"]),
         "e2e": {"value": n * nsteps / (e2e_ms / 1e3), "unit": METRIC, "h2d_bytes_per_step": n * (12 + 12 + 4),
                 "d2h_bytes_per_step": 4 + n * (12 + 4),
                 "includes": "per step: x0, v0, log E uploaded from pinned host memory, forward + adjoint rollout "
@@ -438,6 +434,15 @@ def run_diff(args, rank, world, local_rank):
     }
     sim.close()
     return line
+
+
+def rollout_launches(nsteps: int, every: int) -> int:
+    """Kernel launches of one forward + adjoint rollout.  Forward: 5 ordering kernels, init, box reset, raster, one
+    per substep, 2 that zero the last sums, 2 layout copies.  Backward: 2 layout copies, seed maximum and scale, the
+    recomputed substeps of each segment with its last grid update and sums, one adjoint per substep, finish, zeroing."""
+    segments = [min(every, nsteps - s) for s in range(0, nsteps, every)]
+    recompute = sum((k - 1) + (k > 1) + (k > 2) for k in segments)
+    return (12 + nsteps) + (4 + recompute + nsteps + 2 + (nsteps > 1))
 
 
 def substep_launches(cfg, n_models: int, n_scenes: int = 1) -> int:

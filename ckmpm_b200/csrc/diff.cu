@@ -152,24 +152,6 @@ __device__ __forceinline__ void tile_add(unsigned* lo_word, int plane, long long
   atomicAdd(lo_word + plane, static_cast<unsigned>(v >> 32) + (old + lo < lo ? 1u : 0u));
 }
 
-// Adds the tile's touched words to the grid arrays (kCh channels per node).
-template <int kCh>
-__device__ __forceinline__ void tile_flush(const Dev& d, const CtaBox& b, const unsigned* tile,
-                                           unsigned long long* __restrict__ out) {
-  const int per = b.nodes >> 1, plane = kCh * kTileCap;
-  for (int i = threadIdx.x; i < b.nodes; i += kThreads) {
-    const int g = i >= per ? 1 : 0, j = i - g * per;
-    const int z = j % b.e[2], xy = j / b.e[2], y = xy % b.e[1], x = xy / b.e[1];
-    unsigned long long* q = out + kCh * diff::node_index(d.G, g, b.lo[0] + x, b.lo[1] + y, b.lo[2] + z);
-#pragma unroll
-    for (int c = 0; c < kCh; ++c) {
-      const unsigned long long v = static_cast<unsigned long long>(tile[c * kTileCap + i]) |
-                                   (static_cast<unsigned long long>(tile[c * kTileCap + i + plane]) << 32);
-      if (v) atomicAdd(q + c, v);
-    }
-  }
-}
-
 // First and last node of a particle's stencils over both grids.  A position far
 // outside (or infinite) saturates the base cells, so `hi` may wrap: box_in_grid
 // bounds both ends.
@@ -186,6 +168,86 @@ __device__ __forceinline__ bool box_in_grid(const DenseGrid& G, const int* lo, c
 #pragma unroll
   for (int a = 0; a < 3; ++a) in &= lo[a] >= 0 && lo[a] < G.n[a] && hi[a] >= lo[a] && hi[a] < G.n[a];
   return in;
+}
+
+// Node (g, x, y, z) of entry i of a CTA box.
+__device__ __forceinline__ int box_node(const Dev& d, const CtaBox& b, int i, int& cx, int& cy, int& cz) {
+  const int per = b.nodes >> 1, g = i >= per ? 1 : 0, j = i - g * per;
+  const int z = j % b.e[2], xy = j / b.e[2], y = xy % b.e[1], x = xy / b.e[1];
+  cx = b.lo[0] + x;
+  cy = b.lo[1] + y;
+  cz = b.lo[2] + z;
+  return diff::node_index(d.G, g, cx, cy, cz);
+}
+
+// Entry of a node in a CTA box's tile.
+__device__ __forceinline__ int box_entry(const CtaBox& b, int g, int cx, int cy, int cz) {
+  return g * (b.nodes >> 1) + ((cx - b.lo[0]) * b.e[1] + cy - b.lo[1]) * b.e[2] + cz - b.lo[2];
+}
+
+// Adds the tile's touched words to the grid arrays (kCh channels per node).
+template <int kCh>
+__device__ __forceinline__ void tile_flush(const Dev& d, const CtaBox& b, const unsigned* tile,
+                                           unsigned long long* __restrict__ out) {
+  const int plane = kCh * kTileCap;
+  for (int i = threadIdx.x; i < b.nodes; i += kThreads) {
+    int cx, cy, cz;
+    unsigned long long* q = out + kCh * static_cast<size_t>(box_node(d, b, i, cx, cy, cz));
+#pragma unroll
+    for (int c = 0; c < kCh; ++c) {
+      const unsigned long long v = static_cast<unsigned long long>(tile[c * kTileCap + i]) |
+                                   (static_cast<unsigned long long>(tile[c * kTileCap + i + plane]) << 32);
+      if (v) atomicAdd(q + c, v);
+    }
+  }
+}
+
+// Grid update of one node from its sums: velocity and mass.
+__device__ __forceinline__ float4 node_from_sums(const Dev& d, const unsigned long long* __restrict__ gsum, int id, int cx,
+                                                 int cy, int cz, float dt) {
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(gsum + 4 * static_cast<size_t>(id));
+  const ulonglong2 s01 = q[0], s23 = q[1];
+  const float m = __ll2float_rn(static_cast<long long>(s01.x)) * d.unit;
+  const float mv[3] = {__ll2float_rn(static_cast<long long>(s01.y)) * d.unit,
+                       __ll2float_rn(static_cast<long long>(s23.x)) * d.unit,
+                       __ll2float_rn(static_cast<long long>(s23.y)) * d.unit};
+  float v[3];
+  diff::node_update(d.G, cx, cy, cz, m, mv, dt, v);
+  return make_float4(v[0], v[1], v[2], m);
+}
+
+// Grid-update adjoint of one node: its velocity adjoint -> (mbar, mvbar).
+__device__ __forceinline__ float4 node_adjoint(const Dev& d, const unsigned long long* __restrict__ vbar, const float4& v4,
+                                               int id, int cx, int cy, int cz, float dt) {
+  const unsigned long long* vb = vbar + 3 * static_cast<size_t>(id);
+  const float inv_units = d.adj_scale[1];
+  const float vbv[3] = {__ll2float_rn(static_cast<long long>(vb[0])) * inv_units,
+                        __ll2float_rn(static_cast<long long>(vb[1])) * inv_units,
+                        __ll2float_rn(static_cast<long long>(vb[2])) * inv_units};
+  const float v[3] = {v4.x, v4.y, v4.z};
+  float out[4];
+  diff::node_update_adjoint(d.G, cx, cy, cz, v4.w, v, dt, vbv, out);
+  return make_float4(out[0], out[1], out[2], out[3]);
+}
+
+// Zeroes kCh sums per node over a substep's node box, shared out over the grid.
+template <int kCh>
+__device__ __forceinline__ void zero_box(const Dev& d, const int* __restrict__ b, unsigned long long* __restrict__ sums) {
+  if (!sums || b[0] > b[3]) return;
+  const int ex = b[3] - b[0] + 1, ey = b[4] - b[1] + 1, ez = b[5] - b[2] + 1;
+  const int total = 2 * ex * ey * ez;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const int z = t % ez, xy = t / ez, y = xy % ey, gx = xy / ey, x = gx % ex, g = gx / ex;
+    unsigned long long* q =
+        sums + kCh * static_cast<size_t>(diff::node_index(d.G, g, b[0] + x, b[1] + y, b[2] + z));
+#pragma unroll
+    for (int c = 0; c < kCh; ++c) q[c] = 0ull;
+  }
+}
+
+template <int kCh>
+__global__ void zero_box_kernel(Dev d, const int* __restrict__ b, unsigned long long* __restrict__ sums) {
+  zero_box<kCh>(d, b, sums);
 }
 
 // Deposits of the CTA's particles (per unit mass) into gsum and the merge of their
@@ -216,7 +278,6 @@ __device__ __forceinline__ void cta_deposit(const Dev& d, bool active, const Fwd
     atomicMax(box + 3 + threadIdx.x, s_box[3 + threadIdx.x]);
   }
   if (active) {
-    const int per = b.nodes >> 1;
     diff::particle_deposit(f, d.dx, d.inv_dx, [&](int g, int cx, int cy, int cz, float w, const float* wv) {
       if (!inside && !diff::node_in_grid(d.G, cx, cy, cz)) return;
       if (!(fabsf(wv[0]) < kMaxValue && fabsf(wv[1]) < kMaxValue && fabsf(wv[2]) < kMaxValue)) {
@@ -225,8 +286,8 @@ __device__ __forceinline__ void cta_deposit(const Dev& d, bool active, const Fwd
       }
       const long long v[4] = {__float2ll_rn(w * kScale), __float2ll_rn(wv[0] * kScale), __float2ll_rn(wv[1] * kScale),
                               __float2ll_rn(wv[2] * kScale)};
-      if (per) {
-        unsigned* q = tile + g * per + ((cx - b.lo[0]) * b.e[1] + cy - b.lo[1]) * b.e[2] + cz - b.lo[2];
+      if (b.nodes) {
+        unsigned* q = tile + box_entry(b, g, cx, cy, cz);
 #pragma unroll
         for (int c = 0; c < 4; ++c) tile_add(q + c * kTileCap, 4 * kTileCap, v[c]);
       } else {
@@ -240,8 +301,11 @@ __device__ __forceinline__ void cta_deposit(const Dev& d, bool active, const Fwd
   tile_flush<4>(d, b, tile, gsum);
 }
 
-constexpr size_t kDepositTile = sizeof(unsigned) * 2 * 4 * kTileCap;  // 32 KB
-constexpr size_t kAdjointTile = sizeof(unsigned) * 2 * 3 * kTileCap;  // 24 KB
+constexpr size_t kNodeTile = sizeof(float4) * kTileCap;                // 16 KB
+constexpr size_t kDepositTile = sizeof(unsigned) * 2 * 4 * kTileCap;   // 32 KB
+constexpr size_t kAdjointTile = sizeof(unsigned) * 2 * 3 * kTileCap;   // 24 KB
+constexpr size_t kForwardSmem = kDepositTile + kNodeTile;
+constexpr size_t kAdjointSmem = kAdjointTile + kNodeTile;
 
 // AoS inputs -> SoA state; lambda / mu from log E; F = I.
 __global__ void init_kernel(Dev d, const float* __restrict__ x0, const float* __restrict__ logE, float nu,
@@ -287,7 +351,8 @@ __global__ void box_init_kernel(int* boxes, uint32_t count) {
   if (i < count) box_reset(boxes + 6 * i);
 }
 
-// Grid update over box b: int64 sums -> float4 (v, m); zero the sums read.
+// Grid update over box b: int64 sums -> float4 (v, m); zero the sums read.  For the
+// last state of a recomputed segment, which no forward substep reads.
 __global__ void grid_kernel(Dev d, unsigned long long* __restrict__ gsum, const int* __restrict__ b, float dt,
                             float4* __restrict__ vel) {
   if (b[0] > b[3]) return;
@@ -299,49 +364,41 @@ __global__ void grid_kernel(Dev d, unsigned long long* __restrict__ gsum, const 
     const int x = static_cast<int>((t / (static_cast<int64_t>(ez) * ey)) % ex);
     const int g = static_cast<int>(t / (static_cast<int64_t>(ez) * ey * ex));
     const int cx = b[0] + x, cy = b[1] + y, cz = b[2] + z;
-    const int64_t id = diff::node_index(d.G, g, cx, cy, cz);
-    ulonglong2* q = reinterpret_cast<ulonglong2*>(gsum + 4 * id);
-    const ulonglong2 s01 = q[0], s23 = q[1];
+    const int id = diff::node_index(d.G, g, cx, cy, cz);
+    vel[id] = node_from_sums(d, gsum, id, cx, cy, cz, dt);
+    ulonglong2* q = reinterpret_cast<ulonglong2*>(gsum + 4 * static_cast<size_t>(id));
     q[0] = make_ulonglong2(0ull, 0ull);
     q[1] = make_ulonglong2(0ull, 0ull);
-    const float m = __ll2float_rn(static_cast<long long>(s01.x)) * d.unit;
-    const float mv[3] = {__ll2float_rn(static_cast<long long>(s01.y)) * d.unit,
-                         __ll2float_rn(static_cast<long long>(s23.x)) * d.unit,
-                         __ll2float_rn(static_cast<long long>(s23.y)) * d.unit};
-    float v[3];
-    diff::node_update(d.G, cx, cy, cz, m, mv, dt, v);
-    vel[id] = make_float4(v[0], v[1], v[2], m);
   }
 }
 
-// Reads a float4 per node of a particle's 16; the grid's bounds are checked once
-// for the whole stencil, per node only where it leaves the grid.
-struct NodeReader {
+// Node velocities of G2P: from the CTA's tile; where there is none, from the
+// velocities of the substep or (sums given) from the node sums themselves, and then
+// written to the tape as well.
+struct VelReader {
   const Dev* d;
-  const float4* nodes;
-  bool inside;
-  __device__ NodeReader(const Dev& dev, const float4* q, const diff::Stencil<float>& st) : d(&dev), nodes(q) {
-    int lo[3], hi[3];
-    stencil_box(st, lo, hi);
-    inside = box_in_grid(dev.G, lo, hi);
-  }
-  __device__ bool get(int g, int cx, int cy, int cz, float4& q) const {
-    if (!inside && !diff::node_in_grid(d->G, cx, cy, cz)) return false;
-    q = nodes[diff::node_index(d->G, g, cx, cy, cz)];
-    return true;
-  }
-};
-
-struct VelReader : NodeReader {
-  __device__ VelReader(const Dev& dev, const float4* vel, const float* x) : NodeReader(dev, vel, stencil_at(dev, x)) {}
-  static __device__ diff::Stencil<float> stencil_at(const Dev& dev, const float* x) {
-    diff::Stencil<float> st;
-    diff::make_stencil(x, dev.inv_dx, st);
-    return st;
-  }
+  const CtaBox* b;
+  const float4* tile;
+  float4* vel;
+  const unsigned long long* sums;
+  float dt;
+  bool tiled, inside;  // the particle's stencil lies in the tile / in the grid
   __device__ void operator()(int g, int cx, int cy, int cz, float* v) const {
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (!get(g, cx, cy, cz, q)) atomicOr(d->status, kErrOutside);
+    float4 q;
+    if (tiled) {
+      q = tile[box_entry(*b, g, cx, cy, cz)];
+    } else if (!inside && !diff::node_in_grid(d->G, cx, cy, cz)) {
+      atomicOr(d->status, kErrOutside);
+      q = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+      const int id = diff::node_index(d->G, g, cx, cy, cz);
+      if (sums) {
+        q = node_from_sums(*d, sums, id, cx, cy, cz, dt);
+        vel[id] = q;
+      } else {
+        q = vel[id];
+      }
+    }
     v[0] = q.x;
     v[1] = q.y;
     v[2] = q.z;
@@ -358,30 +415,60 @@ __device__ __forceinline__ void load_particle(const Dev& d, const float* x, cons
   for (int k = 0; k < 9; ++k) pp.F[k] = F[k * d.n + p];
 }
 
-// Forward substep of every particle: G2P at x, x and F update, stress,
-// deposit at x' into gsum_next; new state to (xo, Fo).
-__global__ void __launch_bounds__(kThreads) particle_kernel(Dev d, const float* __restrict__ x,
-                                                            const float* __restrict__ F, const float* __restrict__ lam,
-                                                            const float* __restrict__ mu, const float4* __restrict__ vel,
-                                                            float dt, float ndt, unsigned long long* __restrict__ gsum,
-                                                            int* bnext, float* __restrict__ xo, float* __restrict__ Fo) {
+// Forward substep of every particle: grid update and G2P at x, x and F update,
+// stress, deposit at x' into gsum_out; new state to (xo, Fo).  The grid update runs
+// as the CTA's node tile is filled, from gsum_in (the velocities then go to the
+// tape `vel` too), or, gsum_in null, the velocities are read from `vel`.  The sums are
+// triple-buffered: gsum_zero, which the previous substep read (box bzero), is zeroed
+// here for the next substep's deposits.
+__global__ void __launch_bounds__(kThreads) particle_kernel(
+    Dev d, const float* __restrict__ x, const float* __restrict__ F, const float* __restrict__ lam,
+    const float* __restrict__ mu, float4* __restrict__ vel, const unsigned long long* __restrict__ gsum_in, float dt,
+    float ndt, unsigned long long* __restrict__ gsum_out, int* bnext, unsigned long long* __restrict__ gsum_zero,
+    const int* __restrict__ bzero, float* __restrict__ xo, float* __restrict__ Fo) {
   extern __shared__ __align__(16) unsigned tile[];
-  __shared__ int s_box[6];
+  float4* vtile = reinterpret_cast<float4*>(tile + 8 * kTileCap);
+  __shared__ int s_box[2][6];
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  tile_zero(tile, 8 * kTileCap);
-  if (threadIdx.x == 0) box_reset(s_box);
-  Fwd<float> f;
-  if (p < d.n) {
-    Particle<float> pp;
+  const bool active = p < d.n;
+  if (threadIdx.x < 2) box_reset(s_box[threadIdx.x]);
+  __syncthreads();
+  Particle<float> pp;
+  int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+  bool inside = false;
+  if (active) {
     load_particle(d, x, F, p, pp);
+    diff::Stencil<float> st;
+    diff::make_stencil(pp.x, d.inv_dx, st);
+    stencil_box(st, lo, hi);
+    inside = box_in_grid(d.G, lo, hi);
+  }
+  cta_box_merge(s_box[0], inside, lo, hi);
+  zero_box<4>(d, bzero, gsum_zero);
+  tile_zero(tile, 8 * kTileCap);
+  __syncthreads();
+  const CtaBox b = cta_box(s_box[0]);
+  for (int i = threadIdx.x; i < b.nodes; i += kThreads) {
+    int cx, cy, cz;
+    const int id = box_node(d, b, i, cx, cy, cz);
+    if (gsum_in) {
+      const float4 q = node_from_sums(d, gsum_in, id, cx, cy, cz, dt);
+      vtile[i] = q;
+      vel[id] = q;  // every CTA that reads the node writes the same value
+    } else {
+      vtile[i] = vel[id];
+    }
+  }
+  __syncthreads();
+  Fwd<float> f;
+  if (active) {
     float U[9], S[3], V[9];
-    VelReader vr(d, vel, pp.x);
+    const VelReader vr{&d, &b, vtile, vel, gsum_in, dt, inside && b.nodes, inside};
     diff::particle_forward(pp, lam[p], mu[p], d.vol_over_mass, dt, ndt, d.dx, d.inv_dx, vr, Svd{}, f, U, S, V);
     for (int a = 0; a < 3; ++a) xo[a * d.n + p] = f.xn[a];
     for (int k = 0; k < 9; ++k) Fo[k * d.n + p] = f.Fn[k];
   }
-  __syncthreads();
-  cta_deposit(d, p < d.n, f, tile, s_box, gsum, bnext);
+  cta_deposit(d, active, f, tile, s_box[1], gsum_out, bnext);
 }
 
 // Adjoint of one substep for every particle.  xb / Fb hold the adjoints of the
@@ -406,48 +493,78 @@ __global__ void adj_scale_kernel(float* adj_scale) {
   }
 }
 
+// The adjoint of the deposit at x' (xn, the state after the substep; bit for bit what
+// the forward deposited at) is gathered from a CTA tile that applies the grid-update
+// adjoint of the next substep as it is filled, from vbar_in and that substep's
+// velocities vel_next; both null for the last substep, whose deposit nothing reads.
+// The velocity adjoints go to vbar_out through a tile of exact sums.  vbar is
+// triple-buffered like the forward's sums.
 __global__ void __launch_bounds__(kThreads, 3) particle_adjoint_kernel(
-    Dev d, const float* __restrict__ x, const float* __restrict__ F, const float* __restrict__ lam,
-    const float* __restrict__ mu, const float4* __restrict__ vel, float dt, float ndt, const float4* __restrict__ gadj,
+    Dev d, const float* __restrict__ x, const float* __restrict__ F, const float* __restrict__ xn,
+    const float* __restrict__ lam, const float* __restrict__ mu, float4* __restrict__ vel,
+    const float4* __restrict__ vel_next, float dt, float ndt, const unsigned long long* __restrict__ vbar_in,
     float* __restrict__ xb, float* __restrict__ Fb, float* __restrict__ mub, float* __restrict__ lamb,
-    unsigned long long* __restrict__ vbar) {
+    unsigned long long* __restrict__ vbar_out, unsigned long long* __restrict__ vbar_zero, const int* __restrict__ bzero) {
   extern __shared__ __align__(16) unsigned tile[];
-  __shared__ int s_box[6];
+  float4* gtile = reinterpret_cast<float4*>(tile + 6 * kTileCap);
+  __shared__ int s_box[2][6];
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = p < d.n;
-  tile_zero(tile, 6 * kTileCap);
-  if (threadIdx.x == 0) box_reset(s_box);
+  if (threadIdx.x < 2) box_reset(s_box[threadIdx.x]);
   __syncthreads();
-  // The box of the nodes that G2P reads at x, where the velocity adjoints go.
+  // The boxes of the nodes that G2P reads at x, where the velocity adjoints go, and of
+  // the deposit's at x'.
   Particle<float> pp;
-  int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-  bool inside = false;
+  float xd[3] = {0.f, 0.f, 0.f};
+  int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0}, lo2[3] = {0, 0, 0}, hi2[3] = {0, 0, 0};
+  bool inside = false, inside2 = false;
   if (active) {
     load_particle(d, x, F, p, pp);
+    for (int a = 0; a < 3; ++a) xd[a] = xn[a * d.n + p];
     diff::Stencil<float> st;
     diff::make_stencil(pp.x, d.inv_dx, st);
     stencil_box(st, lo, hi);
     inside = box_in_grid(d.G, lo, hi);
+    diff::make_stencil(xd, d.inv_dx, st);
+    stencil_box(st, lo2, hi2);
+    inside2 = box_in_grid(d.G, lo2, hi2);
   }
-  cta_box_merge(s_box, inside, lo, hi);
+  cta_box_merge(s_box[0], inside, lo, hi);
+  cta_box_merge(s_box[1], inside2, lo2, hi2);
+  zero_box<3>(d, bzero, vbar_zero);
+  tile_zero(tile, 6 * kTileCap);
   __syncthreads();
-  const CtaBox b = cta_box(s_box);
+  const CtaBox b = cta_box(s_box[0]), b2 = cta_box(s_box[1]);
+  if (vbar_in) {
+    for (int i = threadIdx.x; i < b2.nodes; i += kThreads) {
+      int cx, cy, cz;
+      const int id = box_node(d, b2, i, cx, cy, cz);
+      gtile[i] = node_adjoint(d, vbar_in, vel_next[id], id, cx, cy, cz, ndt);
+    }
+  }
+  __syncthreads();
   if (active) {
     Fwd<float> f;
     float U[9], S[3], V[9];
-    VelReader vr(d, vel, pp.x);
-    diff::particle_forward(pp, lam[p], mu[p], d.vol_over_mass, dt, ndt, d.dx, d.inv_dx, vr, Svd{}, f, U, S, V);
-    const NodeReader gr(d, gadj, f.stn);
+    const VelReader vr{&d, &b, nullptr, vel, nullptr, dt, false, inside};
+    diff::particle_forward(pp, lam[p], mu[p], d.vol_over_mass, dt, ndt, d.dx, d.inv_dx, vr, Svd{}, f, U, S, V, xd);
+    const bool tiled2 = inside2 && b2.nodes;
     auto ga = [&](int g, int cx, int cy, int cz, float* out) {
       float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (gadj) gr.get(g, cx, cy, cz, q);
+      if (vbar_in) {
+        if (tiled2) {
+          q = gtile[box_entry(b2, g, cx, cy, cz)];
+        } else if (inside2 || diff::node_in_grid(d.G, cx, cy, cz)) {
+          const int id = diff::node_index(d.G, g, cx, cy, cz);
+          q = node_adjoint(d, vbar_in, vel_next[id], id, cx, cy, cz, ndt);
+        }
+      }
       out[0] = q.x;
       out[1] = q.y;
       out[2] = q.z;
       out[3] = q.w;
     };
     const float units = d.adj_scale[0];
-    const int per = b.nodes >> 1;
     auto vs = [&](int g, int cx, int cy, int cz, const float* vb) {
       if (!inside && !diff::node_in_grid(d.G, cx, cy, cz)) return;
       long long u[3];
@@ -459,12 +576,12 @@ __global__ void __launch_bounds__(kThreads, 3) particle_adjoint_kernel(
         u[c] = fabsf(t) < kAdjMaxUnits ? __float2ll_rn(t) : 0ll;
       }
       if (!ok) atomicOr(d.status, kErrRange);
-      if (per && inside) {
-        unsigned* q = tile + g * per + ((cx - b.lo[0]) * b.e[1] + cy - b.lo[1]) * b.e[2] + cz - b.lo[2];
+      if (inside && b.nodes) {
+        unsigned* q = tile + box_entry(b, g, cx, cy, cz);
 #pragma unroll
         for (int c = 0; c < 3; ++c) tile_add(q + c * kTileCap, 3 * kTileCap, u[c]);
       } else {
-        unsigned long long* q = vbar + 3 * diff::node_index(d.G, g, cx, cy, cz);
+        unsigned long long* q = vbar_out + 3 * static_cast<size_t>(diff::node_index(d.G, g, cx, cy, cz));
 #pragma unroll
         for (int c = 0; c < 3; ++c) atomicAdd(q + c, static_cast<unsigned long long>(u[c]));
       }
@@ -481,39 +598,13 @@ __global__ void __launch_bounds__(kThreads, 3) particle_adjoint_kernel(
     lamb[p] = lb;
   }
   __syncthreads();
-  tile_flush<3>(d, b, tile, vbar);
-}
-
-// Grid-update adjoint over box b: node velocity adjoint -> (mbar, mvbar); zeroes vbar.
-__global__ void grid_adjoint_kernel(Dev d, const int* __restrict__ b, const float4* __restrict__ vel, float dt,
-                                    unsigned long long* __restrict__ vbar, float4* __restrict__ gadj) {
-  if (b[0] > b[3]) return;
-  const int ex = b[3] - b[0] + 1, ey = b[4] - b[1] + 1, ez = b[5] - b[2] + 1;
-  const int64_t total = 2ll * ex * ey * ez;
-  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int z = static_cast<int>(t % ez), y = static_cast<int>((t / ez) % ey);
-    const int x = static_cast<int>((t / (static_cast<int64_t>(ez) * ey)) % ex);
-    const int g = static_cast<int>(t / (static_cast<int64_t>(ez) * ey * ex));
-    const int cx = b[0] + x, cy = b[1] + y, cz = b[2] + z;
-    const int64_t id = diff::node_index(d.G, g, cx, cy, cz);
-    unsigned long long* vb = vbar + 3 * id;
-    const float inv_units = d.adj_scale[1];
-    const float vbv[3] = {__ll2float_rn(static_cast<long long>(vb[0])) * inv_units,
-                          __ll2float_rn(static_cast<long long>(vb[1])) * inv_units,
-                          __ll2float_rn(static_cast<long long>(vb[2])) * inv_units};
-    vb[0] = vb[1] = vb[2] = 0ull;
-    const float4 q = vel[id];
-    const float v[3] = {q.x, q.y, q.z};
-    float out[4];
-    diff::node_update_adjoint(d.G, cx, cy, cz, q.w, v, dt, vbv, out);
-    gadj[id] = make_float4(out[0], out[1], out[2], out[3]);
-  }
+  tile_flush<3>(d, b, tile, vbar_out);
 }
 
 // Rasterisation adjoint and the outputs: gx0 (AoS), gv0 (AoS), glogE.
 __global__ void finish_kernel(Dev d, const float* __restrict__ x, const float* __restrict__ v0,
-                              const float4* __restrict__ gadj, const float* __restrict__ xb,
+                              const unsigned long long* __restrict__ vbar, const float4* __restrict__ vel,
+                              const float* __restrict__ xb,
                               const float* __restrict__ lam, const float* __restrict__ mu,
                               const float* __restrict__ mub, const float* __restrict__ lamb,
                               const uint32_t* __restrict__ perm, float* __restrict__ gx0,
@@ -524,14 +615,13 @@ __global__ void finish_kernel(Dev d, const float* __restrict__ x, const float* _
   const uint32_t u = perm[p];
   const float vp[3] = {v0[3 * u], v0[3 * u + 1], v0[3 * u + 2]};
   float xo[3] = {xb[p], xb[d.n + p], xb[2 * d.n + p]}, vo[3] = {0.f, 0.f, 0.f};
-  const DenseGrid& G = d.G;
   diff::raster_adjoint(xp, vp, d.mass, d.inv_dx,
                        [&](int g, int cx, int cy, int cz, float* out) {
-                         if (!diff::node_in_grid(G, cx, cy, cz)) {
-                           out[0] = out[1] = out[2] = out[3] = 0.f;
-                           return;
+                         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                         if (diff::node_in_grid(d.G, cx, cy, cz)) {
+                           const int id = diff::node_index(d.G, g, cx, cy, cz);
+                           q = node_adjoint(d, vbar, vel[id], id, cx, cy, cz, 0.f);
                          }
-                         const float4 q = gadj[diff::node_index(G, g, cx, cy, cz)];
                          out[0] = q.x;
                          out[1] = q.y;
                          out[2] = q.z;
@@ -585,11 +675,10 @@ struct ckmpm_diff {
   float* tape = nullptr;              // max(every - 1, 1) x 12n: substeps s0 + 1 .. s1 - 1 of a segment
   float4* tapevel = nullptr;          // every x nn
   float4* vel = nullptr;              // scratch node velocities (forward pass)
-  unsigned long long* gsum[2] = {nullptr, nullptr};
+  unsigned long long* gsum[3] = {nullptr, nullptr, nullptr};  // substep s reads [s % 3], deposits into [(s + 1) % 3]
   int* box = nullptr;                 // (nsteps + 1) x 6
   float *xb = nullptr, *Fb = nullptr, *mub = nullptr, *lamb = nullptr;
-  unsigned long long* vbar = nullptr;
-  float4* gadj = nullptr;
+  unsigned long long* vbar[3] = {nullptr, nullptr, nullptr};  // substep s's velocity adjoints: [s % 3]
   // Particle order: perm[slot] = input particle; bins and their scan, each particle's bin and place in it.
   uint32_t *perm = nullptr, *bins = nullptr, *first = nullptr, *scan = nullptr, *bin = nullptr, *rank = nullptr;
   cudaGraphExec_t gfwd = nullptr, gbwd = nullptr;
@@ -701,11 +790,12 @@ ckmpm_status ckmpm_diff_create(const ckmpm_scene_desc* desc, uint32_t n, float m
             dk_alloc(h, &h->tape, static_cast<size_t>(std::max<uint32_t>(h->every, 2) - 1) * 12 * n) == cudaSuccess &&
             dk_alloc(h, &h->tapevel, static_cast<size_t>(h->every) * nn) == cudaSuccess &&
             dk_alloc(h, &h->vel, nn) == cudaSuccess && dk_alloc(h, &h->gsum[0], 4 * nn) == cudaSuccess &&
-            dk_alloc(h, &h->gsum[1], 4 * nn) == cudaSuccess &&
+            dk_alloc(h, &h->gsum[1], 4 * nn) == cudaSuccess && dk_alloc(h, &h->gsum[2], 4 * nn) == cudaSuccess &&
             dk_alloc(h, &h->box, 6 * static_cast<size_t>(nsteps + 1)) == cudaSuccess &&
             dk_alloc(h, &h->xb, 3 * n) == cudaSuccess && dk_alloc(h, &h->Fb, 9 * n) == cudaSuccess &&
             dk_alloc(h, &h->mub, n) == cudaSuccess && dk_alloc(h, &h->lamb, n) == cudaSuccess &&
-            dk_alloc(h, &h->vbar, 3 * nn) == cudaSuccess && dk_alloc(h, &h->gadj, nn) == cudaSuccess &&
+            dk_alloc(h, &h->vbar[0], 3 * nn) == cudaSuccess && dk_alloc(h, &h->vbar[1], 3 * nn) == cudaSuccess &&
+            dk_alloc(h, &h->vbar[2], 3 * nn) == cudaSuccess &&
             dk_alloc(h, &h->d.adj_scale, 4) == cudaSuccess && dk_alloc(h, &h->perm, n) == cudaSuccess &&
             dk_alloc(h, &h->bin, n) == cudaSuccess && dk_alloc(h, &h->rank, n) == cudaSuccess &&
             dk_alloc(h, &h->bins, order_bins(d.G)) == cudaSuccess &&
@@ -713,10 +803,16 @@ ckmpm_status ckmpm_diff_create(const ckmpm_scene_desc* desc, uint32_t n, float m
             dk_alloc(h, &h->scan, scan_tiles(order_bins(d.G))) == cudaSuccess;
   if (!ok) return bail(dfail(h, CKMPM_ERR_CUDA, "device allocation failed"));
   // Sums and velocity adjoints start (and are always left) at zero inside every box.
-  if (cudaMemsetAsync(h->gsum[0], 0, 32 * nn, h->stream) != cudaSuccess ||
-      cudaMemsetAsync(h->gsum[1], 0, 32 * nn, h->stream) != cudaSuccess ||
-      cudaMemsetAsync(h->vbar, 0, 24 * nn, h->stream) != cudaSuccess ||
-      cudaMemsetAsync(h->d.adj_scale, 0, 4 * sizeof(float), h->stream) != cudaSuccess ||
+  if (cudaFuncSetAttribute(reinterpret_cast<const void*>(particle_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(kForwardSmem)) != cudaSuccess ||
+      cudaFuncSetAttribute(reinterpret_cast<const void*>(particle_adjoint_kernel),
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kAdjointSmem)) != cudaSuccess)
+    return bail(dfail(h, CKMPM_ERR_CUDA, "cudaFuncSetAttribute failed"));
+  for (int k = 0; k < 3; ++k)
+    if (cudaMemsetAsync(h->gsum[k], 0, 32 * nn, h->stream) != cudaSuccess ||
+        cudaMemsetAsync(h->vbar[k], 0, 24 * nn, h->stream) != cudaSuccess)
+      return bail(dfail(h, CKMPM_ERR_CUDA, "initialisation failed"));
+  if (cudaMemsetAsync(h->d.adj_scale, 0, 4 * sizeof(float), h->stream) != cudaSuccess ||
       cudaMemsetAsync(h->vel, 0, 16 * nn, h->stream) != cudaSuccess ||
       cudaStreamSynchronize(h->stream) != cudaSuccess)
     return bail(dfail(h, CKMPM_ERR_CUDA, "initialisation failed"));
@@ -745,6 +841,16 @@ ckmpm_status ckmpm_diff_destroy(ckmpm_diff* h) {
 }  // extern "C"
 
 namespace {
+
+// One forward substep s.  `sums` null: its node velocities are in vel already.
+// zero_prev: the sums that substep s - 1 read are still to be zeroed.
+void forward_substep(ckmpm_diff* h, uint32_t s, const float* in, float* outp, float4* vel, const unsigned long long* sums,
+                     float cdt, float ndt, bool zero_prev) {
+  const uint32_t n = h->d.n;
+  particle_kernel<<<blocks_for(n), kThreads, kForwardSmem, h->stream>>>(
+      h->d, in, in + 3 * n, h->lam, h->mu, vel, sums, cdt, ndt, h->gsum[(s + 1) % 3], h->box + 6 * (s + 1),
+      zero_prev ? h->gsum[(s + 2) % 3] : nullptr, h->box + 6 * (s > 0 ? s - 1 : 0), outp, outp + 3 * n);
+}
 
 // The whole forward rollout: init, rasterise, nsteps substeps; checkpoint k
 // (x, F and node velocities of substep k * every) on the way; outputs xT, FT.
@@ -779,16 +885,14 @@ cudaError_t enqueue_rollout(ckmpm_diff* h) {
     const bool ck = (s % h->every) == 0;
     const uint32_t k = s / h->every;
     float4* vs = ck ? h->ckvel + static_cast<size_t>(k) * nn : h->vel;
-    // grid update of substep s (reads gsum[s & 1] in box s; resets box s + 1)
-    grid_kernel<<<ctas, 256, 0, st>>>(d, h->gsum[s & 1], h->box + 6 * s, cdt, vs);
     float* in = state(s);
     float* outp = state(s + 1);
-    particle_kernel<<<blocks_for(n), kThreads, kDepositTile, st>>>(d, in, in + 3 * n, h->lam, h->mu, vs, cdt, ndt,
-                                                        h->gsum[(s + 1) & 1], h->box + 6 * (s + 1), outp,
-                                                        outp + 3 * n);
+    forward_substep(h, s, in, outp, vs, h->gsum[s % 3], cdt, ndt, s > 0);
   }
-  // Leave the last deposit's sums at zero (they are never read).
-  grid_kernel<<<ctas, 256, 0, st>>>(d, h->gsum[h->nsteps & 1], h->box + 6 * h->nsteps, h->dt, h->vel);
+  // Leave the last two substeps' sums at zero (nothing reads the last deposit).
+  const uint32_t N = h->nsteps;
+  zero_box_kernel<4><<<ctas, 256, 0, st>>>(d, h->box + 6 * (N - 1), h->gsum[(N - 1) % 3]);
+  zero_box_kernel<4><<<ctas, 256, 0, st>>>(d, h->box + 6 * N, h->gsum[N % 3]);
   const float* fin = state(h->nsteps);
   soa_to_aos_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 3, h->perm, fin, h->xT);
   soa_to_aos_kernel<<<blocks_for(n), kThreads, 0, st>>>(n, 9, h->perm, fin + 3 * n, h->FT);
@@ -813,10 +917,12 @@ cudaError_t enqueue_backward(ckmpm_diff* h) {
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(h->lamb, 0, sizeof(float) * n, st);
   if (e != cudaSuccess) return e;
-  bool first = true;  // the last substep's deposit has no adjoint
+  const uint32_t N = h->nsteps;
+  const float* xnext = h->xs[N & 1];   // x of the state after the substep at hand (the rollout's last state first)
+  const float4* vnext = nullptr;       // node velocities of the substep after it (none after the last)
   for (int k = static_cast<int>(h->nseg) - 1; k >= 0; --k) {
     const uint32_t s0 = static_cast<uint32_t>(k) * h->every;
-    const uint32_t s1 = std::min(h->nsteps, s0 + h->every);
+    const uint32_t s1 = std::min(N, s0 + h->every);
     // recompute: the segment's first state is its checkpoint, state s0 + j (j >= 1)
     // tape slot j - 1; tapevel slot j holds the node velocities of substep s0 + j
     auto statep = [&](uint32_t s) -> float* {
@@ -825,31 +931,32 @@ cudaError_t enqueue_backward(ckmpm_diff* h) {
     auto velp = [&](uint32_t s) -> float4* {
       return s == s0 ? h->ckvel + static_cast<size_t>(k) * nn : h->tapevel + static_cast<size_t>(s - s0) * nn;
     };
-    for (uint32_t s = s0; s < s1; ++s) {
-      const float cdt = s == 0 ? 0.f : h->dt, ndt = h->dt;
-      float* in = statep(s);
-      if (s > s0)
-        grid_kernel<<<ctas, 256, 0, st>>>(d, h->gsum[s & 1], h->box + 6 * s, cdt, velp(s));
-      if (s + 1 < s1) {
-        float* outp = statep(s + 1);
-        particle_kernel<<<blocks_for(n), kThreads, kDepositTile, st>>>(d, in, in + 3 * n, h->lam, h->mu, velp(s), cdt, ndt,
-                                                            h->gsum[(s + 1) & 1], h->box + 6 * (s + 1), outp,
-                                                            outp + 3 * n);
-      }
+    for (uint32_t s = s0; s + 1 < s1; ++s)
+      forward_substep(h, s, statep(s), statep(s + 1), velp(s), s == s0 ? nullptr : h->gsum[s % 3],
+                      s == 0 ? 0.f : h->dt, h->dt, s > s0 + 1);
+    if (s1 - s0 > 1) {
+      // The last state's velocities; this zeroes its sums, and those read before it.
+      grid_kernel<<<ctas, 256, 0, st>>>(d, h->gsum[(s1 - 1) % 3], h->box + 6 * (s1 - 1), h->dt, velp(s1 - 1));
+      if (s1 - s0 > 2) zero_box_kernel<4><<<ctas, 256, 0, st>>>(d, h->box + 6 * (s1 - 2), h->gsum[(s1 - 2) % 3]);
     }
     // reverse through the segment
-    for (int s = static_cast<int>(s1) - 1; s >= static_cast<int>(s0); --s) {
+    for (int i = static_cast<int>(s1) - 1; i >= static_cast<int>(s0); --i) {
+      const uint32_t s = static_cast<uint32_t>(i);
       const float cdt = s == 0 ? 0.f : h->dt, ndt = h->dt;
-      const float* in = statep(static_cast<uint32_t>(s));
-      particle_adjoint_kernel<<<blocks_for(n), kThreads, kAdjointTile, st>>>(d, in, in + 3 * n, h->lam, h->mu, velp(s), cdt, ndt,
-                                                                  first ? nullptr : h->gadj, h->xb, h->Fb, h->mub,
-                                                                  h->lamb, h->vbar);
-      first = false;
-      grid_adjoint_kernel<<<ctas, 256, 0, st>>>(d, h->box + 6 * s, velp(s), cdt, h->vbar, h->gadj);
+      const float* in = statep(s);
+      // vbar of substep s + 2, which substep s + 1 read, is zeroed here.
+      particle_adjoint_kernel<<<blocks_for(n), kThreads, kAdjointSmem, st>>>(
+          d, in, in + 3 * n, xnext, h->lam, h->mu, velp(s), vnext, cdt, ndt, vnext ? h->vbar[(s + 1) % 3] : nullptr, h->xb,
+          h->Fb, h->mub, h->lamb, h->vbar[s % 3], s + 2 < N ? h->vbar[(s + 2) % 3] : nullptr,
+          h->box + 6 * std::min(s + 2, N));
+      xnext = in;
+      vnext = velp(s);
     }
   }
-  finish_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, h->ck, h->v0, h->gadj, h->xb, h->lam, h->mu, h->mub, h->lamb,
-                                                    h->perm, h->gx0, h->gv0, h->glogE);
+  finish_kernel<<<blocks_for(n), kThreads, 0, st>>>(d, h->ck, h->v0, h->vbar[0], h->ckvel, h->xb, h->lam, h->mu, h->mub,
+                                                    h->lamb, h->perm, h->gx0, h->gv0, h->glogE);
+  zero_box_kernel<3><<<ctas, 256, 0, st>>>(d, h->box, h->vbar[0]);
+  if (N > 1) zero_box_kernel<3><<<ctas, 256, 0, st>>>(d, h->box + 6, h->vbar[1]);
   return cudaGetLastError();
 }
 

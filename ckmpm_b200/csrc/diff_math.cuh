@@ -67,6 +67,17 @@ CKD T dcos(T a) {
 #endif
 }
 
+// a b + c in one rounding.  The node updates below are compiled into several kernels
+// whose results must agree bit for bit, so they leave the compiler nothing to contract.
+template <class T>
+CKD T fused(T a, T b, T c) {
+#if defined(__CUDA_ARCH__)
+  return fma(a, b, c);
+#else
+  return std::fma(a, b, c);
+#endif
+}
+
 // ------------------------------------------------------------------ 3x3 helpers (row-major)
 template <class T>
 CKD void mm(const T* a, const T* b, T* r) {  // r = a b (r may alias neither)
@@ -355,10 +366,11 @@ struct Fwd {
 };
 
 // G2P + x, F update + stress + affine term.  vel(g, cx, cy, cz, T* v) returns
-// the node velocity after the grid update; svd(F, U, S, V) any SVD.
+// the node velocity after the grid update; svd(F, U, S, V) any SVD.  xn, when
+// given, is the new position where it is already known.
 template <class T, class Vel, class Svd>
 CKD void particle_forward(const Particle<T>& p, T lambda, T mu, T vol_over_mass, T dt, T ndt, T dx, T inv_dx,
-                          Vel vel, Svd svd, Fwd<T>& f, T* U, T* S, T* V) {
+                          Vel vel, Svd svd, Fwd<T>& f, T* U, T* S, T* V, const T* xn = nullptr) {
   make_stencil(p.x, inv_dx, f.st);
   CKD_UNROLL
   for (int k = 0; k < 9; ++k) f.B[k] = T(0);
@@ -403,7 +415,7 @@ CKD void particle_forward(const Particle<T>& p, T lambda, T mu, T vol_over_mass,
   sym_full(Di6, f.Di);
   mm(f.B, f.Di, f.C);
   CKD_UNROLL
-  for (int a = 0; a < 3; ++a) f.xn[a] = p.x[a] + dt * f.v[a];
+  for (int a = 0; a < 3; ++a) f.xn[a] = xn ? xn[a] : p.x[a] + dt * f.v[a];
   T dW[9];
   CKD_UNROLL
   for (int k = 0; k < 9; ++k) dW[k] = f.C[k] * dt + ((k & 3) ? T(0) : T(1));
@@ -618,9 +630,10 @@ template <class T>
 CKD bool node_update(const DenseGrid& G, int cx, int cy, int cz, T m, const T* mv, T dt, T* v) {
   v[0] = v[1] = v[2] = T(0);
   if (!(m > static_cast<T>(G.mass_clamp)) || !node_active_block(G, cx, cy, cz)) return false;
+  const T im = T(1) / m;
   CKD_UNROLL
-  for (int i = 0; i < 3; ++i) v[i] = mv[i] / m;
-  v[1] += static_cast<T>(G.gravity) * dt;
+  for (int i = 0; i < 3; ++i) v[i] = mv[i] * im;
+  v[1] = fused(static_cast<T>(G.gravity), dt, v[1]);
   if (G.boundary == 1 && static_cast<T>(cy) < static_cast<T>(G.floor_cells) && v[1] < T(0)) v[1] = T(0);
   return true;
 }
@@ -634,10 +647,11 @@ CKD void node_update_adjoint(const DenseGrid& G, int cx, int cy, int cz, T m, co
   // slip floor clamp: v_y = max(u_y + g dt, 0) passes no gradient where it clamped
   if (G.boundary == 1 && static_cast<T>(cy) < static_cast<T>(G.floor_cells) && v[1] == T(0)) vb[1] = T(0);
   // u = mv / m = v - g dt e_y (where not clamped)
-  const T u[3] = {v[0], v[1] - static_cast<T>(G.gravity) * dt, v[2]};
-  out4[0] = -(vb[0] * u[0] + vb[1] * u[1] + vb[2] * u[2]) / m;
+  const T u[3] = {v[0], fused(-static_cast<T>(G.gravity), dt, v[1]), v[2]};
+  const T im = T(1) / m;
+  out4[0] = -fused(vb[2], u[2], fused(vb[1], u[1], vb[0] * u[0])) * im;
   CKD_UNROLL
-  for (int i = 0; i < 3; ++i) out4[1 + i] = vb[i] / m;
+  for (int i = 0; i < 3; ++i) out4[1 + i] = vb[i] * im;
 }
 
 }  // namespace diff
