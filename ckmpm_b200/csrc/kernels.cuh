@@ -12,18 +12,20 @@
 //    integer reductions, so the sums do not depend on the order they arrive in.
 //  * stamp[2]: per block, the epoch for which it was last zeroed; a block whose
 //    stamp is stale reads as empty.  Only the blocks a substep deposits into
-//    are zeroed, by zero_windows_kernel before that substep.
+//    are zeroed, before that substep (by the compaction in a small domain, by
+//    zero_windows_kernel in a large one).
 //  * per model, particle state SoA (x[3], F[9], aux, Q[9] for the linear
 //    model, id) double-buffered and sorted by particle block; the block list
 //    (keys, start, count) in colour-major key order; a dense block table; 28
 //    outgoing-direction prefix counts per block and a u16 per-particle index
 //    list that records, for each block, which of its particles leave in which
-//    of the 27 directions.
+//    of the 27 directions; next-step totals per block, in traversal order.
 //
 // Every substep is: one fused kernel per model (grid update + G2P + F update,
-// SVD, return map + rebin record + P2G, flushed as exact integer sums), then
+// stress, return map + rebin record + P2G, flushed as exact integer sums), then
 // the colour-major compaction that builds the next block list and the zeroing
-// of the blocks the next substep deposits into.  No host sync.
+// of the blocks the next substep deposits into, whose last CTA advances the
+// clock.  No host sync.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -268,9 +270,8 @@ __device__ __forceinline__ float4 node_velocity(const SceneDev& sc, const long l
   if (m > sc.mass_clamp) {
     const float inv = __frcp_rn(m);  // IEEE-rounded 1/m, as the reference's invMass (the build approximates 1/x)
     v.x = __ll2float_rn(__ldcg(blk + 128 + cell)) * unit * inv;
-    v.y = __ll2float_rn(__ldcg(blk + 256 + cell)) * unit * inv;
+    v.y = fmaf(__ll2float_rn(__ldcg(blk + 256 + cell)) * unit, inv, __fmul_rn(sc.gravity, dt));
     v.z = __ll2float_rn(__ldcg(blk + 384 + cell)) * unit * inv;
-    v.y = fmaf(sc.gravity, dt, v.y);
     if (sc.boundary == 0) {
       const bool out = (bx < 2 || bx + 2 >= sc.dims[0]) || (by < 2 || by + 2 >= sc.dims[1]) ||
                        (bz < 2 || bz + 2 >= sc.dims[2]);
@@ -558,6 +559,12 @@ __device__ __forceinline__ void p2g_scatter(unsigned* __restrict__ ptile, const 
     }
   }
 }
+
+}  // namespace ckmpm
+
+#include "nacc_transfer.cuh"
+
+namespace ckmpm {
 
 // Epilogue shared by the substep and the initial rasterisation: add this
 // block's tile into the 2x2x2 grid blocks it covers with 64-bit integer
@@ -885,7 +892,14 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       if (material_has_aux(kind)) aux = sin.aux[iin];
       bool inside = true;
       float v[3], Cdx[9], Dold[6];  // C dx and D / dx^2
-      g2p(vtile, x, inv_dx, key, v, Cdx, inside, Dold);
+      // Cam-clay's transfers hold C and D in place of C dx and D / dx^2.
+      const bool clayey = KIND == kNacc || (KIND == kMixed && kind == kNacc);
+      if (clayey) {
+        const float xs[3] = {x[0] * inv_dx, x[1] * inv_dx, x[2] * inv_dx};
+        clay::g2p(vtile, xs, key, sc.dx, v, Cdx, inside, Dold);
+      } else {
+        g2p(vtile, x, inv_dx, key, v, Cdx, inside, Dold);
+      }
       float adv[3] = {v[0], v[1], v[2]};
       if (RIGID && rigid_attribute(kind, F, aux) == 0.f) {
         // Rigid: moves with the scene's rigid velocity and carries no velocity,
@@ -901,7 +915,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         }
       }
 #pragma unroll
-      for (int a = 0; a < 3; ++a) x[a] = fmaf(dt, adv[a], x[a]);
+      for (int a = 0; a < 3; ++a) x[a] = clayey ? x[a] + dt * adv[a] : fmaf(dt, adv[a], x[a]);
 
       float tau[9];
       if (kind == kFluid) {
@@ -911,9 +925,15 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         stress_fluid(mp0, mp1, mp2, C, dt, aux, tau);
       } else {
         float dW[9];
+        if (clayey) {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) dW[k] = (k & 3) ? Cdx[k] * dtdx : fmaf(Cdx[k], dtdx, 1.f);
-        matmul3(dW, F, F);
+          for (int k = 0; k < 9; ++k) dW[k] = Cdx[k] * dt + ((k & 3) ? 0.f : 1.f);
+          matmul3_plain(dW, F, F);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 9; ++k) dW[k] = (k & 3) ? Cdx[k] * dtdx : fmaf(Cdx[k], dtdx, 1.f);
+          matmul3(dW, F, F);
+        }
         if (kind == kFixedCorotated) {
           stress_fixed_corotated(mp0, mp1, F, tau);
         } else if (kind == kDruckerPrager) {
@@ -978,10 +998,41 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       // reference adds the new position's D onto the G2P D of the old position
       // (it never resets it, :1524,1604,1729) and inverts half the sum (:1732),
       // so M = (0.5 (D_old + D_new))^-1.
+      float D6[6], Di6[6], Di[9], DT[9];
+      if (clayey) {
+        clay::AxisStencil st[2][3];
+        int lb[2][3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float xs = x[a] * inv_dx;
+          st[0][a] = clay::axis_stencil<-1>(xs);
+          st[1][a] = clay::axis_stencil<1>(xs);
+          lb[0][a] = st[0][a].base - 4 * kk[a];
+          lb[1][a] = st[1][a].base - 4 * kk[a];
+        }
+        clay::d_matrix(st, sc.dx, D6);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) D6[k] = 0.5f * (Dold[k] + D6[k]);
+        clay::inv_sym3(D6[0], D6[1], D6[2], D6[3], D6[4], D6[5], Di6);
+        sym_to_full(Di6, Di);
+        matmul3_plain(Di, tau, DT);
+        float Ah[9];
+        bool finite = true;
+        const float sA = ndt * vol_over_mass;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+          Ah[k] = (Cdx[k] - sA * DT[k]) * sc.dx;
+          finite &= fabsf(Ah[k]) < kFixMaxValue;
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) finite &= fabsf(v[r]) < kFixMaxValue;
+        if (finite) clay::p2g_scatter(ptile, st, lb, v, Ah);
+        else set_status(scal, kStatusNumeric);
+        continue;
+      }
       AxisStencil st[3];
 #pragma unroll
       for (int a = 0; a < 3; ++a) st[a] = axis_stencil(x[a], inv_dx);
-      float D6[6], Di6[6], Di[9], DT[9];
       d_matrix(st, D6);
 #pragma unroll
       for (int k = 0; k < 6; ++k) D6[k] = 0.5f * (Dold[k] + D6[k]);
@@ -1113,9 +1164,29 @@ __global__ void __launch_bounds__(NT, 2) rasterize_kernel(SceneDev sc, ModelDev 
     const uint32_t start = cur.start[item];
     const uint32_t n = cur.count[item];
     const int kk[3] = {key.x, key.y, key.z};
+    const bool clayey = (md.smat ? md.smat[key.w].kind : md.mat.kind) == kNacc;
     for (uint32_t q = threadIdx.x; q < n; q += NT) {
       const uint32_t i = start + q;
       const float v[3] = {md.vel_in[3 * i], md.vel_in[3 * i + 1], md.vel_in[3 * i + 2]};
+      if (clayey) {
+        clay::AxisStencil st[2][3];
+        int lb[2][3];
+        bool ok = true;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float xs = s0.x[a][i] * inv_dx;
+          st[0][a] = clay::axis_stencil<-1>(xs);
+          st[1][a] = clay::axis_stencil<1>(xs);
+          lb[0][a] = st[0][a].base - 4 * kk[a];
+          lb[1][a] = st[1][a].base - 4 * kk[a];
+          ok &= lb[0][a] >= 0 && lb[0][a] <= 6 && lb[1][a] >= 0 && lb[1][a] <= 6;
+        }
+        const bool finite = fabsf(v[0]) < kFixMaxValue && fabsf(v[1]) < kFixMaxValue && fabsf(v[2]) < kFixMaxValue;
+        if (!ok) set_status(scal, kStatusOutsideBlock);
+        if (!finite) set_status(scal, kStatusNumeric);
+        if (ok && finite) clay::p2g_scatter(ptile, st, lb, v, Z);
+        continue;
+      }
       AxisStencil st[3];
       bool ok = true;
 #pragma unroll

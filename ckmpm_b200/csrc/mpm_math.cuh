@@ -63,6 +63,17 @@ CKMPM_DEV void matmul3(const float* a, const float* b, float* r) {
   for (int k = 0; k < 9; ++k) r[k] = t[k];
 }
 
+// The same with the compiler's own contraction, for the Cam-clay path (nacc_transfer.cuh).
+CKMPM_DEV void matmul3_plain(const float* a, const float* b, float* r) {
+  float t[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) t[i * 3 + j] = a[i * 3] * b[j] + a[i * 3 + 1] * b[3 + j] + a[i * 3 + 2] * b[6 + j];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) r[k] = t[k];
+}
+
 // ------------------------------------------------------------------ SVD
 //
 // A = U diag(S) V^T with U, V proper rotations, |S0| >= |S1| >= |S2|, S0, S1 >= 0
@@ -164,7 +175,7 @@ CKMPM_DEV void swap_cols(float* V, float& la, float& lb, int a, int b) {
   }
 }
 
-template <int kSweeps = 3>
+template <int kSweeps = 3, bool PLAIN = false>
 CKMPM_DEV void svd3(const float* A, float* U, float* S, float* V) {
   // M = A^T A (symmetric; 6 unique entries)
   float m00 = A[0] * A[0] + A[3] * A[3] + A[6] * A[6];
@@ -186,7 +197,8 @@ CKMPM_DEV void svd3(const float* A, float* U, float* S, float* V) {
   if (l0 < l2) swap_cols(V, l0, l2, 0, 2);
   if (l1 < l2) swap_cols(V, l1, l2, 1, 2);
   float B[9];
-  matmul3(A, V, B);
+  if (PLAIN) matmul3_plain(A, V, B);
+  else matmul3(A, V, B);
 #pragma unroll
   for (int k = 0; k < 9; ++k) U[k] = (k & 3) ? 0.0f : 1.0f;
   givens_qr_step(B, U, 0, 1, 0);
@@ -483,7 +495,7 @@ CKMPM_DEV void stress_nacc(const float* prm, float* F, float& logJp, float* tau)
   const bool hardening = prm[6] != 0.0f;
   const float K = 2.0f * mu / 3.0f + lambda;
   float U[9], S[3], V[9];
-  svd3(F, U, S, V);
+  svd3<3, true>(F, U, S, V);
   const float p0 = K * (1e-5f + sinhf(xi * (-logJp > 0.0f ? -logJp : 0.0f)));
   const float pmin = -beta * p0;
   const float je = S[0] * S[1] * S[2];

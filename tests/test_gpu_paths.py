@@ -67,6 +67,18 @@ def test_split_blocks_give_the_same_bits(engine_lib, kind, n, blocks):
             assert np.array_equal(p, q)
 
 
+@pytest.mark.parametrize("n", [40, 17000, 60000])
+def test_cam_clay_gives_the_same_bits_everywhere(engine_lib, n):
+    """Cam-clay's F jumps with its last bit (F = U diag(S) V, V not transposed), so its own
+    transfers must agree bit for bit between launch shapes."""
+    cfg, models = box_scene(n, (14, 14, 14))
+    lam, mu = compute_lame_parameters(2e4, 0.4)
+    models[0].material = MPMMaterial.nacc(mu, lam, -0.01, 0.5, 0.8, 2.36, True)
+    a = run(cfg, models, 33, (256, 4, 8)).state(0)
+    for shape in (None, (128, 5, 8), (192, 4, 8), (1024, 1, 8)):
+        assert_same(run(cfg, models, 33, shape).state(0), a, shape)
+
+
 @pytest.mark.parametrize("dims", [(9, 11, 13), (25, 25, 26), (26, 26, 26), (64, 17, 16)])
 def test_domain_size_does_not_matter(engine_lib, dims):
     """The compaction's small and large tiles, odd extents among them: the same body far from
