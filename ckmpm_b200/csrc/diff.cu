@@ -3,12 +3,15 @@
 // substep checkpointing with recomputation.  No counterpart in the reference.
 //
 // Device layout (cells per axis n_c, nodes nn = 2 n_c^3 over both staggered grids):
-//  * gsum[2]: int64 fixed-point node sums [node][m, mvx, mvy, mvz] per unit
-//    particle mass (2^36 scale, as the substep's P2G tile), double-buffered;
-//    exact, so a recomputed segment reproduces the forward bit for bit;
-//  * vel: float4 per node (v after the grid update, m);
+//  * particles sorted once per rollout (perm), so that a CTA's lie in a small box
+//    of nodes: it makes that box's velocities, or their adjoints, itself from the sums and
+//    collects its deposits in a shared tile;
+//  * gsum[3]: int64 fixed-point node sums [node][m, mvx, mvy, mvz] per unit
+//    particle mass (2^36 scale, as the substep's P2G tile), one read, one written
+//    and one cleared in a substep; exact, so a recomputed segment reproduces the
+//    forward bit for bit;
 //  * bbox[s]: node-coordinate box of what substep s reads (min x,y,z, max x,y,z);
-//    the dense passes run over that box only, and every box is zeroed after use;
+//    clearing runs over that box only;
 //  * particles SoA (x[3][n], F[9][n]); checkpoints every K substeps hold x, F
 //    and the node velocities of that substep (the forward writes those states
 //    straight into their checkpoint slots); the backward recomputes one segment
@@ -16,7 +19,7 @@
 //    adjoint.  With K = 1 every substep is a checkpoint and the backward is the
 //    adjoint alone (about 2.2 GB for 50k particles, 200 substeps and a 64^3
 //    grid: HBM, not recomputation, holds the rollout);
-//  * vbar: the node-velocity adjoint the particle adjoints scatter, as exact
+//  * vbar[3]: the node-velocity adjoint the particle adjoints scatter, as exact
 //    int64 fixed-point sums like the forward's, so gradients are bitwise
 //    reproducible too.  Its unit is set on the device at the start of each
 //    backward from the largest incoming adjoint (the backward is linear in its
@@ -106,7 +109,7 @@ __global__ void order_place_kernel(uint32_t n, const uint32_t* __restrict__ firs
 // Deposits go to a shared tile of exact 64-bit sums over that box, two native
 // 32-bit atomics per value with the carry from the low word (as the substep's
 // P2G tile), and from there to the grid, one reduction per touched node and
-// channel; a box of more than kTileNodes nodes deposits into the grid directly.
+// channel; a box of more than kTileCap nodes deposits into the grid directly.
 // The sums are exact either way.  Bound before: 64 global 64-bit reductions per
 // particle, 3.2 M a launch on the 50k-particle cube.
 constexpr int kTileCap = 1024;  // nodes of both grids

@@ -326,9 +326,10 @@ ckmpm_status ckmpm_get_blocks_in(ckmpm_scene* s, uint32_t scene, int32_t model, 
 /* ---- Launch shape of the fused substep kernel.  No counterpart in the
  * reference (fixed launch shapes, include/mpm_engine.cuh:519-866).  Results do
  * not depend on it: the P2G tile and the grid hold exact integer sums, so the
- * order in which blocks deposit never changes a bit. */
+ * order in which blocks deposit never changes a bit.  Unless one is set, setup
+ * takes 256 x occupancy, or the cluster shape where that many CTAs per block fit at once. */
 typedef struct ckmpm_tuning {
-  uint32_t threads;      /* CTA size: 128, 192, 256 or 1024 (one CTA per SM; for small scenes) */
+  uint32_t threads;      /* CTA size: 128, 192 or 256; 1024: 256, each block split over a cluster of CTAs (small scenes) */
   uint32_t ctas_per_sm;  /* resident persistent CTAs per SM, 1..occupancy */
   uint32_t graph_chunk;  /* substeps per captured CUDA graph, even, 2..64 */
   float probe_ms;        /* ckmpm_autotune: measured ms per substep; 0 otherwise */
