@@ -393,12 +393,14 @@ CKMPM_DEV void stress_fixed_corotated(float lambda, float mu, const float* F, fl
 // after F <- U diag(s) V^T; V^T F^T = diag(s) U^T, so tau = U diag(2 mu log s + lambda tr log s) U^T,
 // and log s is known: 0 on the tension branch (s = 1), H elsewhere.
 // An elastic step (dg <= 0, stretches within the clamp) leaves F as it is.
+// An inverted F takes svd3's rotations U and V: F <- U diag(s) V^T with s > 0 undoes the
+// reflection, which the additive map and the untouched elastic step would keep.
 CKMPM_DEV void stress_drucker_prager(float lambda, float mu, float* F, float& logJp, float* tau) {
   const float kYs = 0.816496580927726f * 2.0f * 0.5f / (3.0f - 0.5f);
   const float smu = 2.0f * mu;
   float U[9], W[9], S[3];
   left_stretch(F, U, W, S);
-  const bool good = left_well_conditioned(S) && S[0] > 4e-4f;
+  const bool good = left_well_conditioned(S) && S[0] > 4e-4f && det3(F) > 0.0f;
   if (!good) {
     float V[9];
     svd3(F, U, S, V);

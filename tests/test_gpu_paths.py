@@ -124,6 +124,39 @@ def test_stress_of_ill_conditioned_deformation(engine_lib, oracle_mod, kind):
         assert np.abs(Fg[i] - Fo).max() <= 16 * eps + 2e-6, i
 
 
+@pytest.mark.parametrize("branch", ["tension", "elastic", "plastic"])
+def test_inverted_sand_leaves_unreflected(engine_lib, oracle_mod, branch):
+    """Drucker-Prager writes F = U diag(exp h) V^T with rotations U and V, so an inverted F leaves with a positive
+    determinant in every branch, at stretch ratios under and over the 4 at which the return map goes back to the
+    full SVD.  F and the FP64 oracle's differ by the singular vectors' error, 2^-23 over the smallest gap of the
+    squared stretches to the largest (the stretches are kept apart), times exp h: the tolerance is 32 of those."""
+    rng = np.random.default_rng(5)
+    n = 240
+    ratio = np.exp(rng.uniform(math.log(1.3), math.log(40.0), n))
+    s = np.stack([np.ones(n), ratio ** -rng.uniform(0.35, 0.65, n), 1 / ratio], 1)
+    gap = np.minimum(1 - s[:, 1] ** 2, s[:, 1] ** 2 - s[:, 2] ** 2)
+    s *= np.exp(rng.uniform(-0.3, 0.3, (n, 1)))
+    volume = np.log(s).sum(1)
+    aux = {"tension": 1.0 - volume, "elastic": np.full(n, -30.0), "plastic": -0.05 - volume}[branch].astype(np.float32)
+    s[:, 2] *= -1
+    F = ((rotations(rng, n) * s[:, None, :]) @ rotations(rng, n).transpose(0, 2, 1)).astype(np.float32)
+    lam, mu = 2.0e4, 3.0e4
+    mat = capi.Material()
+    mat.kind = capi.DRUCKER_PRAGER
+    mat.p[0], mat.p[1] = lam, mu
+    Fg, ag, tau = F.copy(), aux.copy(), np.zeros_like(F)
+    capi.check(engine_lib.ckmpm_debug_constitutive(mat, n, capi.fptr(np.zeros_like(F)), 0.0, capi.fptr(Fg),
+                                                   capi.fptr(ag), capi.fptr(tau), None, None, None), "debug")
+    assert (np.linalg.det(Fg.astype(np.float64)) > 0).all()
+    for i in range(n):
+        Fo, ao, to = oracle_mod.constitutive(capi.DRUCKER_PRAGER, [lam, mu, 0.0, 0.0], np.zeros((3, 3)), 0.0,
+                                             F[i].astype(np.float64), float(aux[i]))
+        eps = 2.0 ** -23
+        assert np.abs(Fg[i] - Fo).max() <= 32 * eps / gap[i] * max(1.0, np.abs(Fo).max()), i
+        assert np.abs(tau[i] - to).max() <= 8 * eps * float(ratio[i]) * 5 * max(lam, mu) + 2e-5 * np.abs(to).max(), i
+        assert abs(ag[i] - ao) <= 16 * eps * float(ratio[i]), i
+
+
 @pytest.mark.parametrize("boundary", ["sticky_blocks", "slip_floor"])
 def test_adaptive_frame_equals_its_substeps(engine_lib, boundary):
     """A frame in one call (substeps replayed from graphs, the dt taken on the device) against the
