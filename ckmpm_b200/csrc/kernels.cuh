@@ -816,6 +816,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
   load_classes(sc, sh.classes);
   for (int i = threadIdx.x; i < 2 * kTilePlane / 4; i += NT)
     reinterpret_cast<uint4*>(ptile)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();  // the classes, before a cluster's first block (the ticket's barrier below is not its)
   // Blocks come from the ticket, one at a time when a CTA is free (taking the next one
   // early lengthens the launch's tail: 6 % on the sand column); clusters, which
   // seldom have a second block, stride.
