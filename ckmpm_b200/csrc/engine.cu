@@ -81,7 +81,7 @@ struct ckmpm_scene {
   std::string err;
   int sm_count = 0;
   int fused_ctas = 0;
-  uint32_t parts = 1;      // cluster shape: CTAs per block
+  uint32_t parts = 1;      // cluster shape: CTAs per cluster
   bool tuned = false;      // the caller chose the launch shape (ckmpm_set_tuning, ckmpm_autotune)
   int occ[4] = {0, 0, 0, 0};  // resident fused CTAs per SM at 128 / 256 / cluster shape / 192 threads
   uint32_t nstack = 1;     // stacked domains: 1, or the scene count of a batch
@@ -220,6 +220,7 @@ cudaError_t launch_fused_any(ckmpm_scene* s, const ModelHost& m, int parity) {
 // fixed-corotated box at 256 threads x 4, and in clusters of 2 / 4 / 8:
 //   27 blocks 28.5, 24.4 / 23.7 / 23.8 us;  115 blocks 36.5, 31.8 / 28.4 / 40.1 us;
 //   216 blocks 42.1, 36.9 / 43.0 / 66.8 us;  343 blocks 45.6, 54.3 / 69.7 us.
+// The count is the setup's; the kernel itself goes back to whole blocks when they outgrow it.
 uint32_t cluster_parts(int sm_count, uint32_t nblocks) {
   const uint32_t slots = 4u * static_cast<uint32_t>(sm_count);
   return nblocks * 4u <= slots ? 4u : nblocks * 2u <= slots ? 2u : 1u;

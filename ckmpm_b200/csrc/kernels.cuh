@@ -734,6 +734,7 @@ struct SharedSmall {
   ColourClasses classes;
   int64_t blk[8];
   uint32_t item;
+  uint32_t next;  // clusters: the block shared by this one's CTAs, then past the end
   uint32_t off[28];
   uint32_t idx[27];
   uint32_t src[27];
@@ -763,6 +764,9 @@ constexpr size_t kSmemFused = kSmemVTile + kSmemPTile + kSmemCodes;
 // with tiles of its own, flushed into the grid like any others (the sums are
 // exact), and only the direction counts of the rebin ranking cross CTAs, through
 // distributed shared memory.  The particles' order, and every bit, stays the same.
+// A scene may spread after its shape was chosen, in the middle of a graph: as soon as
+// the substep's own blocks are too many for a cluster each, its CTAs take whole
+// blocks instead.
 template <int NT>
 constexpr int fused_min_ctas() { return NT == 128 ? 5 : 1024 / NT; }
 
@@ -807,25 +811,34 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
   const float dtdx = dt * inv_dx;
   const uint32_t maxp = min(md.max_per_block, static_cast<uint32_t>(kMaxParticlesPerBlock));
 
-  // Cluster of nparts CTAs per block (1 without CLUSTER), this one taking part `part`.
+  // Cluster of nparts CTAs per block (1 without CLUSTER), this one taking part `part`,
+  // while there is a cluster for every block (`split`).
   namespace cg = cooperative_groups;
   const uint32_t nparts = CLUSTER ? cg::this_cluster().num_blocks() : 1u;
   const uint32_t part = CLUSTER ? cg::this_cluster().block_rank() : 0u;
-  const uint32_t first = blockIdx.x / nparts, nworkers = gridDim.x / nparts;
+  const bool split = CLUSTER && nb <= gridDim.x / nparts;
+  const bool leads = !split || part == 0;
+  const uint32_t first = split ? blockIdx.x / nparts : blockIdx.x;
   if (first >= nb) return;
   load_classes(sc, sh.classes);
   for (int i = threadIdx.x; i < 2 * kTilePlane / 4; i += NT)
     reinterpret_cast<uint4*>(ptile)[i] = make_uint4(0u, 0u, 0u, 0u);
-  __syncthreads();  // the classes, before a cluster's first block (the ticket's barrier below is not its)
+  if (CLUSTER && threadIdx.x == 0) sh.next = first;
   // Blocks come from the ticket, one at a time when a CTA is free (taking the next one
-  // early lengthens the launch's tail: 6 % on the sand column); clusters, which
-  // seldom have a second block, stride.
-  for (uint32_t item = first;; item += nworkers) {
-    if constexpr (!CLUSTER) {
-      if (threadIdx.x == 0) sh.item = atomicAdd(md.ticket, 1u);
-      __syncthreads();
-      item = sh.item;
+  // early lengthens the launch's tail: 6 % on the sand column); a split block is its
+  // cluster's only one.  Every instantiation takes its block through the same barrier
+  // (the colour classes need it too): a barrier in one of two branches costs 70 bytes of spills.
+  for (;;) {
+    if (threadIdx.x == 0) {
+      if (split) {
+        sh.item = sh.next;
+        sh.next = nb;
+      } else {
+        sh.item = atomicAdd(md.ticket, 1u);
+      }
     }
+    __syncthreads();
+    const uint32_t item = sh.item;
     if (item >= nb) break;
     const int4 key = cur.keys[item];
     const uint32_t start = cur.start[item];
@@ -860,7 +873,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
     // The block's output slots [start, start + n) must lie in the state arrays;
     // counts that say otherwise are flagged and clamped, never written past.
     const uint32_t room = start < md.cap_particles ? md.cap_particles - start : 0u;
-    if (threadIdx.x == 0 && part == 0) {
+    if (threadIdx.x == 0 && leads) {
       uint32_t flags = 0;
       if (sh.off[27] != n || n > room) flags |= kStatusConsistency;
       if (n > maxp) flags |= kStatusCapacity;
@@ -870,7 +883,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
 
     // This CTA's particles [q0, q1) of the block, whole warps of them.
     uint32_t q0 = 0, q1 = n;
-    if (CLUSTER) {
+    if (split) {
       const uint32_t each = (((n + 31) >> 5) + nparts - 1) / nparts * 32;
       q0 = min(part * each, n);
       q1 = min(q0 + each, n);
@@ -1085,11 +1098,11 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       }
       if constexpr (CLUSTER) pc.count[lane] = mine;
     }
-    if (CLUSTER) cg::this_cluster().sync();
+    if (CLUSTER && split) cg::this_cluster().sync();
     uint32_t total = mine;  // of the block, in direction `lane`
     if (threadIdx.x < 32) {
       uint32_t before = 0;  // in the parts before this one
-      if constexpr (CLUSTER) {
+      if (CLUSTER && split) {
         for (uint32_t r = 0; r < nparts; ++r) {
           const uint32_t t = r == part || lane >= 28 ? 0u : cg::this_cluster().map_shared_rank(pc.count, r)[lane];
           total += t;
@@ -1107,15 +1120,15 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         const uint32_t pre = incl - cv;
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) rk.wcnt[w][lane] += pre + before;
-        if (part == 0) cur.prefix28[item * 28 + lane] = pre;
+        if (leads) cur.prefix28[item * 28 + lane] = pre;
       }
-      if (lane == 26 && part == 0) cur.prefix28[item * 28 + 27] = incl;
+      if (lane == 26 && leads) cur.prefix28[item * 28 + 27] = incl;
     }
     __syncthreads();
-    // The parts' counts have been read: the next block may overwrite them once all arrive.
-    if (CLUSTER) cg::this_cluster().barrier_arrive();
+    // The parts' counts have been read: the CTAs that hold them may end once all arrive.
+    if (CLUSTER && split) cg::this_cluster().barrier_arrive();
     // The next list's totals.
-    if (threadIdx.x < 28 && part == 0 && total > 0) {
+    if (threadIdx.x < 28 && leads && total > 0) {
       if (lane == 27) {
         atomicAdd(&scal->lost, total);
       } else {
@@ -1136,7 +1149,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       __syncwarp();
     }
     flush_tile<NT>(sc, key, ptile, ratio, gout);
-    if (CLUSTER) cg::this_cluster().barrier_wait();
+    if (CLUSTER && split) cg::this_cluster().barrier_wait();
   }
 }
 

@@ -67,6 +67,26 @@ def test_split_blocks_give_the_same_bits(engine_lib, kind, n, blocks):
             assert np.array_equal(p, q)
 
 
+def test_a_spreading_scene_outgrows_its_clusters(engine_lib):
+    """A cloud set up with so few blocks that each is split over 4 CTAs, flying apart to more blocks than
+    clusters within its graphs: the same bits as with one CTA per block throughout, and no slower than that
+    (2.7 times as slow while the split stayed as it was set up; the bound is 1.4)."""
+    cfg, models = box_scene(17000, (20, 20, 20), kind="drucker_prager", v0=(0.0, 0.0, 0.0))
+    cfg.gravity = 0.0
+    x = models[0].particle_position
+    models[0].particle_velocity = (30.0 * (x - x.mean(0))).astype(np.float32)
+    scene = [run(cfg, models, 0), run(cfg, models, 0, (256, 4, 8))]
+    sms = 148
+    assert scene[0].tuning()["threads"] == 1024 and len(scene[0].blocks(0, 0)[1]) <= sms
+    for _ in range(5):
+        for s in scene:
+            s.step(56, 1e-4)
+        assert_same(scene[0].state(0), scene[1].state(0), "spreading")
+    assert len(scene[0].blocks(0, 0)[1]) > 2 * sms
+    ms = [min(s.step_profiled(16, 1e-7)[0] for _ in range(5)) for s in scene]
+    assert ms[0] < 1.4 * ms[1], ms
+
+
 @pytest.mark.parametrize("n", [40, 17000, 60000])
 def test_cam_clay_gives_the_same_bits_everywhere(engine_lib, n):
     """Cam-clay's F jumps with its last bit (F = U diag(S) V, V not transposed), so its own
