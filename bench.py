@@ -447,8 +447,8 @@ def rollout_launches(nsteps: int, every: int) -> int:
 
 def substep_launches(cfg, n_models: int, n_scenes: int = 1) -> int:
     """Kernel launches of one substep: per model the fused kernel, the compaction (two kernels in a domain of more
-    than 16384 blocks) and the window zeroing, which the compaction of a small domain with few blocks includes; the
-    last launch also ends the substep."""
+    than 16384 blocks) and the window zeroing, which the compaction of a smaller domain includes; the last launch also
+    ends the substep."""
     entries = n_scenes * int(np.prod(cfg.domain_blocks))
     return n_models * (2 if entries <= 16384 else 4)
 

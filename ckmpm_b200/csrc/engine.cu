@@ -291,6 +291,14 @@ cudaError_t fused_attributes(int device, int* occ4) {
   return cudaSuccess;
 }
 
+// Whether the compaction also zeroes the next windows: in every small domain. Per substep with the
+// zeroing in a launch of its own, and folded (kFoldCtas CTAs), fixed-corotated boxes:
+//   16^3-block domain:   27 blocks 21.9, 18.5 us;   125: 27.5, 26.2;    343: 37.7, 36.1;   1728: 50.7, 47.9;
+//   25^3-block domain:  216 blocks 32.5, 30.1 us;  1331: 76.3, 74.5;   4913: 118, 115;     9261: 218, 215.
+// With one CTA per tile 1728 blocks took 56.4 and 9261 blocks 228 us; 128 and 512 CTAs are within 2 % of 256.
+bool folds_zero(const SceneDev& sc) { return sc.tile_shift == 8; }
+constexpr uint32_t kFoldCtas = 256;
+
 // Compaction of one model's next block list, bl[list], from the totals of `parity`.
 // With `zero_grid` >= 0 it also zeroes the windows of its blocks in that grid (epoch
 // step + 2) and, `end`, ends the substep.
@@ -300,9 +308,10 @@ cudaError_t launch_compact(const SceneDev& sc, const ModelDev& d, const GridDev&
     compact_reduce_kernel<4><<<ntiles, kCompactThreads, 0, st>>>(sc, d.dense_total[parity], d.tile_sums);
   auto launch = [&](auto kernel) {
     const int z = zero_grid < 0 ? 0 : zero_grid;
-    kernel<<<ntiles, kCompactThreads, 0, st>>>(sc, d.dense_total[parity], d.dense_total[parity ^ 1], d.tile_sums,
-                                               d.bl[list], d.cap_slots, d.ticket, scal, gd.grid[z], gd.stamp[z], 2,
-                                               end ? 1 : 0);
+    const uint32_t copies = zero_grid < 0 ? 1u : std::max(1u, kFoldCtas / ntiles);
+    kernel<<<ntiles * copies, kCompactThreads, 0, st>>>(sc, d.dense_total[parity], d.dense_total[parity ^ 1],
+                                                        d.tile_sums, d.bl[list], d.cap_slots, d.ticket, scal,
+                                                        gd.grid[z], gd.stamp[z], 2, end ? 1 : 0);
   };
   if (sc.tile_shift == 10) launch(compact_scatter_kernel<4, false>);
   else if (zero_grid < 0) launch(compact_scatter_kernel<1, false>);
@@ -339,23 +348,16 @@ cudaError_t launch_zero(ckmpm_scene* s, int list_parity, int grid_parity, int32_
   return cudaGetLastError();
 }
 
-// Whether the compaction also zeroes the next windows: in a small domain with few
-// blocks. A tile's CTA clears its own blocks' windows, up to 1 MB; a kernel of its own
-// spreads that over the whole GPU but costs a launch. With the launches saved, 100 substeps of a
-// 115-block cube took 4.25 ms against 4.77, and 8 of a 27-block one 455 us against 523;
-// 256 scenes (tens of thousands of blocks) keep the separate kernel, 44 us there.
-bool folds_zero(const SceneDev& sc, uint32_t nblocks) { return sc.tile_shift == 8 && nblocks <= 1024u; }
-
 // Enqueue one substep for every model: two launches each (fused; compaction and
-// zeroing) in a small scene, else three in a small domain and four in a large one,
-// where the compaction is two.  The last launch also ends the substep.
+// zeroing) in a small domain, four in a large one, where the compaction is two.  The
+// last launch also ends the substep.
 // The compaction of each model writes the block list the fused kernel did not
 // read: that of the other parity.  Once every model's fused kernel has read
 // grid[parity], its blocks that the next substep deposits into are zeroed for it
 // (epoch step + 2).
 cudaError_t enqueue_substep(ckmpm_scene* s, int parity) {
   cudaError_t e = cudaSuccess;
-  const bool fold = folds_zero(s->sc, s->nblocks0);
+  const bool fold = folds_zero(s->sc);
   for (auto& m : s->models) {
     if (e == cudaSuccess) e = launch_fused_any(s, m, parity);
     if (e == cudaSuccess && !fold) e = launch_compact(s, m, parity ^ 1, parity);

@@ -1366,9 +1366,10 @@ __global__ void __launch_bounds__(kCompactThreads) compact_reduce_kernel(SceneDe
 // (PER 1), without a reduce launch, from the totals themselves, at most 16 loads a thread.
 // The totals are left at zero: a large domain's in place, a small one's by the next
 // compaction (`clear`, the other parity's), since other tiles still read them here.
-// ZERO also does zero_windows_kernel's work for the tile's blocks and, with `end`, ends
-// the substep: one launch less, for scenes whose few blocks a tile's CTA clears in no
-// time (a 16^3-block domain has 16 tiles).
+// ZERO (small domains) also does zero_windows_kernel's work for the tile's blocks and, with
+// `end`, ends the substep: one launch less. A 16^3-block domain has 16 tiles, too few CTAs to clear
+// many blocks, so every tile is scanned by several CTAs (copies), which share its
+// blocks out and of which the first writes the list.
 // Bound: latency; one 16-byte load and store per 4 entries.
 template <int PER, bool ZERO>
 __global__ void __launch_bounds__(kCompactThreads)
@@ -1380,23 +1381,25 @@ __global__ void __launch_bounds__(kCompactThreads)
   __shared__ int4 active[ZERO ? kCompactThreads * PER : 1];
   __shared__ uint32_t n_active;
   const uint32_t n = sc.nblocks_domain;
-  const uint32_t t0 = (blockIdx.x * kCompactThreads + threadIdx.x) * PER;
-  const bool last = blockIdx.x == gridDim.x - 1;
+  const uint32_t ntiles = ZERO ? (n + kCompactThreads * PER - 1) / (kCompactThreads * PER) : gridDim.x;
+  const uint32_t tile = ZERO ? blockIdx.x % ntiles : blockIdx.x, copy = ZERO ? blockIdx.x / ntiles : 0u;
+  const uint32_t t0 = (tile * kCompactThreads + threadIdx.x) * PER;
+  const bool last = tile == ntiles - 1;
   const int32_t epoch = ZERO ? scal->step + epoch_offset : 0;
   if (threadIdx.x == 0) n_active = 0u;
   int slots[PER];
 #pragma unroll
   for (int k = 0; k < PER; ++k) slots[k] = -1;
-  if (PER == 1 || last || tile_sums[blockIdx.x]) {
+  if (PER == 1 || last || tile_sums[tile]) {
     unsigned long long pre = 0;
     if (PER == 1) {
-      for (uint32_t t = 4 * threadIdx.x; t < blockIdx.x * kCompactThreads; t += 4 * kCompactThreads) {
+      for (uint32_t t = 4 * threadIdx.x; t < tile * kCompactThreads; t += 4 * kCompactThreads) {
         const uint4 q = *reinterpret_cast<const uint4*>(total + t);
         pre += (static_cast<unsigned long long>((q.x > 0u) + (q.y > 0u) + (q.z > 0u) + (q.w > 0u)) << 32) +
                (q.x + q.y + q.z + q.w);
       }
     } else {
-      for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kCompactThreads) pre += tile_sums[t];
+      for (uint32_t t = threadIdx.x; t < tile; t += kCompactThreads) pre += tile_sums[t];
     }
     uint32_t c[PER];
     load_totals<PER>(total, t0, n, c);
@@ -1412,11 +1415,16 @@ __global__ void __launch_bounds__(kCompactThreads)
       if (!c[k]) continue;
       if (slot < cap_slots) {
         const int4 key = traversal_key(sc, t0 + k);
-        out.keys[slot] = key;
-        out.start[slot] = part;
-        out.count[slot] = c[k];
+        if (copy == 0) {
+          out.keys[slot] = key;
+          out.start[slot] = part;
+          out.count[slot] = c[k];
+        }
         slots[k] = static_cast<int>(slot);
-        if (ZERO) active[atomicAdd(&n_active, 1u)] = key;
+        if (ZERO) {
+          active[slot - static_cast<uint32_t>(before >> 32)] = key;  // the same place in every copy
+          atomicAdd(&n_active, 1u);
+        }
       } else {
         overflow = true;
       }
@@ -1425,17 +1433,17 @@ __global__ void __launch_bounds__(kCompactThreads)
       if (PER == 4) total[t0 + k] = 0u;
     }
     if (overflow) set_status(scal, kStatusCapacity);
-    if (last && threadIdx.x == kCompactThreads - 1) {
+    if (last && copy == 0 && threadIdx.x == kCompactThreads - 1) {
       *out.nblocks = min(slot, cap_slots);
       *out.nparticles = part;
       *ticket = 0;
     }
   }
-  if (PER == 1 && t0 < n) clear[t0] = 0u;
+  if (PER == 1 && copy == 0 && t0 < n) clear[t0] = 0u;
   if (PER == 4 && t0 + 4 <= n) {
     *reinterpret_cast<int4*>(out.table + t0) =
         make_int4(slots[0], slots[PER > 1 ? 1 : 0], slots[PER > 2 ? 2 : 0], slots[PER > 3 ? 3 : 0]);
-  } else {
+  } else if (copy == 0) {
 #pragma unroll
     for (int k = 0; k < PER; ++k)
       if (t0 + k < n) out.table[t0 + k] = slots[k];
@@ -1443,12 +1451,9 @@ __global__ void __launch_bounds__(kCompactThreads)
   if constexpr (ZERO) {
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    for (uint32_t base = threadIdx.x & ~31u; base < n_active * 8u; base += kCompactThreads) {
-      const uint32_t t = base + lane;
-      int64_t f = -1;
-      if (t < n_active * 8u) f = claim_window(sc, active[t >> 3], static_cast<int>(t & 7u), stamp, epoch);
-      clear_claimed(f, g);
-    }
+    const uint32_t warps = gridDim.x / ntiles * (kCompactThreads / 32);
+    for (uint32_t b = copy * (kCompactThreads / 32) + (threadIdx.x >> 5); b < n_active; b += warps)
+      clear_claimed(lane < 8 ? claim_window(sc, active[b], lane, stamp, epoch) : -1, g);
     if (end) end_substep_by_last_cta(scal);
   }
 }

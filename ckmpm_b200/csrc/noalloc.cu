@@ -327,7 +327,6 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
 
   // Substeps: the launch sequence of ckmpm_step without graphs, in its launch shape.
   const uint32_t parts = cluster_parts(sms, counts[0]);
-  const bool fold = folds_zero(sc, counts[0]);
   const FusedFn fused = parts > 1 ? na_fused<true>(material->kind) : na_fused<false>(material->kind);
   if (nsteps > 0) set_next_dt_kernel<<<1, 32, 0, st>>>(scal, dt);
   for (uint32_t i = 0; i < nsteps; ++i) {
@@ -338,10 +337,7 @@ extern "C" ckmpm_status ckmpm_simulate_noalloc(const ckmpm_scene_desc* desc, con
       NA_CUDA(launch_clusters(fused, cluster_ctas(sms), kFusedThreads, parts, st, sc, md, gd, scal));
     else
       fused<<<ctas, kFusedThreads, kSmemFused, st>>>(sc, md, gd, scal);
-    NA_CUDA(launch_compact(sc, d, grid, scal, ntiles, st, parity ^ 1, parity, fold ? parity : -1, true));
-    if (!fold)
-      zero_windows_kernel<<<sms * 4, 256, 0, st>>>(sc, d.bl[parity ^ 1], grid.grid[parity], grid.stamp[parity], scal, 2,
-                                                   1);
+    NA_CUDA(launch_compact(sc, d, grid, scal, ntiles, st, parity ^ 1, parity, parity, true));
   }
   NA_CUDA(cudaGetLastError());
 

@@ -87,6 +87,23 @@ def test_a_spreading_scene_outgrows_its_clusters(engine_lib):
     assert ms[0] < 1.4 * ms[1], ms
 
 
+@pytest.mark.parametrize("n,small,large", [(130000, 16, 26), (460000, 24, 26)])
+def test_small_domain_is_no_slower_than_a_large_one(engine_lib, n, small, large):
+    """A body of many blocks in a domain whose compaction also zeroes the next windows, against the same body
+    in the smallest domain that gives the zeroing a launch of its own: no slower (1.2
+    times as slow at 343 blocks while one CTA per tile did the zeroing; the bound is 1.1)."""
+    import time
+    scene = [run(*box_scene(n, (b,) * 3, kind="drucker_prager", v0=(0.0, 0.0, 0.0)), 0) for b in (small, large)]
+    seconds = [math.inf, math.inf]
+    for _ in range(9):
+        for k, s in enumerate(scene):
+            t = time.perf_counter()
+            s.step(64, 1e-7)
+            seconds[k] = min(seconds[k], time.perf_counter() - t)
+    assert len(scene[0].blocks(0, 0)[1]) >= 300
+    assert seconds[0] < 1.1 * seconds[1], seconds
+
+
 @pytest.mark.parametrize("n", [40, 17000, 60000])
 def test_cam_clay_gives_the_same_bits_everywhere(engine_lib, n):
     """Cam-clay's F jumps with its last bit (F = U diag(S) V, V not transposed), so its own
