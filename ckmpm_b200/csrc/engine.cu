@@ -355,17 +355,36 @@ cudaError_t launch_zero(ckmpm_scene* s, int list_parity, int grid_parity, int32_
 // read: that of the other parity.  Once every model's fused kernel has read
 // grid[parity], its blocks that the next substep deposits into are zeroed for it
 // (epoch step + 2).
-cudaError_t enqueue_substep(ckmpm_scene* s, int parity) {
+// `mark(model, k)` is called before (k = 0) and after (1) a model's fused kernel, and before
+// (2) and after (3) its other launches: ckmpm_step_profiled records events there.
+template <typename Mark>
+cudaError_t enqueue_substep(ckmpm_scene* s, int parity, Mark mark) {
   cudaError_t e = cudaSuccess;
+  auto run = [&](cudaError_t r) {
+    if (e == cudaSuccess) e = r;
+  };
   const bool fold = folds_zero(s->sc);
-  for (auto& m : s->models) {
-    if (e == cudaSuccess) e = launch_fused_any(s, m, parity);
-    if (e == cudaSuccess && !fold) e = launch_compact(s, m, parity ^ 1, parity);
+  const size_t nm = s->models.size();
+  for (size_t i = 0; i < nm && e == cudaSuccess; ++i) {
+    run(mark(i, 0));
+    run(launch_fused_any(s, s->models[i], parity));
+    run(mark(i, 1));
+    if (fold) continue;
+    run(mark(i, 2));
+    run(launch_compact(s, s->models[i], parity ^ 1, parity));
+    if (i + 1 == nm && e == cudaSuccess) run(launch_zero(s, parity ^ 1, parity, 2, true));
+    run(mark(i, 3));
   }
-  if (!fold) return e == cudaSuccess ? launch_zero(s, parity ^ 1, parity, 2, true) : e;
-  for (auto& m : s->models)
-    if (e == cudaSuccess) e = launch_compact(s, m, parity ^ 1, parity, parity, &m == &s->models.back());
+  for (size_t i = 0; i < nm && fold && e == cudaSuccess; ++i) {
+    run(mark(i, 2));
+    run(launch_compact(s, s->models[i], parity ^ 1, parity, parity, i + 1 == nm));
+    run(mark(i, 3));
+  }
   return e;
+}
+
+cudaError_t enqueue_substep(ckmpm_scene* s, int parity) {
+  return enqueue_substep(s, parity, [](size_t, int) { return cudaSuccess; });
 }
 
 // One adaptive substep: the CFL dt from the grid it reads, then the substep.
@@ -1562,28 +1581,20 @@ ckmpm_status ckmpm_step_profiled(ckmpm_scene* s, uint32_t nsteps, float dt, doub
   set_next_dt_kernel<<<1, 32, 0, s->stream>>>(s->scal, dt);
   std::vector<cudaEvent_t> ev;
   const size_t nm = s->models.size();
-  ev.resize(nsteps * nm * 3);
+  ev.resize(nsteps * nm * 4);
   for (auto& x : ev) CK_CUDA(s, cudaEventCreate(&x));
   for (uint32_t i = 0; i < nsteps; ++i) {
-    const int parity = static_cast<int>((step + i) & 1);
-    for (size_t mi = 0; mi < nm; ++mi) {
-      auto& m = s->models[mi];
-      cudaEvent_t* E = &ev[(i * nm + mi) * 3];
-      CK_CUDA(s, cudaEventRecord(E[0], s->stream));
-      CK_CUDA(s, launch_fused_any(s, m, parity));
-      CK_CUDA(s, cudaEventRecord(E[1], s->stream));
-      CK_CUDA(s, launch_compact(s, m, parity ^ 1, parity));
-      if (mi + 1 == nm) CK_CUDA(s, launch_zero(s, parity ^ 1, parity, 2, true));
-      CK_CUDA(s, cudaEventRecord(E[2], s->stream));
-    }
+    CK_CUDA(s, enqueue_substep(s, static_cast<int>((step + i) & 1), [&](size_t model, int k) {
+              return cudaEventRecord(ev[(i * nm + model) * 4 + static_cast<size_t>(k)], s->stream);
+            }));
     ++s->host_step;
   }
   CK_CUDA(s, cudaStreamSynchronize(s->stream));
   double fused = 0, other = 0;
   for (uint32_t i = 0; i < nsteps * nm; ++i) {
     float a = 0, b = 0;
-    cudaEventElapsedTime(&a, ev[i * 3], ev[i * 3 + 1]);
-    cudaEventElapsedTime(&b, ev[i * 3 + 1], ev[i * 3 + 2]);
+    cudaEventElapsedTime(&a, ev[i * 4], ev[i * 4 + 1]);
+    cudaEventElapsedTime(&b, ev[i * 4 + 2], ev[i * 4 + 3]);
     fused += a;
     other += b;
   }

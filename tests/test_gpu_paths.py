@@ -104,6 +104,30 @@ def test_small_domain_is_no_slower_than_a_large_one(engine_lib, n, small, large)
     assert seconds[0] < 1.1 * seconds[1], seconds
 
 
+@pytest.mark.parametrize("blocks,bodies", [(12, 1), (12, 2), (26, 2)])
+def test_profiled_substeps_are_the_ones_that_run(engine_lib, blocks, bodies):
+    """step_profiled launches the kernels of step, in small and large domains, for one model and two, and moves
+    the scene alike."""
+    torch = pytest.importorskip("torch")
+    cfg, models = box_scene(5000, (blocks,) * 3)
+    if bodies == 2:
+        models += box_scene(3000, (blocks,) * 3, kind="fluid", seed=1)[1]
+    plain, profiled = run(cfg, models, 0), run(cfg, models, 0)
+
+    def kernels(step):
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            step()
+            torch.cuda.synchronize()
+        return sorted((e.key, e.count) for e in prof.key_averages() if "compact" in e.key or "zero_windows" in e.key)
+
+    a, b = kernels(lambda: plain.step(7, 1e-4)), kernels(lambda: profiled.step_profiled(7, 1e-4))
+    if not a and not b:
+        pytest.skip("no kernel records here (another profiler holds them)")
+    assert a == b
+    for m in range(bodies):
+        assert_same(profiled.state(m), plain.state(m), m)
+
+
 @pytest.mark.parametrize("n", [40, 17000, 60000])
 def test_cam_clay_gives_the_same_bits_everywhere(engine_lib, n):
     """Cam-clay's F jumps with its last bit (F = U diag(S) V, V not transposed), so its own
