@@ -676,12 +676,13 @@ struct ckmpm_diff {
   float* ck = nullptr;                // checkpoints: nseg x 12n
   float4* ckvel = nullptr;            // nseg x nn
   float* tape = nullptr;              // max(every - 1, 1) x 12n: substeps s0 + 1 .. s1 - 1 of a segment
-  float4* tapevel = nullptr;          // every x nn
-  float4* vel = nullptr;              // scratch node velocities (forward pass)
+  float4* tapevel = nullptr;          // every x nn; a segment's first substep has its checkpoint's, so slot 0 is free:
+  float4* vel = nullptr;              // scratch node velocities (forward pass), in that slot
   unsigned long long* gsum[3] = {nullptr, nullptr, nullptr};  // substep s reads [s % 3], deposits into [(s + 1) % 3]
   int* box = nullptr;                 // (nsteps + 1) x 6
   float *xb = nullptr, *Fb = nullptr, *mub = nullptr, *lamb = nullptr;
-  unsigned long long* vbar[3] = {nullptr, nullptr, nullptr};  // substep s's velocity adjoints: [s % 3]
+  // Substep s's velocity adjoints: [s % 3].  In gsum's memory when every substep is a checkpoint.
+  unsigned long long* vbar[3] = {nullptr, nullptr, nullptr};
   // Particle order: perm[slot] = input particle; bins and their scan, each particle's bin and place in it.
   uint32_t *perm = nullptr, *bins = nullptr, *first = nullptr, *scan = nullptr, *bin = nullptr, *rank = nullptr;
   cudaGraphExec_t gfwd = nullptr, gbwd = nullptr;
@@ -792,18 +793,23 @@ ckmpm_status ckmpm_diff_create(const ckmpm_scene_desc* desc, uint32_t n, float m
             dk_alloc(h, &h->ckvel, static_cast<size_t>(h->nseg) * nn) == cudaSuccess &&
             dk_alloc(h, &h->tape, static_cast<size_t>(std::max<uint32_t>(h->every, 2) - 1) * 12 * n) == cudaSuccess &&
             dk_alloc(h, &h->tapevel, static_cast<size_t>(h->every) * nn) == cudaSuccess &&
-            dk_alloc(h, &h->vel, nn) == cudaSuccess && dk_alloc(h, &h->gsum[0], 4 * nn) == cudaSuccess &&
+            dk_alloc(h, &h->gsum[0], 4 * nn) == cudaSuccess &&
             dk_alloc(h, &h->gsum[1], 4 * nn) == cudaSuccess && dk_alloc(h, &h->gsum[2], 4 * nn) == cudaSuccess &&
             dk_alloc(h, &h->box, 6 * static_cast<size_t>(nsteps + 1)) == cudaSuccess &&
             dk_alloc(h, &h->xb, 3 * n) == cudaSuccess && dk_alloc(h, &h->Fb, 9 * n) == cudaSuccess &&
             dk_alloc(h, &h->mub, n) == cudaSuccess && dk_alloc(h, &h->lamb, n) == cudaSuccess &&
-            dk_alloc(h, &h->vbar[0], 3 * nn) == cudaSuccess && dk_alloc(h, &h->vbar[1], 3 * nn) == cudaSuccess &&
-            dk_alloc(h, &h->vbar[2], 3 * nn) == cudaSuccess &&
             dk_alloc(h, &h->d.adj_scale, 4) == cudaSuccess && dk_alloc(h, &h->perm, n) == cudaSuccess &&
             dk_alloc(h, &h->bin, n) == cudaSuccess && dk_alloc(h, &h->rank, n) == cudaSuccess &&
             dk_alloc(h, &h->bins, order_bins(d.G)) == cudaSuccess &&
             dk_alloc(h, &h->first, order_bins(d.G)) == cudaSuccess &&
             dk_alloc(h, &h->scan, scan_tiles(order_bins(d.G))) == cudaSuccess;
+  // A backward that recomputes nothing touches no node sums, and every pass leaves them and
+  // the velocity adjoints at zero: they share their memory then.
+  for (int k = 0; k < 3; ++k) {
+    if (h->every == 1) h->vbar[k] = h->gsum[k];
+    else ok = ok && dk_alloc(h, &h->vbar[k], 3 * nn) == cudaSuccess;
+  }
+  h->vel = h->tapevel;
   if (!ok) return bail(dfail(h, CKMPM_ERR_CUDA, "device allocation failed"));
   // Sums and velocity adjoints start (and are always left) at zero inside every box.
   if (cudaFuncSetAttribute(reinterpret_cast<const void*>(particle_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -813,7 +819,7 @@ ckmpm_status ckmpm_diff_create(const ckmpm_scene_desc* desc, uint32_t n, float m
     return bail(dfail(h, CKMPM_ERR_CUDA, "cudaFuncSetAttribute failed"));
   for (int k = 0; k < 3; ++k)
     if (cudaMemsetAsync(h->gsum[k], 0, 32 * nn, h->stream) != cudaSuccess ||
-        cudaMemsetAsync(h->vbar[k], 0, 24 * nn, h->stream) != cudaSuccess)
+        (h->vbar[k] != h->gsum[k] && cudaMemsetAsync(h->vbar[k], 0, 24 * nn, h->stream) != cudaSuccess))
       return bail(dfail(h, CKMPM_ERR_CUDA, "initialisation failed"));
   if (cudaMemsetAsync(h->d.adj_scale, 0, 4 * sizeof(float), h->stream) != cudaSuccess ||
       cudaMemsetAsync(h->vel, 0, 16 * nn, h->stream) != cudaSuccess ||

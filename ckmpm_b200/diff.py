@@ -7,7 +7,7 @@ checkpoint every `checkpoint_every` substeps; backward recomputes one segment
 at a time from its checkpoint and runs the adjoint of P2G, the grid update,
 G2P and the SVD-based stress (ckmpm_b200/csrc/diff_math.cuh).  By default the
 interval is the smallest whose checkpoints and tape fit in half of the free
-device memory: 1 (the whole rollout kept, nothing recomputed) whenever it fits.  Inputs and
+device memory, and beside the working buffers: 1 (the whole rollout kept, nothing recomputed) whenever it fits.  Inputs and
 outputs are CUDA float32 tensors; the work is ordered on torch's current
 stream.
 
@@ -72,6 +72,17 @@ def rollout_bytes(config: MPMConfig, n: int, nsteps: int, every: int) -> int:
     return nseg * (state + vel) + max(every - 1, 1) * state + every * vel
 
 
+def working_bytes(config: MPMConfig, n: int, every: int) -> int:
+    """Device bytes of a rollout besides rollout_bytes: three buffers of node sums (32 B per
+    node), three of node-velocity adjoints (24 B) where substeps are recomputed (every > 1;
+    they share memory with the sums otherwise), the particle order's bins (1 B) and 81 words
+    per particle."""
+    nodes = 2
+    for b in config.domain_blocks:
+        nodes *= 4 * int(b)
+    return nodes * (3 * 32 + (3 * 24 if every > 1 else 0) + 1) + 4 * 81 * n
+
+
 def auto_checkpoint_interval(config: MPMConfig, n: int, nsteps: int, budget_bytes: int) -> int:
     """The smallest checkpoint interval whose checkpoints and tape fit in budget_bytes;
     when none does, the interval that needs the least memory."""
@@ -81,17 +92,23 @@ def auto_checkpoint_interval(config: MPMConfig, n: int, nsteps: int, budget_byte
     return min(range(1, nsteps + 1), key=lambda k: (rollout_bytes(config, n, nsteps, k), k))
 
 
+def checkpoint_budget(config: MPMConfig, n: int, free_bytes: int) -> int:
+    """Memory for the checkpoints and the tape of a device with free_bytes left: half of it,
+    or what the working buffers of a recomputing rollout leave of 31/32 of it."""
+    return max(0, min(free_bytes // 2, free_bytes - free_bytes // 32 - working_bytes(config, n, 2)))
+
+
 class DiffRollout:
     """A differentiable rollout of n fixed-corotated particles (ckmpm_diff_* handle).
     checkpoint_every None picks the interval by memory (auto_checkpoint_interval
-    over half of the device's free memory)."""
+    over checkpoint_budget)."""
 
     def __init__(self, config: MPMConfig, n: int, mass: float, volume: float, nu: float = 0.3, nsteps: int = 200,
                  dt: float = 1e-4, checkpoint_every: int | None = None):
         self.config, self.n, self.nsteps, self.dt = config, n, nsteps, dt
         if checkpoint_every is None:
             free, _ = torch.cuda.mem_get_info(config.device)
-            checkpoint_every = auto_checkpoint_interval(config, n, nsteps, free // 2)
+            checkpoint_every = auto_checkpoint_interval(config, n, nsteps, checkpoint_budget(config, n, free))
         self.checkpoint_every = checkpoint_every
         self._h = C.c_void_p()
         desc = config.to_c()

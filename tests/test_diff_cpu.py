@@ -87,3 +87,31 @@ def test_checkpoint_interval_by_memory():
     least = auto_checkpoint_interval(cfg, n, nsteps, 0)
     assert all(rollout_bytes(cfg, n, nsteps, least) <= rollout_bytes(cfg, n, nsteps, e) for e in range(1, nsteps + 1))
     assert 1 < least < nsteps
+
+
+@pytest.mark.parametrize("free_gb", [10.6, 10.8, 11, 11.2, 12, 16, 40, 180])
+def test_automatic_rollout_fits_the_free_memory(monkeypatch, free_gb):
+    """The interval chosen for a 64^3-block domain leaves room for the working buffers as well: node sums, velocity
+    adjoints and the order's bins (169 B per node in all where substeps are recomputed) and 324 B per particle."""
+    import torch
+    from ckmpm_b200 import diff
+    from ckmpm_b200.engine import MPMConfig
+    asked = []
+
+    class Library:
+        def ckmpm_diff_create(self, desc, n, mass, volume, nu, nsteps, dt, every, out):
+            asked.append(every)
+            return 0
+
+        def ckmpm_diff_destroy(self, handle):
+            return 0
+
+    free = int(free_gb * 1e9)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (free, 183 << 30))
+    monkeypatch.setattr(diff, "_lib", Library)
+    n, nsteps, nodes = 50_000, 20, 2 * 256 ** 3
+    diff.DiffRollout(MPMConfig(dx=1 / 256, domain_blocks=(64,) * 3), n, 1e-6, 1e-9, nsteps=nsteps)
+    every = asked[0]
+    held = -(-nsteps // every) * (48 * n + 16 * nodes) + max(every - 1, 1) * 48 * n + every * 16 * nodes
+    assert held + 169 * nodes + 324 * n <= free
+    assert held <= free // 2

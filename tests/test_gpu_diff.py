@@ -251,3 +251,21 @@ def test_config5_per_particle_gradients_against_fp64_differences(engine_lib, ora
         for kd, p, fd, ad in rows:
             if kd == kind:
                 assert abs(fd - ad) <= 2e-3 * abs(fd) + 1e-3 * scale, (kind, p, fd, ad)
+
+
+@pytest.mark.parametrize("every", [1, 4])
+def test_rollout_memory_is_what_is_announced(engine_lib, every):
+    """rollout_bytes and working_bytes against the device memory that a rollout takes (allocations of 2 MB and more
+    are rounded up: 64 arrays at most)."""
+    torch = pytest.importorskip("torch")
+    from ckmpm_b200.diff import DiffRollout, rollout_bytes, working_bytes
+    from ckmpm_b200.engine import MPMConfig
+    cfg = MPMConfig(dx=1 / 128, domain_blocks=(32,) * 3)
+    n, nsteps = 20_000, 12
+    torch.cuda.synchronize()
+    before, _ = torch.cuda.mem_get_info(0)
+    sim = DiffRollout(cfg, n, 1e-6, 1e-9, nsteps=nsteps, checkpoint_every=every)
+    taken = before - torch.cuda.mem_get_info(0)[0]
+    sim.close()
+    announced = rollout_bytes(cfg, n, nsteps, every) + working_bytes(cfg, n, every)
+    assert announced <= taken + (1 << 20) and taken <= announced + 64 * (2 << 20), (taken, announced)
