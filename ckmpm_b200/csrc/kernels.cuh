@@ -909,8 +909,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
       // Cam-clay's transfers hold C and D in place of C dx and D / dx^2.
       const bool clayey = KIND == kNacc || (KIND == kMixed && kind == kNacc);
       if (clayey) {
-        const float xs[3] = {x[0] * inv_dx, x[1] * inv_dx, x[2] * inv_dx};
-        clay::g2p(vtile, xs, key, sc.dx, v, Cdx, inside, Dold);
+        clay::g2p(vtile, x, key, sc.dx, inv_dx, v, Cdx, inside, Dold);
       } else {
         g2p(vtile, x, inv_dx, key, v, Cdx, inside, Dold);
       }
@@ -929,7 +928,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         }
       }
 #pragma unroll
-      for (int a = 0; a < 3; ++a) x[a] = clayey ? x[a] + dt * adv[a] : fmaf(dt, adv[a], x[a]);
+      for (int a = 0; a < 3; ++a) x[a] = fmaf(dt, adv[a], x[a]);
 
       float tau[9];
       if (kind == kFluid) {
@@ -941,8 +940,8 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         float dW[9];
         if (clayey) {
 #pragma unroll
-          for (int k = 0; k < 9; ++k) dW[k] = Cdx[k] * dt + ((k & 3) ? 0.f : 1.f);
-          matmul3_plain(dW, F, F);
+          for (int k = 0; k < 9; ++k) dW[k] = fmaf(Cdx[k], dt, (k & 3) ? 0.f : 1.f);
+          matmul3_nacc(dW, F, F);
         } else {
 #pragma unroll
           for (int k = 0; k < 9; ++k) dW[k] = (k & 3) ? Cdx[k] * dtdx : fmaf(Cdx[k], dtdx, 1.f);
@@ -1018,9 +1017,8 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         int lb[2][3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          const float xs = x[a] * inv_dx;
-          st[0][a] = clay::axis_stencil<-1>(xs);
-          st[1][a] = clay::axis_stencil<1>(xs);
+          st[0][a] = clay::axis_stencil<-1>(x[a], inv_dx);
+          st[1][a] = clay::axis_stencil<1>(x[a], inv_dx);
           lb[0][a] = st[0][a].base - 4 * kk[a];
           lb[1][a] = st[1][a].base - 4 * kk[a];
         }
@@ -1035,7 +1033,7 @@ __global__ void __launch_bounds__(NT, fused_min_ctas<NT>())
         const float sA = ndt * vol_over_mass;
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
-          Ah[k] = (Cdx[k] - sA * DT[k]) * sc.dx;
+          Ah[k] = __fmul_rn(fmaf(-sA, DT[k], Cdx[k]), sc.dx);
           finite &= fabsf(Ah[k]) < kFixMaxValue;
         }
 #pragma unroll
@@ -1188,9 +1186,8 @@ __global__ void __launch_bounds__(NT, 2) rasterize_kernel(SceneDev sc, ModelDev 
         bool ok = true;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          const float xs = s0.x[a][i] * inv_dx;
-          st[0][a] = clay::axis_stencil<-1>(xs);
-          st[1][a] = clay::axis_stencil<1>(xs);
+          st[0][a] = clay::axis_stencil<-1>(s0.x[a][i], inv_dx);
+          st[1][a] = clay::axis_stencil<1>(s0.x[a][i], inv_dx);
           lb[0][a] = st[0][a].base - 4 * kk[a];
           lb[1][a] = st[1][a].base - 4 * kk[a];
           ok &= lb[0][a] >= 0 && lb[0][a] <= 6 && lb[1][a] >= 0 && lb[1][a] <= 6;

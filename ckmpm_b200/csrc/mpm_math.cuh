@@ -63,7 +63,19 @@ CKMPM_DEV void matmul3(const float* a, const float* b, float* r) {
   for (int k = 0; k < 9; ++k) r[k] = t[k];
 }
 
-// The same with the compiler's own contraction, for the Cam-clay path (nacc_transfer.cuh).
+// For the Cam-clay path (nacc_transfer.cuh): the first product fused into the rounded second, then the third.
+CKMPM_DEV void matmul3_nacc(const float* a, const float* b, float* r) {
+  float t[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      t[i * 3 + j] = fmaf(a[i * 3 + 2], b[6 + j], fmaf(a[i * 3], b[j], __fmul_rn(a[i * 3 + 1], b[3 + j])));
+#pragma unroll
+  for (int k = 0; k < 9; ++k) r[k] = t[k];
+}
+
+// The same with the compiler's own contraction (Cam-clay's D^-1 tau).
 CKMPM_DEV void matmul3_plain(const float* a, const float* b, float* r) {
   float t[9];
 #pragma unroll
@@ -175,7 +187,7 @@ CKMPM_DEV void swap_cols(float* V, float& la, float& lb, int a, int b) {
   }
 }
 
-template <int kSweeps = 3, bool PLAIN = false>
+template <int kSweeps = 3, bool NACC = false>
 CKMPM_DEV void svd3(const float* A, float* U, float* S, float* V) {
   // M = A^T A (symmetric; 6 unique entries)
   float m00 = A[0] * A[0] + A[3] * A[3] + A[6] * A[6];
@@ -197,7 +209,7 @@ CKMPM_DEV void svd3(const float* A, float* U, float* S, float* V) {
   if (l0 < l2) swap_cols(V, l0, l2, 0, 2);
   if (l1 < l2) swap_cols(V, l1, l2, 1, 2);
   float B[9];
-  if (PLAIN) matmul3_plain(A, V, B);
+  if (NACC) matmul3_nacc(A, V, B);
   else matmul3(A, V, B);
 #pragma unroll
   for (int k = 0; k < 9; ++k) U[k] = (k & 3) ? 0.0f : 1.0f;

@@ -140,6 +140,37 @@ def test_cam_clay_gives_the_same_bits_everywhere(engine_lib, n):
         assert_same(run(cfg, models, 33, shape).state(0), a, shape)
 
 
+@pytest.mark.parametrize("n,dx", [(40, 1 / 64), (17000, 1 / 64), (17000, 1 / 37)])
+def test_cam_clay_gives_the_same_bits_in_every_kernel(engine_lib, n, dx):
+    """The rigid form and the mixed kernel of a batch (a von Mises scene beside two of clay) against the single
+    scene's kernel, with particles on the faces of cells and blocks and an ulp beside them: every stencil lies in
+    its block's window (a base cell other than the binning's raises a status)."""
+    from ckmpm_b200.batch import SceneBatch
+    cfg, models = box_scene(n, (14, 14, 14), dx=dx, v0=(0.4, -3.0, 0.3))
+    lam, mu = compute_lame_parameters(2e4, 0.4)
+    body = models[0]
+    body.material = MPMMaterial.nacc(mu, lam, -0.01, 0.5, 0.8, 2.36, True)
+    x = body.particle_position
+    cells = np.rint(x[::3] / dx - 0.25) + 0.75  # faces of grid -dx/4's cells
+    x[::3] = (cells * dx).astype(np.float32)
+    x[::6] = np.nextafter(x[::6], np.float32(0))
+    x[1::6] = np.nextafter(x[1::6], np.float32(1e3))
+    ref = run(cfg, models, 33, (256, 4, 8))
+    rigid = Scene(cfg)
+    rigid.add_model(body)
+    rigid.set_rigid(1, (0.1, 0.0, 0.0))
+    rigid.setup()
+    rigid.step(33, 1e-4)
+    assert_same(rigid.state(0), ref.state(0), "rigid")
+    metal = MPMModel(body.particle_mass, body.particle_volume, x, body.particle_velocity,
+                     MPMMaterial.von_mises(mu, lam, 500.0))
+    batch = SceneBatch(cfg, [body, metal, body])
+    batch.setup()
+    batch.step(33, 1e-4)
+    for i in (0, 2):
+        assert_same(batch.scene_state(i), ref.state(0), i)
+
+
 @pytest.mark.parametrize("dims", [(9, 11, 13), (25, 25, 26), (26, 26, 26), (64, 17, 16)])
 def test_domain_size_does_not_matter(engine_lib, dims):
     """The compaction's small and large tiles, odd extents among them: the same body far from
