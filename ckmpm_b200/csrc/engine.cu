@@ -1220,7 +1220,8 @@ static cudaError_t ensure_export_buffers(ckmpm_scene*, ModelHost& m) {
 // export buffers (input order when ids are tracked).  n_upper bounds the live
 // count; n_dev, when given, is the device copy of it, else n_upper is the count.
 // While no particle has been lost, input order is the order of the ids, and the
-// passes that place live ids are left out (or, the count not known here, do nothing).
+// passes that place live ids are left out.  Where the count is not known here, the
+// listing and marking of ids return at once then; the flags' reset and scan still run.
 static cudaError_t enqueue_export(ckmpm_scene* s, ModelHost& m, bool x, bool v, bool F, bool aux, bool id,
                                   uint32_t n_upper, const uint32_t* n_dev) {
   const size_t cap_p = m.dev.cap_particles;
