@@ -39,6 +39,10 @@ constexpr int kThreads = 128;
 constexpr float kScale = 68719476736.0f;  // 2^36
 constexpr float kMaxValue = 131072.0f;    // 2^17
 constexpr uint32_t kErrOutside = 1u, kErrRange = 2u;
+// CTAs of a particle kernel at least: those past the particles help to zero a box that is
+// large for the few particles in it (500 particles spread over a 64^3-cell domain: 93 us a forward
+// substep zeroed by their 4 CTAs, 25 by 296, 26 by 592).
+constexpr uint32_t kZeroCtas = 296;
 constexpr float kAdjUnits = 1099511627776.0f;  // 2^40 fixed-point units per largest seed component
 constexpr float kAdjMaxUnits = 4.6e18f;        // |contribution| bound in units (< 2^62)
 
@@ -53,6 +57,8 @@ struct Dev {
   uint32_t* status;
   float* adj_scale;  // [0]: fixed-point units per adjoint unit, [1]: its inverse; [2]: max |seed| (bits)
 };
+
+__device__ __forceinline__ uint32_t particle_ctas(const Dev& d) { return (d.n + kThreads - 1) / kThreads; }
 
 __device__ __forceinline__ void box_reset(int* b) {
   b[0] = b[1] = b[2] = INT_MAX;
@@ -206,10 +212,17 @@ __device__ __forceinline__ void tile_flush(const Dev& d, const CtaBox& b, const 
 }
 
 // Grid update of one node from its sums: velocity and mass.
-__device__ __forceinline__ float4 node_from_sums(const Dev& d, const unsigned long long* __restrict__ gsum, int id, int cx,
-                                                 int cy, int cz, float dt) {
+struct NodeSums {
+  ulonglong2 s01, s23;
+};
+
+__device__ __forceinline__ NodeSums load_sums(const unsigned long long* __restrict__ gsum, int id) {
   const ulonglong2* q = reinterpret_cast<const ulonglong2*>(gsum + 4 * static_cast<size_t>(id));
-  const ulonglong2 s01 = q[0], s23 = q[1];
+  return {q[0], q[1]};
+}
+
+__device__ __forceinline__ float4 node_from_sums(const Dev& d, const NodeSums& s, int cx, int cy, int cz, float dt) {
+  const ulonglong2 s01 = s.s01, s23 = s.s23;
   const float m = __ll2float_rn(static_cast<long long>(s01.x)) * d.unit;
   const float mv[3] = {__ll2float_rn(static_cast<long long>(s01.y)) * d.unit,
                        __ll2float_rn(static_cast<long long>(s23.x)) * d.unit,
@@ -233,13 +246,17 @@ __device__ __forceinline__ float4 node_adjoint(const Dev& d, const unsigned long
   return make_float4(out[0], out[1], out[2], out[3]);
 }
 
-// Zeroes kCh sums per node over a substep's node box, shared out over the grid.
+// Zeroes kCh sums per node over a substep's node box, shared out over the grid's first
+// `ctas` CTAs, or over all of them if the box has more nodes than those have threads.
 template <int kCh>
-__device__ __forceinline__ void zero_box(const Dev& d, const int* __restrict__ b, unsigned long long* __restrict__ sums) {
+__device__ __forceinline__ void zero_box(const Dev& d, const int* __restrict__ b, unsigned long long* __restrict__ sums,
+                                         uint32_t ctas) {
   if (!sums || b[0] > b[3]) return;
   const int ex = b[3] - b[0] + 1, ey = b[4] - b[1] + 1, ez = b[5] - b[2] + 1;
   const int total = 2 * ex * ey * ez;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+  if (static_cast<uint32_t>(total) > ctas * blockDim.x) ctas = gridDim.x;
+  if (blockIdx.x >= ctas) return;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += ctas * blockDim.x) {
     const int z = t % ez, xy = t / ez, y = xy % ey, gx = xy / ey, x = gx % ex, g = gx / ex;
     unsigned long long* q =
         sums + kCh * static_cast<size_t>(diff::node_index(d.G, g, b[0] + x, b[1] + y, b[2] + z));
@@ -250,7 +267,7 @@ __device__ __forceinline__ void zero_box(const Dev& d, const int* __restrict__ b
 
 template <int kCh>
 __global__ void zero_box_kernel(Dev d, const int* __restrict__ b, unsigned long long* __restrict__ sums) {
-  zero_box<kCh>(d, b, sums);
+  zero_box<kCh>(d, b, sums, gridDim.x);
 }
 
 // Deposits of the CTA's particles (per unit mass) into gsum and the merge of their
@@ -368,7 +385,7 @@ __global__ void grid_kernel(Dev d, unsigned long long* __restrict__ gsum, const 
     const int g = static_cast<int>(t / (static_cast<int64_t>(ez) * ey * ex));
     const int cx = b[0] + x, cy = b[1] + y, cz = b[2] + z;
     const int id = diff::node_index(d.G, g, cx, cy, cz);
-    vel[id] = node_from_sums(d, gsum, id, cx, cy, cz, dt);
+    vel[id] = node_from_sums(d, load_sums(gsum, id), cx, cy, cz, dt);
     ulonglong2* q = reinterpret_cast<ulonglong2*>(gsum + 4 * static_cast<size_t>(id));
     q[0] = make_ulonglong2(0ull, 0ull);
     q[1] = make_ulonglong2(0ull, 0ull);
@@ -386,6 +403,49 @@ struct VelReader {
   const unsigned long long* sums;
   float dt;
   bool tiled, inside;  // the particle's stencil lies in the tile / in the grid
+  // The nodes (g, cx, cy + i, cz + j), v[2 i + j].  All four are loaded before the first is
+  // used: one after another, each behind the branches of the last one's grid update, the 16
+  // loads of a particle took 4 us of a 20 us substep of a sparse cloud.
+  __device__ void quad(int g, int cx, int cy, int cz, float (*v)[3]) const {
+    float4 q[4];
+    if (tiled) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = tile[box_entry(*b, g, cx, cy + (k >> 1), cz + (k & 1))];
+    } else {
+      int id[4];
+      bool in[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        in[k] = inside || diff::node_in_grid(d->G, cx, cy + (k >> 1), cz + (k & 1));
+        id[k] = in[k] ? diff::node_index(d->G, g, cx, cy + (k >> 1), cz + (k & 1)) : 0;
+      }
+      if (sums) {
+        NodeSums s[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s[k] = load_sums(sums, id[k]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          q[k] = node_from_sums(*d, s[k], cx, cy + (k >> 1), cz + (k & 1), dt);
+          if (in[k]) vel[id[k]] = q[k];
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = vel[id[k]];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (in[k]) continue;
+        atomicOr(d->status, kErrOutside);
+        q[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k][0] = q[k].x;
+      v[k][1] = q[k].y;
+      v[k][2] = q[k].z;
+    }
+  }
   __device__ void operator()(int g, int cx, int cy, int cz, float* v) const {
     float4 q;
     if (tiled) {
@@ -394,13 +454,7 @@ struct VelReader {
       atomicOr(d->status, kErrOutside);
       q = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
-      const int id = diff::node_index(d->G, g, cx, cy, cz);
-      if (sums) {
-        q = node_from_sums(*d, sums, id, cx, cy, cz, dt);
-        vel[id] = q;
-      } else {
-        q = vel[id];
-      }
+      q = vel[diff::node_index(d->G, g, cx, cy, cz)];
     }
     v[0] = q.x;
     v[1] = q.y;
@@ -433,6 +487,10 @@ __global__ void __launch_bounds__(kThreads) particle_kernel(
   float4* vtile = reinterpret_cast<float4*>(tile + 8 * kTileCap);
   __shared__ int s_box[2][6];
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x * kThreads >= d.n) {  // no particles: a CTA that only zeroes
+    zero_box<4>(d, bzero, gsum_zero, particle_ctas(d));
+    return;
+  }
   const bool active = p < d.n;
   if (threadIdx.x < 2) box_reset(s_box[threadIdx.x]);
   __syncthreads();
@@ -447,7 +505,7 @@ __global__ void __launch_bounds__(kThreads) particle_kernel(
     inside = box_in_grid(d.G, lo, hi);
   }
   cta_box_merge(s_box[0], inside, lo, hi);
-  zero_box<4>(d, bzero, gsum_zero);
+  zero_box<4>(d, bzero, gsum_zero, particle_ctas(d));
   tile_zero(tile, 8 * kTileCap);
   __syncthreads();
   const CtaBox b = cta_box(s_box[0]);
@@ -455,7 +513,7 @@ __global__ void __launch_bounds__(kThreads) particle_kernel(
     int cx, cy, cz;
     const int id = box_node(d, b, i, cx, cy, cz);
     if (gsum_in) {
-      const float4 q = node_from_sums(d, gsum_in, id, cx, cy, cz, dt);
+      const float4 q = node_from_sums(d, load_sums(gsum_in, id), cx, cy, cz, dt);
       vtile[i] = q;
       vel[id] = q;  // every CTA that reads the node writes the same value
     } else {
@@ -512,6 +570,10 @@ __global__ void __launch_bounds__(kThreads, 3) particle_adjoint_kernel(
   float4* gtile = reinterpret_cast<float4*>(tile + 6 * kTileCap);
   __shared__ int s_box[2][6];
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x * kThreads >= d.n) {  // no particles: a CTA that only zeroes
+    zero_box<3>(d, bzero, vbar_zero, particle_ctas(d));
+    return;
+  }
   const bool active = p < d.n;
   if (threadIdx.x < 2) box_reset(s_box[threadIdx.x]);
   __syncthreads();
@@ -534,7 +596,7 @@ __global__ void __launch_bounds__(kThreads, 3) particle_adjoint_kernel(
   }
   cta_box_merge(s_box[0], inside, lo, hi);
   cta_box_merge(s_box[1], inside2, lo2, hi2);
-  zero_box<3>(d, bzero, vbar_zero);
+  zero_box<3>(d, bzero, vbar_zero, particle_ctas(d));
   tile_zero(tile, 6 * kTileCap);
   __syncthreads();
   const CtaBox b = cta_box(s_box[0]), b2 = cta_box(s_box[1]);
@@ -723,6 +785,8 @@ using namespace ckmpm::diffk;
 
 unsigned blocks_for(uint32_t n) { return (n + kThreads - 1) / kThreads; }
 
+unsigned zeroing_blocks(uint32_t n) { return std::max<unsigned>(blocks_for(n), kZeroCtas); }
+
 int grid_ctas(const ckmpm_diff* h) {
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
@@ -856,7 +920,7 @@ namespace {
 void forward_substep(ckmpm_diff* h, uint32_t s, const float* in, float* outp, float4* vel, const unsigned long long* sums,
                      float cdt, float ndt, bool zero_prev) {
   const uint32_t n = h->d.n;
-  particle_kernel<<<blocks_for(n), kThreads, kForwardSmem, h->stream>>>(
+  particle_kernel<<<zeroing_blocks(n), kThreads, kForwardSmem, h->stream>>>(
       h->d, in, in + 3 * n, h->lam, h->mu, vel, sums, cdt, ndt, h->gsum[(s + 1) % 3], h->box + 6 * (s + 1),
       zero_prev ? h->gsum[(s + 2) % 3] : nullptr, h->box + 6 * (s > 0 ? s - 1 : 0), outp, outp + 3 * n);
 }
@@ -954,7 +1018,7 @@ cudaError_t enqueue_backward(ckmpm_diff* h) {
       const float cdt = s == 0 ? 0.f : h->dt, ndt = h->dt;
       const float* in = statep(s);
       // vbar of substep s + 2, which substep s + 1 read, is zeroed here.
-      particle_adjoint_kernel<<<blocks_for(n), kThreads, kAdjointSmem, st>>>(
+      particle_adjoint_kernel<<<zeroing_blocks(n), kThreads, kAdjointSmem, st>>>(
           d, in, in + 3 * n, xnext, h->lam, h->mu, velp(s), vnext, cdt, ndt, vnext ? h->vbar[(s + 1) % 3] : nullptr, h->xb,
           h->Fb, h->mub, h->lamb, h->vbar[s % 3], s + 2 < N ? h->vbar[(s + 2) % 3] : nullptr,
           h->box + 6 * std::min(s + 2, N));

@@ -365,6 +365,18 @@ struct Fwd {
   T tau[9], M[9], A[9];     // M = (0.5 (D + D'))^-1, A per unit mass
 };
 
+// The velocities of nodes (cx, cy + i, cz + j) in v[2 i + j]: by vel's own quad, else one by one.
+template <class T, class Vel>
+CKD auto read_quad(const Vel& vel, int g, int cx, int cy, int cz, T (*v)[3], int) -> decltype(vel.quad(g, cx, cy, cz, v)) {
+  vel.quad(g, cx, cy, cz, v);
+}
+
+template <class T, class Vel>
+CKD void read_quad(const Vel& vel, int g, int cx, int cy, int cz, T (*v)[3], long) {
+  CKD_UNROLL
+  for (int k = 0; k < 4; ++k) vel(g, cx, cy + (k >> 1), cz + (k & 1), v[k]);
+}
+
 // G2P + x, F update + stress + affine term.  vel(g, cx, cy, cz, T* v) returns
 // the node velocity after the grid update; svd(F, U, S, V) any SVD.  xn, when
 // given, is the new position where it is already known.
@@ -385,16 +397,13 @@ CKD void particle_forward(const Particle<T>& p, T lambda, T mu, T vol_over_mass,
     T Sy[2][3], Ty[2][3], Tz[2][3];
     CKD_UNROLL
     for (int i = 0; i < 2; ++i) {
-      T a0[3], a1[3], b0[3], b1[3];
-      vel(g, ax->base + i, ay->base, az->base, a0);
-      vel(g, ax->base + i, ay->base, az->base + 1, a1);
-      vel(g, ax->base + i, ay->base + 1, az->base, b0);
-      vel(g, ax->base + i, ay->base + 1, az->base + 1, b1);
+      T q[4][3];
+      read_quad(vel, g, ax->base + i, ay->base, az->base, q, 0);
       CKD_UNROLL
       for (int r = 0; r < 3; ++r) {
-        const T ta = wz1 * a1[r], tb = wz1 * b1[r];
-        Ty[i][r] = wy1 * (wz0 * b0[r] + tb);
-        Sy[i][r] = wy0 * (wz0 * a0[r] + ta) + Ty[i][r];
+        const T ta = wz1 * q[1][r], tb = wz1 * q[3][r];
+        Ty[i][r] = wy1 * (wz0 * q[2][r] + tb);
+        Sy[i][r] = wy0 * (wz0 * q[0][r] + ta) + Ty[i][r];
         Tz[i][r] = wy0 * ta + wy1 * tb;
       }
     }
